@@ -48,12 +48,12 @@ METRIC = ("unique faces/s of one density flux-advection step at %d^3 (move_subst
 UNIT = "faces/s"
 VELOCITY_SEED, DENSITY_SEED = 101, 102
 CFL = 2.0
-# FP32 operation count of one 1D WENO6 evaluation as implemented in fia_device.cuh
-# (weno6_eval, FP32 form: differences 12, three cubic candidates 18, three smoothness
-# indicators in Horner form with eps as the start of each chain 45, nonlinear weights by
-# reciprocals 9, the weighted sum and its normalisation 9; an FMA counted as two, a
-# reciprocal as one).  The face kernel counts the 1D evaluations it executes.
-WENO1D_FLOP = 93
+# FP32 operation count of one 1D WENO6 evaluation as implemented in fia_weno_rec.cuh, averaged
+# over the evaluations of a piece at 3 Gauss points (an FMA counted as two, a reciprocal as one):
+# z from a stored record 23; y 63 for the data of a stencil that 3 points share and 21 a point; x
+# 84: 2196 for the 70 evaluations of a piece in the lower half of its cell, 3204 for 91 in the
+# upper half, 222 for 7 in the zero-velocity pass.  The face kernel counts the 1D evaluations.
+WENO1D_FLOP = 33
 FP32_LANES_PER_SM = 128
 SMS = 152
 L2_BYTES = 129 * 2 ** 20

@@ -7,6 +7,8 @@
 namespace fia {
 
 constexpr int kMaxGauss = 15;
+// bytes of a z-pass record of the FP32 form (fia_weno_rec.cuh): of the advected field, of psi
+constexpr int kRecBytes = 36, kPsiRecBytes = 32;
 
 // Triangulation of pieces above minimal_area bisects each triangle's longest edge
 // (facecutter.h:255-324).  Edges whose squared lengths agree to within this relative amount
@@ -61,8 +63,7 @@ enum StatusBits : unsigned {
 // clipped pieces of every face of a pass, contiguous per face, and per face its range.
 struct PieceStore {
     float4* rec = nullptr;       // (cx, cy, cz, ny): centroid in cells relative to the face anchor, y-normal
-    int* face = nullptr;         // family << 29 | face index
-    float* flux = nullptr;       // flux of each piece
+    int* face = nullptr;         // family << 29 | face index; after the quadrature the piece's flux (its bits)
     int2* range[3] = {nullptr, nullptr, nullptr};   // per face: start, nfwd | nrev << 15 | multi << 30
     float2* normal[3] = {nullptr, nullptr, nullptr};  // per face: y-normal sums of both clips (lower, upper cell)
     unsigned* count = nullptr;   // device counters: [0] pieces, [1] faces listed for the local-memory clipper
@@ -107,6 +108,8 @@ struct PassWork {
     cudaEvent_t* prof_ev;   // 2 * prof_cap events, or null
     int* prof_n;            // pairs recorded so far
     int prof_cap;
+    void* arec = nullptr;           // FP32 form: z-pass records of the advected field and of psi (fia_weno_rec.cuh)
+    void* prec = nullptr;
     PieceStore* pieces = nullptr;   // FP32 form only
     PieceStore64* pieces64 = nullptr;   // FP64 form: the piece pipeline; null: one thread per face (k_faces)
 };

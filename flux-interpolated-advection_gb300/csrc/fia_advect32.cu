@@ -18,6 +18,7 @@
 #include "fia_advect.cuh"
 #include "fia_local.cuh"
 #include "fia_clip32.cuh"
+#include "fia_weno_rec.cuh"
 
 #include <algorithm>
 
@@ -157,74 +158,163 @@ __global__ void k_forward32(PassDesc d, const float* __restrict__ u, const float
 // ---------------------------------------------------------------------------------
 // faces
 // ---------------------------------------------------------------------------------
-// The quadrature of one piece (polygon_3D.cpp:257-487): density points on the y-interval
-// below the centroid and one psi point; returns the number of 1D WENO6 evaluations.
+// One record per node row and stencil base (fia_weno_rec.cuh): of the advected field, and of psi
+// (WenoNewton; the pairs' differences, free of psi's magnitude).  One thread per record, coalesced
+// in both directions: bound by the 32 or 36 bytes written.
+template <bool PSI>
+__global__ void k_records_newton(NodeField F, const void* __restrict__ field, float4* __restrict__ rec) {
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= weno_rec_count(F)) return;
+    const long long row = id / (F.Mz + 1);
+    const int b = (int)(id - row * (F.Mz + 1)) - 1;
+    float f[6], lo[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const long long n = row * F.Mz + clampi(b - 2 + i, F.Mz - 1);
+        if (PSI) {
+            const float2 v = __ldg(static_cast<const float2*>(field) + n);
+            f[i] = v.x; lo[i] = v.y;
+        } else {
+            f[i] = __ldg(static_cast<const float*>(field) + n);
+        }
+    }
+    float D[5];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) D[i] = PSI ? (f[i + 1] - f[i]) + (lo[i + 1] - lo[i]) : f[i + 1] - f[i];
+    const WenoRec<float> r = weno_record(f[2], D[0], D[1], D[2], D[3], D[4]);
+    rec[2 * id] = make_float4(r.f, r.d, r.s1, r.s2);
+    rec[2 * id + 1] = make_float4(r.t0, r.t2, r.q0, r.q2);
+}
+__global__ void k_records_samples(NodeField F, const float* __restrict__ field, float4* __restrict__ rec,
+                                  float* __restrict__ rec2) {
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= weno_rec_count(F)) return;
+    const long long row = id / (F.Mz + 1);
+    const int b = (int)(id - row * (F.Mz + 1)) - 1;
+    float f[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) f[i] = __ldg(field + row * F.Mz + clampi(b - 2 + i, F.Mz - 1));
+    const Weno6Data w = weno6_data(f);
+    rec[2 * id] = make_float4(f[0], f[1], f[2], f[3]);
+    rec[2 * id + 1] = make_float4(f[4], f[5], w.r0, w.r1);
+    rec2[id] = w.r2;
+}
+
+// The y-interval below a piece's centroid (polygon_3D.cpp:275-286): the y-face ylo = fl + oy and
+// the fraction f of the cell up to the centroid.  The density points are k on [ylo, cy] when f <
+// 1/2, else k on each of [ylo, ylo + 1/2] and [ylo + 1/2, cy].
+struct YSpan {
+    float ylo, f;
+    int fl;
+};
+__device__ __forceinline__ YSpan y_span(const PassDesc& d, float cy) {
+    const float oy = (d.comp == 1) ? -0.5f : 0.f;
+    const float r = snap_int(cy - oy);
+    const float fl = floorf(r);
+    return YSpan{fl + oy, r - fl, (int)fl};
+}
+
 constexpr int kQuadThreads = 128;
 
-__device__ int piece_quad32(const PassDesc& d, const int* anc, float cx, float cy, float cz, float ny,
-                            const float* __restrict__ a, const PsiLoad& pl, Kahan& F, float* zs) {
-    const PlainLoad al{a};
-    const float invh = d.invhf;   // psi carries a length; the face terms are per cell volume
-    int evals = 0;
-    if (d.use_integral) {
-        const float oy = (d.comp == 1) ? -0.5f : 0.f;
-        const float r = snap_int(cy - oy);
-        const float fl = floorf(r);
-        const float f = r - fl;
-        const float ylo = fl + oy;   // local y of the y-face below the centroid
-        // the density quadrature points (polygon_3D.cpp:286-453): k on [ylo, cy] when the
-        // centroid is in the lower half of the cell, else k on each of [ylo, ylo+1/2], [ylo+1/2, cy];
-        // point m is generated on demand (no per-thread arrays)
-        const bool two = !(f < 0.5f);
-        const float lo0 = ylo, hl0 = two ? 0.25f : (cy - ylo) * 0.5f, wf0 = two ? ny * 0.5f : ny * f;
-        const float lo1 = ylo + 0.5f, hl1 = (cy - lo1) * 0.5f, wf1 = ny * (f - 0.5f);
-        const int k = d.k, np = two ? 2 * k : k;
-        auto point = [&](int m, float& y, float& w) {
-            const bool second = m >= k;
-            const int q = second ? m - k : m;
-            const float hl = second ? hl1 : hl0;
-            y = hl * d.gxf[q] + hl + (second ? lo1 : lo0);
-            w = (second ? wf1 : wf0) * d.gwf[q];
-        };
-        bool shared = false;
-        if (d.interp == INTERP_WENO6) {
-            const int n1d = weno6_ycolumn<kQuadThreads>(al, d.A, anc, cx, cz, ylo, cy, np, point, F, zs);
-            shared = n1d > 0;
-            evals += n1d;          // 1D WENO6 evaluations executed
-        }
-        if (!shared) {
-            for (int m = 0; m < np; ++m) {
-                float y, w;
-                point(m, y, w);
-                const float qq[3] = {cx, y, cz};
-                F.add(interp_loc(d.interp, al, d.A, anc, qq) * w);
-            }
-            if (d.interp == INTERP_WENO6) evals += 43 * np;
-        }
-        // the psi point lies on the psi node row of the y-face below the centroid
-        const float qp[3] = {cx, ylo, cz};
-        float v;
-        const int n1d = d.interp == INTERP_WENO6 ? weno6_3d_noderow<kQuadThreads>(pl, d.P, anc, qp, v, zs) : 0;
-        if (n1d == 0) {
-            v = interp_loc(d.interp, pl, d.P, anc, qp);
-            if (d.interp == INTERP_WENO6) evals += 43;
-        }
-        evals += n1d;
-        F.add(v * (ny * invh));
-    } else {
+// The WENO6 quadrature of one piece (polygon_3D.cpp:257-487); returns the number of 1D WENO6
+// evaluations.  The advected field's nodes sit half a cell from the y-faces, so the points of
+// one half share their six y-rows, the points of the other half the rows one further up.
+//
+// Density: bound by the L1 data path (86% busy; issue slots 64%, 16 warps per SM by registers): a
+// piece reads 42 + 6 records of 32 bytes, and the lanes of a warp spread over several cells.  One
+// launch on the main pass at 128^3 (18.6M pieces): 4.99 ms evaluating every 1D interpolant from its
+// samples, 2.22 ms now; a density step's launches at 256^3: 44.5 -> 21.4 ms.  Measured beside it:
+// five CTAs per SM 2.88 against 2.58 ms a step (spills), three 2.84; the records as two planes of
+// 16 bytes 2.50 (but 21.8 against 21.3 ms at 256^3); the pieces of a warp's faces interleaved
+// in the store 2.67, with planes 2.48 and 21.7.
+// Velocity: by its registers and FP32 issue (psi from its samples, coefficients of 12 words); the
+// launches of a velocity step on 120 x 161 x 77 cells: 11.95 -> 7.47 ms.  Two points of a half at a
+// time 8.13, three 8.6 (spills), three CTAs per SM 8.3.
+template <class W>
+__device__ __forceinline__ int piece_quad32(const PassDesc& d, const int* anc, float cx, float cy, float cz, float ny,
+                                            const typename W::Records& ar, const float4* __restrict__ prec,
+                                            const PsiLoad& pl, Kahan& F, float* zs) {
+    const float nyh = ny * d.invhf;   // psi carries a length; the face terms are per cell volume
+    int bx, bz;
+    float sx, sz;
+    locate(anc[0], cx, d.A.oxf, bx, sx);     // psi has the field's x and z offsets
+    locate(anc[2], cz, d.A.ozf, bz, sz);
+    const typename W::Coef kz = W::coef(sz);
+    if (!d.use_integral) {
         // psi at the centroid; on an unmoved y-face (the zero-velocity pass) the centroid lies
         // on a psi node row
-        const float qp[3] = {cx, cy, cz};
-        float v;
-        const int n1d = d.interp == INTERP_WENO6 ? weno6_3d_noderow<kQuadThreads>(pl, d.P, anc, qp, v, zs) : 0;
-        if (n1d == 0) {
-            v = interp_loc(d.interp, pl, d.P, anc, qp);
-            if (d.interp == INTERP_WENO6) evals += 43;
+        int by;
+        float sy;
+        locate(anc[1], cy, d.P.oyf, by, sy);
+        if (sy == 0.f) {
+            F.add(psi_noderow<W>(W::psi_rows(prec, pl, d.P.Mz, bz), d.P, bx, by, kz, W::coef(sx)) * nyh);
+            return 7;
         }
-        evals += n1d;
-        F.add(v * (ny * invh));
+        const float q[3] = {cx, cy, cz};
+        F.add(weno6_3d_loc(pl, d.P, anc, q) * nyh);
+        return 43;
     }
-    return evals;
+    const YSpan Y = y_span(d, cy);
+    const bool two = !(Y.f < 0.5f);
+    const int jlo = anc[1] + Y.fl;             // the y-face below the centroid: psi row jlo
+    rec_zpass<W, kQuadThreads>(ar, d.A, bx, clampi(bz + 1, d.A.Mz), jlo - 1, kz, zs);
+    const typename W::Coef kx = W::coef(sx);
+    const int k = d.k;
+#pragma unroll 1
+    for (int half = 0; half < (two ? 2 : 1); ++half) {
+        const float lo = half ? Y.ylo + 0.5f : Y.ylo;
+        const float hl = half ? (cy - lo) * 0.5f : (two ? 0.25f : (cy - Y.ylo) * 0.5f);
+        const float wf = half ? ny * (Y.f - 0.5f) : (two ? ny * 0.5f : ny * Y.f);
+        const float base = float(Y.fl - 1 + half);   // the half's third row, relative to the anchor
+#pragma unroll 1
+        for (int q0 = 0; q0 < k; q0 += W::kGroup) {
+            const int n = min(W::kGroup, k - q0);
+            typename W::Coef ky[W::kGroup];
+#pragma unroll
+            for (int q = 0; q < W::kGroup; ++q) {
+                const float y = hl * d.gxf[q < n ? q0 + q : q0] + hl + lo;
+                ky[q] = W::coef((y - d.A.oyf) - base);
+            }
+            float v[W::kGroup];
+            rec_yx<W, kQuadThreads>(zs, half, ky, n, kx, v);
+#pragma unroll
+            for (int q = 0; q < W::kGroup; ++q)
+                if (q < n) F.add(v[q] * (wf * d.gwf[q0 + q]));
+        }
+    }
+    // the psi point lies on the psi node row of the y-face below the centroid
+    F.add(psi_noderow<W>(W::psi_rows(prec, pl, d.P.Mz, bz), d.P, bx, jlo, kz, kx) * nyh);
+    return two ? 49 + 14 * k : 49 + 7 * k;
+}
+
+// The same with linear interpolation (main passes with interpolation_method linear) or linear in
+// y with the nearest column (the error pass).
+template <int METHOD, class L>
+__device__ __forceinline__ float linear_loc(const L& load, const NodeField& F, const int* anc, const float* q) {
+    return METHOD == INTERP_LINEAR ? lin3d_loc(load, F, anc, q) : lin1dy_loc(load, F, anc, q);
+}
+template <int METHOD>
+__device__ __forceinline__ void piece_quad32_linear(const PassDesc& d, const int* anc, float cx, float cy, float cz,
+                                                    float ny, const float* __restrict__ a, const PsiLoad& pl, Kahan& F) {
+    const PlainLoad al{a};
+    float yp = cy;
+    if (d.use_integral) {
+        const YSpan Y = y_span(d, cy);
+        const bool two = !(Y.f < 0.5f);
+        const int k = d.k, np = two ? 2 * k : k;
+        for (int m = 0; m < np; ++m) {
+            const bool second = m >= k;
+            const int q = second ? m - k : m;
+            const float lo = second ? Y.ylo + 0.5f : Y.ylo;
+            const float hl = second ? (cy - lo) * 0.5f : (two ? 0.25f : (cy - Y.ylo) * 0.5f);
+            const float w = (second ? ny * (Y.f - 0.5f) : (two ? ny * 0.5f : ny * Y.f)) * d.gwf[q];
+            const float qq[3] = {cx, hl * d.gxf[q] + hl + lo, cz};
+            F.add(linear_loc<METHOD>(al, d.A, anc, qq) * w);
+        }
+        yp = Y.ylo;
+    }
+    const float qp[3] = {cx, yp, cz};
+    F.add(linear_loc<METHOD>(pl, d.P, anc, qp) * (ny * d.invhf));
 }
 
 __device__ __forceinline__ void corners(int fam, int i, int j, int k, int* ci, int* cj, int* ck) {
@@ -252,6 +342,11 @@ __device__ __forceinline__ int2* range_of(const PieceStore& ps, int fam) {
 }
 __device__ __forceinline__ float2* normal_of(const PieceStore& ps, int fam) {
     return fam == 0 ? ps.normal[0] : (fam == 1 ? ps.normal[1] : ps.normal[2]);
+}
+
+// a face's range word: pieces of the lower cell's clip and of the upper cell's, second clip or not
+__device__ __forceinline__ int range_bits(int nfwd, int nrev, bool multi) {
+    return nfwd | (nrev << 15) | ((multi ? 1 : 0) << 30);
 }
 
 // Face pipeline of the chosen form, per pass:
@@ -369,7 +464,7 @@ __global__ void __launch_bounds__(kClipThreads, 4) k_clip32(PassDesc d, int fam,
         }
         // a range beyond the capacity is kept as it is: the host sees the count, grows the
         // store and runs the pass again
-        range_of(ps, fam)[id] = make_int2((int)start, nfwd | ((cnt - nfwd) << 15) | ((multi ? 1 : 0) << 30));
+        range_of(ps, fam)[id] = make_int2((int)start, range_bits(nfwd, cnt - nfwd, multi));
     }
     warp_counters((unsigned long long)npieces, ok ? 1u : 0u, (ok && multi) ? 1u : 0u, 0u, lane, status, counters);
 }
@@ -413,7 +508,7 @@ __global__ void __launch_bounds__(128) k_clip32_deferred(PassDesc d, const float
         if (valid) {
             if (start + cnt <= ps.cap)
                 for (int q = 0; q < cnt; ++q) { ps.rec[start + q] = sink.p[q]; ps.face[start + q] = tag; }
-            range_of(ps, fam)[id] = make_int2((int)start, nfwd | ((cnt - nfwd) << 15) | ((multi ? 1 : 0) << 30));
+            range_of(ps, fam)[id] = make_int2((int)start, range_bits(nfwd, cnt - nfwd, multi));
         }
         warp_counters((unsigned long long)npieces, valid ? 1u : 0u, (unsigned)nmulti, st, lane, status, counters);
     }
@@ -445,7 +540,7 @@ __global__ void k_rest_clip32(PassDesc d, int fam, PieceStore ps) {
         Nr = sink.ny.value();
     }
     reinterpret_cast<int4*>(ps.rest)[0] =
-        make_int4(sink.n, nfwd | ((sink.n - nfwd) << 15) | ((multi ? 1 : 0) << 30), npieces, (int)st);
+        make_int4(sink.n, range_bits(nfwd, sink.n - nfwd, multi), npieces, (int)st);
     ps.rest[1] = make_float4(N, Nr, 0.f, 0.f);
     for (int q = 0; q < sink.n; ++q) ps.rest[2 + q] = sink.p[q];
 }
@@ -473,25 +568,64 @@ __global__ void k_rest_fill32(PassDesc d, int fam, PieceStore ps, unsigned* stat
     normal_of(ps, fam)[id] = make_float2(nr.x, nr.y);
 }
 
-__global__ void __launch_bounds__(kQuadThreads, 4) k_quad32(PassDesc d, const float* __restrict__ a,
-                                                         const float2* __restrict__ psi, PieceStore ps, long long npc,
-                                                         unsigned long long* counters) {
-    __shared__ float zcol[48 * kQuadThreads];   // each thread's z- and y-pass column (weno6_ycolumn)
-    unsigned long long ec = 0;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < npc; t += (long long)gridDim.x * blockDim.x) {
-        const float4 p = ps.rec[t];
-        const int tag = ps.face[t];
-        const int fam = tag >> 29;
-        int anc[3];
-        face_of32(fam, d.A, (unsigned)(tag & ((1 << 29) - 1)), anc[0], anc[1], anc[2]);
-        const float2 b = __ldg(psi + psi_node(d.P, anc[0], anc[1], anc[2]));
-        const PsiLoad pl{psi, b.x, b.y};
-        Kahan F;
-        ec += (unsigned long long)piece_quad32(d, anc, p.x, p.y, p.z, p.w, a, pl, F, zcol + threadIdx.x);
-        ps.flux[t] = F.value();
+// Tiles of kQuadThreads pieces, `run` consecutive ones at a time per CTA: pieces are stored
+// nearly in face order, so a run covers neighbouring z-lines and finds their records in L1.
+// The next tile's piece is loaded before the present one is integrated.  Each piece's flux takes
+// the place of its face tag.
+template <class Body>
+__device__ __forceinline__ void for_pieces(const PassDesc& d, const PieceStore& ps, long long npc, int run, const Body& body) {
+    const long long ntile = (npc + kQuadThreads - 1) / kQuadThreads;
+    long long tile = (long long)blockIdx.x * run;
+    int left = run;
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    long long t = tile * kQuadThreads + threadIdx.x;
+    bool on = tile < ntile && t < npc;
+    float4 p = on ? ps.rec[t] : none;
+    int tag = on ? ps.face[t] : 0;
+    while (tile < ntile) {
+        if (--left > 0) ++tile;
+        else { left = run; tile += (long long)(gridDim.x - 1) * run + 1; }
+        const long long tn = tile * kQuadThreads + threadIdx.x;
+        const bool next = tile < ntile && tn < npc;
+        const float4 pn = next ? ps.rec[tn] : none;
+        const int tagn = next ? ps.face[tn] : 0;
+        if (on) {
+            int anc[3];
+            face_of32(tag >> 29, d.A, (unsigned)(tag & ((1 << 29) - 1)), anc[0], anc[1], anc[2]);
+            ps.face[t] = __float_as_int(body(p, anc));
+        }
+        p = pn; tag = tagn; t = tn; on = next;
     }
+}
+
+template <class W>
+__global__ void __launch_bounds__(kQuadThreads, 4) k_quad32(PassDesc d, typename W::Records ar,
+                                                            const float4* __restrict__ prec,
+                                                            const float2* __restrict__ psi, PieceStore ps, long long npc,
+                                                            int run, unsigned long long* counters) {
+    __shared__ float zcol[42 * kQuadThreads];   // each thread's z-pass column (rec_zpass)
+    unsigned long long ec = 0;
+    for_pieces(d, ps, npc, run, [&](const float4& p, const int* anc) {
+        const float2 b = __ldg(psi + psi_node(d.P, anc[0], anc[1], anc[2]));
+        Kahan F;
+        ec += (unsigned long long)piece_quad32<W>(d, anc, p.x, p.y, p.z, p.w, ar, prec, PsiLoad{psi, b.x, b.y}, F,
+                                                  zcol + threadIdx.x);
+        return F.value();
+    });
     for (int o = 16; o > 0; o >>= 1) ec += __shfl_down_sync(0xffffffffu, ec, o);
     if ((threadIdx.x & 31) == 0 && ec) atomicAdd(&counters[3], ec);
+}
+
+template <int METHOD>
+__global__ void __launch_bounds__(kQuadThreads) k_quad32_linear(PassDesc d, const float* __restrict__ a,
+                                                                const float2* __restrict__ psi, PieceStore ps,
+                                                                long long npc, int run) {
+    for_pieces(d, ps, npc, run, [&](const float4& p, const int* anc) {
+        const float2 b = __ldg(psi + psi_node(d.P, anc[0], anc[1], anc[2]));
+        Kahan F;
+        piece_quad32_linear<METHOD>(d, anc, p.x, p.y, p.z, p.w, a, PsiLoad{psi, b.x, b.y}, F);
+        return F.value();
+    });
 }
 
 // flux = wgt (F, N) (acc = 0) or flux + wgt (F, N) (acc = 1): the weighted faces of the flux
@@ -507,8 +641,8 @@ __global__ void k_facesum32(PassDesc d, int fam, PieceStore ps, float2* __restri
     const int nf = r.y & 0x7fff, nr = (r.y >> 15) & 0x7fff;
     const bool multi = (r.y >> 30) & 1;
     Kahan F, Fr;
-    for (int q = 0; q < nf; ++q) F.add(ps.flux[(long long)r.x + q]);
-    for (int q = 0; q < nr; ++q) Fr.add(ps.flux[(long long)r.x + nf + q]);
+    for (int q = 0; q < nf; ++q) F.add(__int_as_float(ps.face[(long long)r.x + q]));
+    for (int q = 0; q < nr; ++q) Fr.add(__int_as_float(ps.face[(long long)r.x + nf + q]));
     const float f = F.value(), fr = multi ? Fr.value() : -f;
     const float2 nrm = normal_of(ps, fam)[id];
     float2 a = make_float2(wgt * f, wgt * nrm.x), b = make_float2(wgt * fr, wgt * nrm.y);
@@ -647,8 +781,20 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
     }
     if ((long long)npc > ps.cap) return cudaErrorMemoryAllocation;
     if (npc > 0) {
+        const long long ntile = ((long long)npc + kQuadThreads - 1) / kQuadThreads;
+        const unsigned grid = (unsigned)std::min<long long>(ntile, 152 * 8);
+        const int run = (int)std::max<long long>(1, std::min<long long>(8, ntile / (4 * grid)));
         prof_mark(w, 0, s);
-        k_quad32<<<152 * 8, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, w.counters);
+        if (d.interp == INTERP_WENO6 && d.comp < 0)
+            k_quad32<WenoNewton><<<grid, kQuadThreads, 0, s>>>(d, newton_records(d.A, w.arec), (const float4*)w.prec, psi,
+                                                               ps, (long long)npc, run, w.counters);
+        else if (d.interp == INTERP_WENO6)
+            k_quad32<WenoSamples><<<grid, kQuadThreads, 0, s>>>(d, sample_records(d.A, w.arec), nullptr, psi, ps,
+                                                                (long long)npc, run, w.counters);
+        else if (d.interp == INTERP_LINEAR)
+            k_quad32_linear<INTERP_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, run);
+        else
+            k_quad32_linear<INTERP_1DY_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, run);
         prof_mark(w, 1, s);
     }
     for (int fam = 0; fam < 3; ++fam)
@@ -668,6 +814,19 @@ cudaError_t run_pass<float>(const PassDesc& d64, const VelocityFields& vel64, co
     float2* psi = (float2*)w.psi;
     const long long cols = (long long)d.A.Mx * d.A.Mz;
     k_psi32<<<nblk(cols, 128), 128, 0, s>>>(d, a, psi);
+    if (d.interp == INTERP_WENO6) {
+        // without the y-integral no point of the field itself is interpolated
+        if (d.comp >= 0) {
+            const WenoSamples::Records r = sample_records(d.A, w.arec);
+            if (d.use_integral)
+                k_records_samples<<<nblk(weno_rec_count(d.A), 256), 256, 0, s>>>(d.A, a, const_cast<float4*>(r.r),
+                                                                                 const_cast<float*>(r.r2));
+        } else {
+            if (d.use_integral)
+                k_records_newton<false><<<nblk(weno_rec_count(d.A), 256), 256, 0, s>>>(d.A, a, (float4*)w.arec);
+            k_records_newton<true><<<nblk(weno_rec_count(d.P), 256), 256, 0, s>>>(d.P, psi, (float4*)w.prec);
+        }
+    }
     const long long nv = (long long)(d.A.Mx + 1) * (d.A.My + 1) * (d.A.Mz + 1);
     if (!d.zero_velocity)
         k_backtrace32<<<nblk(nv, 128), 128, 0, s>>>(d, (const float*)vel.u, (const float*)vel.v, (const float*)vel.w,
@@ -704,11 +863,10 @@ cudaError_t run_pass<float>(const PassDesc& d64, const VelocityFields& vel64, co
 cudaError_t piece_store_reserve(PieceStore& p, long long pieces, long long faces_per_family) {
     cudaDeviceSynchronize();
     if (pieces > p.cap) {
-        cudaFree(p.rec); cudaFree(p.face); cudaFree(p.flux);
-        p.rec = nullptr; p.face = nullptr; p.flux = nullptr; p.cap = 0;
+        cudaFree(p.rec); cudaFree(p.face);
+        p.rec = nullptr; p.face = nullptr; p.cap = 0;
         cudaError_t e = cudaMalloc(&p.rec, pieces * sizeof(float4));
         if (e == cudaSuccess) e = cudaMalloc(&p.face, pieces * sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc(&p.flux, pieces * sizeof(float));
         if (e != cudaSuccess) return e;
         p.cap = pieces;
     }
@@ -731,7 +889,7 @@ cudaError_t piece_store_reserve(PieceStore& p, long long pieces, long long faces
 }
 
 void piece_store_free(PieceStore& p) {
-    cudaFree(p.rec); cudaFree(p.face); cudaFree(p.flux); cudaFree(p.count); cudaFree(p.deferred); cudaFree(p.rest);
+    cudaFree(p.rec); cudaFree(p.face); cudaFree(p.count); cudaFree(p.deferred); cudaFree(p.rest);
     cudaFree(p.saved);
     for (int f = 0; f < 3; ++f) { cudaFree(p.range[f]); cudaFree(p.normal[f]); }
     p = PieceStore();

@@ -33,6 +33,7 @@ struct fia_session {
     void* vel[3]; void* vel_next[3];
     void* cbuf;                  // correction field (pass 2 result)
     void* psi; void* verts; void* flux[3]; void* flux_rev[3];
+    void* arec; void* prec;      // FP32 form: z-pass records of the advected field and of psi
     void* verts2 = nullptr;      // flux MacCormack: the vertices traced back (allocated on first use)
     // cell-volume correction (allocated on first use): per-face y n_y sums, cell volumes, the
     // right-hand side and the potential of its Poisson solve
@@ -241,6 +242,7 @@ PassWork<T> work(fia_session* s) {
     w.prof_ev = s->prof_ev.empty() ? nullptr : s->prof_ev.data();
     w.prof_n = &s->prof_n;
     w.prof_cap = (int)(s->prof_ev.size() / 2);
+    w.arec = s->arec; w.prec = s->prec;
     w.pieces = &s->pieces;
     w.pieces64 = (s->precision == FIA_FP64 && s->piece_pipeline) ? &s->pieces64 : nullptr;
     return w;
@@ -971,6 +973,8 @@ fia_session* fia_create(int nx, int ny, int nz, double cell_length, int precisio
     A(s->rho, fb); A(s->rho_next, fb); A(s->pres, fb); A(s->cbuf, (size_t)big * 8); A(s->psi, pb);
     for (int c = 0; c < 3; ++c) { A(s->vel[c], fb); A(s->vel_next[c], fb); A(s->flux[c], pb); A(s->flux_rev[c], pb); }
     A(s->verts, 3 * fb);
+    s->arec = s->prec = nullptr;
+    if (precision == FIA_FP32C) { A(s->arec, (size_t)big * kRecBytes); A(s->prec, (size_t)big * kPsiRecBytes); }
     s->verts_bytes = fb;
     for (int q = 0; q < 5; ++q) A(s->pw[q], fb);
     { void* t2; A(t2, 4 * sizeof(unsigned)); s->ticket = (unsigned*)t2; }

@@ -98,34 +98,83 @@ __device__ __forceinline__ WenoCoef<T> weno_coef(const T* t) {
 // (no term in the samples themselves survives: the indicators are shift invariant).  In
 // FP32 the sample-product form cancels to an absolute error of ~1e-3 f^2, far above the
 // 1e-6 regularisation; the difference form keeps full relative accuracy and costs less.
+//
+// FP32 form, split into what depends on the six samples alone (Weno6Data) and the interpolant at
+// a position (weno6_at).  The indicators in Horner form, all three (and eps) scaled by 180, which
+// cancels in the normalised weights, with 180 eps as the start of each chain; then alpha_i = C_i
+// r_i^2 with r_i = 1/e_i (approximate reciprocals, 1 ulp) and one approximate division by the
+// weight sum.  All e_i carry a factor 2^-10, which no rounding and no quotient sees: the alpha_i
+// are 2^20 larger and stay normal numbers for sample differences up to 1e10.  Products that could
+// be fused into either of two terms are written out, so that every kernel that evaluates in this
+// form rounds alike.
+struct Weno6Data {
+    float f0, f1, f2, D0, D1, D2, S0, S1, S2, T0, T1, T2;   // samples, first to third differences
+    float r0, r1, r2;
+};
+// 1/x to 1 ulp for indicators and weight sums (normal numbers; 0 for x > 2^126)
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// a x - b y, the second product rounded
+__device__ __forceinline__ float prod_diff(float a, float x, float b, float y) { return fmaf(a, x, -__fmul_rn(b, y)); }
+__device__ __forceinline__ void weno6_recips(float D0, float D1, float D2, float D3, float D4, float& r0, float& r1,
+                                             float& r2) {
+    constexpr float K = 1.f / 1024.f;
+    const float eps180 = 0.00018f * K;
+    const float w2 = __fmul_rn(814.f * K, D2);
+    const float e0 = fmaf(D0, fmaf(683.f * K, D2, prod_diff(244.f * K, D0, 1171.f * K, D1)),
+                          fmaf(D1, prod_diff(1561.f * K, D1, 1951.f * K, D2), fmaf(w2, D2, eps180)));
+    const float e1 = fmaf(D1, fmaf(293.f * K, D3, prod_diff(244.f * K, D1, 781.f * K, D2)),
+                          fmaf(D2, prod_diff(961.f * K, D2, 781.f * K, D3), fmaf(__fmul_rn(244.f * K, D3), D3, eps180)));
+    const float e2 = fmaf(D2, fmaf(683.f * K, D4, fmaf(-1951.f * K, D3, w2)),
+                          fmaf(D3, prod_diff(1561.f * K, D3, 1171.f * K, D4), fmaf(__fmul_rn(244.f * K, D4), D4, eps180)));
+    r0 = rcp_approx(e0); r1 = rcp_approx(e1); r2 = rcp_approx(e2);
+}
+// differences of six samples, the r_i left to the caller
+__device__ __forceinline__ Weno6Data weno6_differences(const float* f, float& D3, float& D4) {
+    Weno6Data w;
+    w.f0 = f[0]; w.f1 = f[1]; w.f2 = f[2];
+    w.D0 = f[1] - f[0]; w.D1 = f[2] - f[1]; w.D2 = f[3] - f[2];
+    D3 = f[4] - f[3]; D4 = f[5] - f[4];
+    w.S0 = w.D1 - w.D0; w.S1 = w.D2 - w.D1; w.S2 = D3 - w.D2;
+    w.T0 = w.S1 - w.S0; w.T1 = w.S2 - w.S1; w.T2 = (D4 - D3) - w.S2;
+    return w;
+}
+__device__ __forceinline__ Weno6Data weno6_data(const float* f) {
+    float D3, D4;
+    Weno6Data w = weno6_differences(f, D3, D4);
+    weno6_recips(w.D0, w.D1, w.D2, D3, D4, w.r0, w.r1, w.r2);
+    return w;
+}
+// the interpolant at a position as a quotient num * rcp
+__device__ __forceinline__ void weno6_quotient(const Weno6Data& d, const WenoCoef<float>& w, float& num, float& rcp) {
+    const float P0 = fmaf(d.T0, w.c[0], fmaf(d.S0, w.b[0], fmaf(d.D0, w.a[0], d.f0)));
+    const float P1 = fmaf(d.T1, w.c[1], fmaf(d.S1, w.b[1], fmaf(d.D1, w.a[1], d.f1)));
+    const float P2 = fmaf(d.T2, w.c[2], fmaf(d.S2, w.b[2], fmaf(d.D2, w.a[2], d.f2)));
+    const float a0 = __fmul_rn(__fmul_rn(w.C[0], d.r0), d.r0), a1 = __fmul_rn(__fmul_rn(w.C[1], d.r1), d.r1);
+    const float a2 = __fmul_rn(__fmul_rn(w.C[2], d.r2), d.r2);
+    num = fmaf(a2, P2, fmaf(a1, P1, __fmul_rn(a0, P0)));
+    rcp = rcp_approx(__fadd_rn(__fadd_rn(a0, a1), a2));
+}
+__device__ __forceinline__ float weno6_at(const Weno6Data& d, const WenoCoef<float>& w) {
+    float num, rcp;
+    weno6_quotient(d, w, num, rcp);
+    return __fmul_rn(num, rcp);
+}
+
 template <typename T, bool FASTDIV = false>
 __device__ __forceinline__ T weno6_eval(const T* f, const WenoCoef<T>& w) {
-    const T D0 = f[1] - f[0], D1 = f[2] - f[1], D2 = f[3] - f[2], D3 = f[4] - f[3], D4 = f[5] - f[4];
-    const T S0 = D1 - D0, S1 = D2 - D1, S2 = D3 - D2;      // second differences
-    const T D[3] = {D0, D1, D2}, S[3] = {S0, S1, S2};
-    const T Tt[3] = {S1 - S0, S2 - S1, (D4 - D3) - S2};    // third differences
-    T P[3];
+    if constexpr (FASTDIV) return weno6_at(weno6_data(f), w);
+    else {
+        const T D0 = f[1] - f[0], D1 = f[2] - f[1], D2 = f[3] - f[2], D3 = f[4] - f[3], D4 = f[5] - f[4];
+        const T S0 = D1 - D0, S1 = D2 - D1, S2 = D3 - D2;      // second differences
+        const T D[3] = {D0, D1, D2}, S[3] = {S0, S1, S2};
+        const T Tt[3] = {S1 - S0, S2 - S1, (D4 - D3) - S2};    // third differences
+        T P[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) P[i] = f[i] + D[i] * w.a[i] + S[i] * w.b[i] + Tt[i] * w.c[i];
-    if constexpr (FASTDIV) {
-        // FP32 form: the indicators in Horner form, all three (and eps) scaled by 180, which
-        // cancels in the normalised weights, with 180 eps as the start of each chain; then
-        // alpha_i = C_i r_i^2 with r_i = 1/e_i (approximate reciprocals, 1 ulp) and one
-        // approximate division by the weight sum.  Range: e_i >= 180 eps = 1.8e-4, so
-        // r_i^2 <= 3.1e7; for sample differences of order 1 the e_i stay far below the 1e19
-        // at which r_i^2 would leave the normal range.
-        const T eps180 = T(0.00018);
-        const T w2 = T(814) * D2;
-        const T e0 = fmaf(D0, T(244) * D0 - T(1171) * D1 + T(683) * D2,
-                          fmaf(D1, T(1561) * D1 - T(1951) * D2, fmaf(w2, D2, eps180)));
-        const T e1 = fmaf(D1, T(244) * D1 - T(781) * D2 + T(293) * D3,
-                          fmaf(D2, T(961) * D2 - T(781) * D3, fmaf(T(244) * D3, D3, eps180)));
-        const T e2 = fmaf(D2, w2 - T(1951) * D3 + T(683) * D4,
-                          fmaf(D3, T(1561) * D3 - T(1171) * D4, fmaf(T(244) * D4, D4, eps180)));
-        const T r0 = __fdividef(T(1), e0), r1 = __fdividef(T(1), e1), r2 = __fdividef(T(1), e2);
-        const T a0 = (w.C[0] * r0) * r0, a1 = (w.C[1] * r1) * r1, a2 = (w.C[2] * r2) * r2;
-        return __fdividef(fmaf(a2, P[2], fmaf(a1, P[1], a0 * P[0])), (a0 + a1) + a2);
-    } else {
+        for (int i = 0; i < 3; ++i) P[i] = f[i] + D[i] * w.a[i] + S[i] * w.b[i] + Tt[i] * w.c[i];
         const T r180 = T(1) / T(180);
         const T b0 = (T(244) * D0 * D0 - T(1171) * D0 * D1 + T(683) * D0 * D2 + T(1561) * D1 * D1
                       - T(1951) * D1 * D2 + T(814) * D2 * D2) * r180;

@@ -38,13 +38,6 @@ __device__ __forceinline__ float2 weno6_call2(const float* a, const float* b, co
     return weno6_f2(a[0], a[1], a[2], a[3], a[4], a[5], b[0], b[1], b[2], b[3], b[4], b[5], w);
 }
 
-// Two evaluations with shared coefficients, inlined: for a loop whose body is one pair (the
-// z-pass of the quadrature kernel), so one copy of the code serves the whole loop and the
-// coefficients stay in registers across its iterations.
-__device__ __forceinline__ float2 weno6_pair(const float* a, const float* b, const WenoCoef<float>& w) {
-    return make_float2(weno6_eval<float, true>(a, w), weno6_eval<float, true>(b, w));
-}
-
 // error-free sum of two floats (Knuth TwoSum)
 __host__ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     s = a + b;
@@ -65,15 +58,11 @@ struct Kahan {
 };
 
 // Loads node values as floats: plain array, or psi pairs relative to a base pair.
-// row(i) gives a row pointer; at(row, k) the value k nodes further along the row (k a
-// compile-time constant in an unrolled loop, so one load with an immediate offset).
 // Node offsets are 32-bit: fia_create admits grids with (nx+2)(ny+2)(nz+2) <= 2^31, which
 // bounds every node field of the path.
 struct PlainLoad {
     const float* __restrict__ a;
     __device__ __forceinline__ float operator()(int i) const { return __ldg(a + i); }
-    __device__ __forceinline__ const float* row(int i) const { return a + i; }
-    __device__ __forceinline__ float at(const float* p, int k) const { return __ldg(p + k); }
 };
 struct PsiLoad {
     const float2* __restrict__ a;
@@ -82,27 +71,7 @@ struct PsiLoad {
         const float2 v = __ldg(a + i);
         return (v.x - hi0) + (v.y - lo0);
     }
-    __device__ __forceinline__ const float2* row(int i) const { return a + i; }
-    __device__ __forceinline__ float at(const float2* p, int k) const {
-        const float2 v = __ldg(p + k);
-        return (v.x - hi0) + (v.y - lo0);
-    }
 };
-
-// the six z-values of two stencil rows: row pointers and immediate offsets when the z-stencil
-// lies inside the field (zin), else the clamped indices kk
-template <class L>
-__device__ __forceinline__ void load_rows(const L& load, int row0, int row1, bool zin, int bz,
-                                          const int* kk, float* f0, float* f1) {
-    if (zin) {
-        const auto p0 = load.row(row0 + bz - 2), p1 = load.row(row1 + bz - 2);
-#pragma unroll
-        for (int iz = 0; iz < 6; ++iz) { f0[iz] = load.at(p0, iz); f1[iz] = load.at(p1, iz); }
-    } else {
-#pragma unroll
-        for (int iz = 0; iz < 6; ++iz) { f0[iz] = load(row0 + kk[iz]); f1[iz] = load(row1 + kk[iz]); }
-    }
-}
 
 // stencil base and fractional offset of the local position along one axis
 __device__ __forceinline__ void locate(int anchor, float q, float off, int& base, float& s) {
@@ -152,91 +121,6 @@ __device__ float weno6_3d_loc(const L& load, const NodeField& F, const int* anc,
         yv[ix] = weno6_call(zv, cy);
     }
     return weno6_call(yv, cx);
-}
-
-// WENO6 at npts points that share x and z and lie within one cell in y (the density
-// quadrature points of one piece, polygon_3D.cpp:286-453): the z-pass over the 6 x 7
-// (x, y) stencil rows is done once and shared; each point then needs 6 y- and 1 x-
-// evaluation instead of 43.  Bit-identical to evaluating the points one by one.  The points
-// come from point(m, y, w) and lie in [ya, yb]; returns the number of 1D evaluations made, or
-// 0 (nothing accumulated) if [ya, yb] spans more than one cell of the field.
-// The 6 x 7 z-pass results live in shared memory, zs[(7 ix + r) * stride] (the calling
-// thread's column of a block-wide array, stride = threads per block, 48 words: in registers
-// they held 42 of the face kernel's 128); a point's six y-pass results stay in registers.
-template <int STRIDE, class L, class P>
-__device__ int weno6_ycolumn(const L& load, const NodeField& F, const int* anc, float qx, float qz, float ya,
-                             float yb, int npts, const P& point, Kahan& acc, float* zs) {
-    int bx, bz, by0, by1;
-    float sx, sz, s;
-    locate(anc[0], qx, F.oxf, bx, sx);
-    locate(anc[2], qz, F.ozf, bz, sz);
-    locate(anc[1], ya, F.oyf, by0, s);
-    locate(anc[1], yb, F.oyf, by1, s);
-    if (by1 - by0 > 1) return 0;
-    const bool seven = by1 > by0;
-    float tx[6], tz[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) { tx[i] = sx + float(2 - i); tz[i] = sz + float(2 - i); }
-    const WenoCoef<float> cx = weno_coef(tx), cz = weno_coef(tz);
-    int kk[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) kk[i] = clampi(bz - 2 + i, F.Mz - 1);
-    const int nr = seven ? 7 : 6;
-    const bool zin = bz >= 2 && bz + 3 <= F.Mz - 1;
-#pragma unroll 1
-    for (int ix = 0; ix < 6; ix += 2) {
-        const int i0 = clampi(bx - 2 + ix, F.Mx - 1), i1 = clampi(bx - 1 + ix, F.Mx - 1);
-        float* z0 = zs + 7 * ix * STRIDE;
-        float* z1 = z0 + 7 * STRIDE;
-        // two rows per iteration: two independent pairs of evaluations in flight
-        int r = 0;
-#pragma unroll 1
-        for (; r + 1 < nr; r += 2) {
-            const int ja = clampi(by0 - 2 + r, F.My - 1), jb = clampi(by0 - 1 + r, F.My - 1);
-            float fa0[6], fa1[6], fb0[6], fb1[6];
-            load_rows(load, F.Mz * (F.My * i0 + ja), F.Mz * (F.My * i1 + ja), zin, bz, kk, fa0, fa1);
-            load_rows(load, F.Mz * (F.My * i0 + jb), F.Mz * (F.My * i1 + jb), zin, bz, kk, fb0, fb1);
-            const float2 va = weno6_pair(fa0, fa1, cz);
-            const float2 vb = weno6_pair(fb0, fb1, cz);
-            z0[r * STRIDE] = va.x; z1[r * STRIDE] = va.y;
-            z0[(r + 1) * STRIDE] = vb.x; z1[(r + 1) * STRIDE] = vb.y;
-        }
-        if (r < nr) {
-            const int jj = clampi(by0 - 2 + r, F.My - 1);
-            const int row0 = F.Mz * (F.My * i0 + jj), row1 = F.Mz * (F.My * i1 + jj);
-            float f0[6], f1[6];
-            load_rows(load, row0, row1, zin, bz, kk, f0, f1);
-            const float2 v = weno6_pair(f0, f1, cz);
-            z0[r * STRIDE] = v.x; z1[r * STRIDE] = v.y;
-        }
-    }
-    for (int m = 0; m < npts; ++m) {
-        float y, w;
-        point(m, y, w);
-        int by;
-        float sy;
-        locate(anc[1], y, F.oyf, by, sy);
-        const bool up = by > by0;
-        float ty[6];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) ty[i] = sy + float(2 - i);
-        const WenoCoef<float> cy = weno_coef(ty);
-        const float* zb = zs + (up ? STRIDE : 0);
-        float yv[6];
-#pragma unroll
-        for (int ix = 0; ix < 6; ix += 2) {
-            float f0[6], f1[6];
-#pragma unroll
-            for (int i = 0; i < 6; ++i) {
-                f0[i] = zb[(7 * ix + i) * STRIDE];
-                f1[i] = zb[(7 * ix + 7 + i) * STRIDE];
-            }
-            const float2 v = weno6_pair(f0, f1, cy);
-            yv[ix] = v.x; yv[ix + 1] = v.y;
-        }
-        acc.add(weno6_eval<float, true>(yv, cx) * w);
-    }
-    return (seven ? 42 : 36) + 7 * npts;
 }
 
 template <class L>
@@ -289,47 +173,6 @@ __device__ float lin1dy_loc(const L& load, const NodeField& F, const int* anc, c
     const float f0 = load(F.Mz * (F.My * ix + clampi(by, F.My - 1)) + iz);
     const float f1 = load(F.Mz * (F.My * ix + clampi(by + 1, F.My - 1)) + iz);
     return (1.f - sy) * f0 + sy * f1;
-}
-
-// WENO6 at a point whose y lies on a node row of F (fractional offset exactly 0, as for the
-// psi point of a piece, which sits on the y-face below the centroid).  Every candidate
-// polynomial of the y-pass interpolates that node and the weights sum to one, so the y-pass
-// returns the row's value: the interpolant is the (x, z) WENO6 of the row, 7 evaluations
-// instead of 43, equal to the full form in exact arithmetic.  Returns the number of 1D
-// evaluations, or 0 (out untouched) if y is not on a node row.  The six z-pass results pass
-// through words 42-47 of the thread's shared column zs (as in weno6_ycolumn).
-template <int STRIDE, class L>
-__device__ int weno6_3d_noderow(const L& load, const NodeField& F, const int* anc, const float* q, float& out,
-                                float* zs) {
-    int bx, by, bz;
-    float sx, sy, sz;
-    locate(anc[1], q[1], F.oyf, by, sy);
-    if (sy != 0.f) return 0;
-    locate(anc[0], q[0], F.oxf, bx, sx);
-    locate(anc[2], q[2], F.ozf, bz, sz);
-    float tx[6], tz[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) { tx[i] = sx + float(2 - i); tz[i] = sz + float(2 - i); }
-    const WenoCoef<float> cx = weno_coef(tx), cz = weno_coef(tz);
-    int kk[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) kk[i] = clampi(bz - 2 + i, F.Mz - 1);
-    const int jj = clampi(by, F.My - 1);
-    const bool zin = bz >= 2 && bz + 3 <= F.Mz - 1;
-#pragma unroll 1
-    for (int ix = 0; ix < 6; ix += 2) {
-        const int i0 = clampi(bx - 2 + ix, F.Mx - 1), i1 = clampi(bx - 1 + ix, F.Mx - 1);
-        const int row0 = F.Mz * (F.My * i0 + jj), row1 = F.Mz * (F.My * i1 + jj);
-        float f0[6], f1[6];
-        load_rows(load, row0, row1, zin, bz, kk, f0, f1);
-        const float2 v = weno6_pair(f0, f1, cz);
-        zs[(42 + ix) * STRIDE] = v.x; zs[(43 + ix) * STRIDE] = v.y;
-    }
-    float xv[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) xv[i] = zs[(42 + i) * STRIDE];
-    out = weno6_eval<float, true>(xv, cx);
-    return 7;
 }
 
 // WENO6 in which every axis whose fractional offset is exactly 0 is collapsed to its centre
