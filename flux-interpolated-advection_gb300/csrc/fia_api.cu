@@ -45,6 +45,7 @@ struct fia_session {
     double* part; double* scal; double* sums;
     unsigned* status; unsigned long long* counters;
     unsigned* ticket;            // last-block counters of the fused CG kernels
+    unsigned long long* slots;   // where the blocks of the one-kernel PCG meet
     double* red_part; double* red_out;
     std::vector<void*> allocations;
     // solids and the pinned pressure cell
@@ -433,7 +434,7 @@ template <typename T>
 PressureWork<T> pressure_work(fia_session* s) {
     PressureWork<T> W;
     W.p = (T*)s->pres; W.r = (T*)s->pw[0]; W.z = (T*)s->pw[1]; W.d = (T*)s->pw[2]; W.q = (T*)s->pw[3];
-    W.d2 = (T*)s->pw[4]; W.ticket = s->ticket;
+    W.d2 = (T*)s->pw[4]; W.ticket = s->ticket; W.slots = s->slots;
     W.part = s->part; W.scal = s->scal; W.sums = s->sums;
     return W;
 }
@@ -980,6 +981,7 @@ fia_session* fia_create(int nx, int ny, int nz, double cell_length, int precisio
     { void* t2; A(t2, 4 * sizeof(unsigned)); s->ticket = (unsigned*)t2; }
     void* t;
     A(t, pressure_partials() * sizeof(double)); s->part = (double*)t;
+    A(t, pressure_slots() * sizeof(unsigned long long)); s->slots = (unsigned long long*)t;
     A(t, kScalDoubles * sizeof(double)); s->scal = (double*)t;
     A(t, 8 * sizeof(double)); s->sums = (double*)t;
     A(t, sizeof(unsigned)); s->status = (unsigned*)t;

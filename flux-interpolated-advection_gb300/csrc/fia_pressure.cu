@@ -496,6 +496,337 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update(PoissonGrid g, double
     }
 }
 
+// ---------------------------------------------------------------------------------
+// Jacobi-PCG as one kernel
+// ---------------------------------------------------------------------------------
+// Many iterations per launch (cooperative; the blocks meet twice an iteration).  Block b owns the
+// cells [b chunk, (b + 1) chunk) in linear order and keeps d of them, and of one z-line on either
+// side, in shared memory; q, r and x of them too as far as they fit (NS arrays of the four).
+// Along y and z the operator reads shared memory; along x the neighbour's d = z + beta d_old is
+// formed from the z and d_old that its block stored before the last meeting, as in
+// k_cg_direction_apply.  The arithmetic on the vectors is that of the two kernels above, cell by
+// cell; only the order of the (FP64-accurate) dot sums differs.
+//
+// What an iteration costs is latency: FP64 operations run in one thread (one of every thread of a
+// block takes a quarter of a microsecond; the FP32 form adds its dots up as float pairs), the
+// neighbours' loads are issued before the block's own cells are updated, and what a group of cells
+// needs of its place in the grid is one word, made once.  Microseconds an iteration, with the two
+// kernels above and with this one: FP32 16^3 18 -> 7.0, 64^3 23 -> 10.7, 128^3 36 -> 18.7, 160^3 53 ->
+// 48, 176^3 71 -> 71; FP64 64^3 46 -> 18, 128^3 134 -> 79.  (Slots polled by every block, with the
+// meeting's number beside the value instead of a counter, were slower: 19.8 against 14 us at 64^3.)
+// Larger grids, whose chunks leave no room for two shared arrays, keep the two kernels: there the
+// vectors' traffic is the time (256^3: 152 us for 11 vectors of 67 MB, 108 us at the copy rate).
+constexpr int kPcgThreadsMax = 1024;
+constexpr int kPcgIters = 256;           // iterations per launch
+constexpr int kPcgSpinLimit = 1 << 21;   // polls of a meeting before the kernel gives up
+constexpr unsigned kPcgStuck = 1u << 30; // set in the counter when one did
+constexpr size_t kPcgSmem = 224 * 1024;  // dynamic shared memory of a block (227 KB less the static part)
+constexpr int kPcgPartWords = 3;         // 64-bit words a block: one value, then two
+constexpr int kPcgBlocksMax = 1024;
+constexpr unsigned kPcgOneBlock = 1024;  // groups that one block takes alone
+
+template <typename T>
+struct PcgArgs {
+    PoissonGrid g;
+    T *x, *r, *z, *d0, *d1;
+    double* scal;
+    unsigned long long* parts;   // kPcgPartWords * gridDim.x
+    unsigned* bar;               // arrivals, zero at launch
+    unsigned chunk;              // cells per block, a multiple of W
+    int iters;                   // at most this many iterations
+    int first;                   // no direction yet
+};
+
+template <typename T, int W>
+__device__ __forceinline__ void ldcgv(const T* p, T (&v)[W]) {
+    if constexpr (W == 4) {
+        const float4 t = __ldcg(reinterpret_cast<const float4*>(p));
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else if constexpr (W == 2) {
+        const double2 t = __ldcg(reinterpret_cast<const double2*>(p));
+        v[0] = t.x; v[1] = t.y;
+    } else {
+        v[0] = __ldcg(p);
+    }
+}
+
+// Place of a group of W cells: bits 0-5 the neighbours inside the grid (x-, x+, y-, y+, z- of the
+// first cell, z+ of the last), then 3 bits a cell: the diagonal of B, 7 where the cell is
+// excluded.  Excluded cells need no further care: their z and d are zero.
+template <int W>
+__device__ __forceinline__ unsigned pcg_place(const PoissonGrid& g, unsigned c) {
+    const Cell k = decode(c, g.ny, g.nz);
+    unsigned p = (k.ix > 0) | (k.ix < g.nx - 1) << 1 | (k.iy > 0) << 2 | (k.iy < g.ny - 1) << 3 | (k.iz > 0) << 4 |
+                 (k.iz + W < g.nz) << 5;
+#pragma unroll
+    for (int e = 0; e < W; ++e) p |= (excluded(g, c + e) ? 7u : (unsigned)diag_at<W>(g, c, k, e)) << (6 + 3 * e);
+    return p;
+}
+
+// Sums of accumulators, kept as accumulators (a float pair in the FP32 form, whose sums then need
+// no FP64 operation).
+__device__ __forceinline__ void acc_join(DotAcc<float>& a, float hi, float lo) {
+    const float s = __fadd_rn(a.hi, hi);
+    const float bb = __fsub_rn(s, a.hi);
+    const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(hi, bb));
+    a.hi = s;
+    a.lo = __fadd_rn(__fadd_rn(a.lo, lo), e);
+}
+__device__ __forceinline__ DotAcc<float> acc_warp(DotAcc<float> a) {
+    for (int o = 16; o > 0; o >>= 1)
+        acc_join(a, __shfl_down_sync(0xffffffffu, a.hi, o), __shfl_down_sync(0xffffffffu, a.lo, o));
+    return a;
+}
+__device__ __forceinline__ DotAcc<double> acc_warp(DotAcc<double> a) {
+    a.s = warp_sum(a.s);
+    return a;
+}
+
+// All blocks meet: publishes the block's NV sums of its threads' accumulators and returns their
+// sums over the blocks in tot[] (thread 0; every block adds them up in the same order).  What the
+// block's threads stored to global memory before is visible to every block after (loads past L1).
+// parts: NV words a block, not those of the meeting before.  False when the wait ran out.
+template <typename T, int NV>
+__device__ __forceinline__ bool pcg_meet(const DotAcc<T> (&acc)[NV], unsigned long long* parts, unsigned* bar,
+                                         unsigned target, double* tot) {
+    static_assert(sizeof(DotAcc<T>) == 8, "an accumulator is one 64-bit word");
+    __shared__ DotAcc<T> sh[NV][32];
+    __shared__ DotAcc<T> bsum[NV][kPcgBlocksMax / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, nb = gridDim.x;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        const DotAcc<T> t = acc_warp(acc[q]);
+        if (lane == 0) sh[q][warp] = t;
+    }
+    __syncthreads();
+    bool ok = true;
+    if (warp == 0) {
+        DotAcc<T> t[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) t[q] = acc_warp(lane < nw ? sh[q][lane] : DotAcc<T>());
+        if (lane == 0) {
+            if (nb == 1) {
+#pragma unroll
+                for (int q = 0; q < NV; ++q) tot[q] = t[q].value();
+            } else {
+#pragma unroll
+                for (int q = 0; q < NV; ++q)
+                    __stcg(parts + (size_t)q * nb + blockIdx.x, *reinterpret_cast<const unsigned long long*>(&t[q]));
+                unsigned seen;
+                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+                int it = 0;
+                do {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+                } while (seen < target && ++it < kPcgSpinLimit);
+                ok = seen >= target && seen < kPcgStuck;
+                if (!ok) atomicOr(bar, kPcgStuck);   // the others leave at once
+            }
+        }
+    }
+    if (nb == 1) return true;
+    if (!__syncthreads_and(ok)) return false;
+    const int per = (nb + 31) >> 5;
+    for (int job = warp; job < NV * per; job += nw) {
+        const int q = job / per, b = (job - q * per) * 32 + lane;
+        DotAcc<T> t;
+        if (b < nb) {
+            const unsigned long long w = __ldcg(parts + (size_t)q * nb + b);
+            t = *reinterpret_cast<const DotAcc<T>*>(&w);
+        }
+        t = acc_warp(t);
+        if (lane == 0) bsum[q][job - q * per] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            double t = 0.0;
+            for (int j = 0; j < per; ++j) t += bsum[q][j].value();
+            tot[q] = t;
+        }
+    }
+    return true;
+}
+
+// G > 0: at most G groups a thread, their places in registers; 0: any number, placed as visited
+template <typename T, int W, int NS, int G>
+__global__ void __launch_bounds__(kPcgThreadsMax) k_pcg(PcgArgs<T> A) {
+    extern __shared__ __align__(16) unsigned char pcg_smem[];
+    __shared__ double tot[2];
+    __shared__ T step;      // alpha, then beta
+    __shared__ int done;
+    __shared__ T inv[8];    // 1 / diagonal, 0 for excluded cells
+    const PoissonGrid g = A.g;
+    const unsigned n = (unsigned)g.nx * g.ny * g.nz, sx = (unsigned)g.ny * g.nz, sy = (unsigned)g.nz;
+    const unsigned c0 = blockIdx.x * A.chunk, c1 = min(n, c0 + A.chunk);
+    // shared cells [lo, hi): the chunk and a z-line either side (nz is a multiple of W)
+    const unsigned lo = c0 > sy ? c0 - sy : 0u, hi = min(n, c1 + sy);
+    T* sd = reinterpret_cast<T*>(pcg_smem);
+    T* own = sd + A.chunk + 2 * sy;
+    T* const sq = own;
+    T* const r = NS >= 3 ? own + A.chunk : A.r + c0;
+    T* const x = NS >= 4 ? own + 2 * (size_t)A.chunk : A.x + c0;
+    if (A.scal[S_DONE] != 0.0) return;
+    double rz = 0.0, beta_d = 0.0, rr = 0.0, its = 0.0, threshold = 0.0;   // thread 0
+    if (threadIdx.x == 0) {
+        rz = A.scal[S_RZ]; beta_d = A.scal[S_BETA]; rr = A.scal[S_RR]; its = A.scal[S_ITERS];
+        threshold = A.scal[S_THRESH];
+        step = (T)beta_d;
+        done = 0;
+    }
+    if (threadIdx.x < 8) inv[threadIdx.x] = threadIdx.x < 7 ? inv_count<T>((int)threadIdx.x) : T(0);
+    T* dold = A.d0;
+    T* dnew = A.d1;
+    const unsigned cstep = blockDim.x * W, cfirst = c0 + threadIdx.x * W;
+    unsigned places[G > 0 ? G : 1];
+    // f(cell, place) for every group of this thread
+    auto each = [&](auto&& f) {
+        if constexpr (G > 0) {
+#pragma unroll
+            for (int i = 0; i < G; ++i) {
+                const unsigned c = cfirst + i * cstep;
+                if (c < c1) f(c, places[i]);
+            }
+        } else {
+            for (unsigned c = cfirst; c < c1; c += cstep) f(c, pcg_place<W>(g, c));
+        }
+    };
+    if constexpr (G > 0) {
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            const unsigned c = cfirst + i * cstep;
+            places[i] = c < c1 ? pcg_place<W>(g, c) : 0u;
+        }
+    }
+    for (unsigned c = cfirst; c < c1; c += cstep) {
+        T v[W];
+        if (NS >= 3) { ldv<T, W>(A.r + c, v); stv<T, W>(r + (c - c0), v); }
+        if (NS >= 4) { ldv<T, W>(A.x + c, v); stv<T, W>(x + (c - c0), v); }
+        if (!A.first) { ldv<T, W>(dold + c, v); stv<T, W>(sd + (c - lo), v); }
+    }
+    __syncthreads();
+    bool first = A.first != 0;
+    unsigned target = 0;
+    for (int it = 0; it < A.iters && !done; ++it) {
+        const T beta = step;
+        // d of another block's group
+        auto far = [&](unsigned o, T (&v)[W]) {
+            ldcgv<T, W>(A.z + o, v);
+            if (!first) {
+                T b[W];
+                ldcgv<T, W>(dold + o, b);
+#pragma unroll
+                for (int e = 0; e < W; ++e) v[e] = fma(beta, b[e], v[e]);
+            }
+        };
+        auto near = [&](unsigned o) { return o >= lo && o < hi; };
+        // x-neighbours' part of the operator's sum; `late`: taken after the block's d are in place
+        auto xsum = [&](unsigned c, unsigned p, bool late, T (&s)[W]) {
+            const bool xm = p & 1u, xp = p & 2u;
+            const bool wait = (xm && near(c - sx)) || (xp && near(c + sx));
+            if (wait != late) return wait;
+            T a[W], b[W];
+#pragma unroll
+            for (int e = 0; e < W; ++e) { a[e] = T(0); b[e] = T(0); }
+            if (xm) { if (near(c - sx)) ldv<T, W>(sd + (c - sx - lo), a); else far(c - sx, a); }
+            if (xp) { if (near(c + sx)) ldv<T, W>(sd + (c + sx - lo), b); else far(c + sx, b); }
+#pragma unroll
+            for (int e = 0; e < W; ++e) s[e] = a[e] + b[e];
+            return wait;
+        };
+        // the z-lines either side
+        for (unsigned i = threadIdx.x * W; i < (c0 - lo) + (hi - c1); i += cstep) {
+            const unsigned c = i < c0 - lo ? lo + i : c1 + (i - (c0 - lo));
+            T v[W];
+            far(c, v);
+            stv<T, W>(sd + (c - lo), v);
+        }
+        // d = z + beta d_old, with z = r / diag as it was stored
+        each([&](unsigned c, unsigned p) {
+            T v[W], o[W], s[W];
+            if (!xsum(c, p, false, s)) stv<T, W>(sq + (c - c0), s);
+            ldv<T, W>(r + (c - c0), v);
+            if (!first) ldv<T, W>(sd + (c - lo), o);
+#pragma unroll
+            for (int e = 0; e < W; ++e) {
+                v[e] *= inv[(p >> (6 + 3 * e)) & 7u];
+                if (!first) v[e] = fma(beta, o[e], v[e]);
+            }
+            stv<T, W>(sd + (c - lo), v);
+            stv<T, W>(dnew + c, v);
+        });
+        __syncthreads();
+        // q = B d
+        DotAcc<T> dq[1];
+        each([&](unsigned c, unsigned p) {
+            T dc[W], s[W], a[W], b[W], q[W];
+            if (!xsum(c, p, true, s)) ldv<T, W>(sq + (c - c0), s);
+            ldv<T, W>(sd + (c - lo), dc);
+#pragma unroll
+            for (int e = 0; e < W; ++e) { a[e] = T(0); b[e] = T(0); }
+            if (p & 4u) ldv<T, W>(sd + (c - sy - lo), a);
+            if (p & 8u) ldv<T, W>(sd + (c + sy - lo), b);
+            const T zm = p & 16u ? sd[c - 1 - lo] : T(0), zp = p & 32u ? sd[c + W - lo] : T(0);
+#pragma unroll
+            for (int e = 0; e < W; ++e) {
+                s[e] += a[e];
+                s[e] += b[e];
+                s[e] += e > 0 ? dc[e > 0 ? e - 1 : 0] : zm;
+                s[e] += e < W - 1 ? dc[e < W - 1 ? e + 1 : 0] : zp;
+                const unsigned dg = (p >> (6 + 3 * e)) & 7u;
+                q[e] = dg == 7u ? T(0) : fma(T((int)dg), dc[e], -s[e]);
+                dq[0].add(dc[e], q[e]);
+            }
+            stv<T, W>(sq + (c - c0), q);
+        });
+        if (!pcg_meet<T, 1>(dq, A.parts, A.bar, target += gridDim.x, tot)) break;
+        if (threadIdx.x == 0) step = (T)(tot[0] != 0.0 ? rz / tot[0] : 0.0);
+        __syncthreads();
+        const T al = step;
+        DotAcc<T> acc[2];   // r.z, r.r
+        each([&](unsigned c, unsigned p) {
+            T xv[W], dv[W], rv[W], qv[W], zv[W];
+            ldv<T, W>(x + (c - c0), xv); ldv<T, W>(sd + (c - lo), dv);
+            ldv<T, W>(r + (c - c0), rv); ldv<T, W>(sq + (c - c0), qv);
+#pragma unroll
+            for (int e = 0; e < W; ++e) {
+                xv[e] = fma(al, dv[e], xv[e]);
+                rv[e] = fma(-al, qv[e], rv[e]);
+                zv[e] = rv[e] * inv[(p >> (6 + 3 * e)) & 7u];
+            }
+            stv<T, W>(A.z + c, zv);
+            stv<T, W>(x + (c - c0), xv);
+            stv<T, W>(r + (c - c0), rv);
+#pragma unroll
+            for (int e = 0; e < W; ++e) {
+                acc[1].add(rv[e], rv[e]);
+                acc[0].add(rv[e], zv[e]);
+            }
+        });
+        if (!pcg_meet<T, 2>(acc, A.parts + gridDim.x, A.bar, target += gridDim.x, tot)) break;
+        if (threadIdx.x == 0) {
+            beta_d = rz != 0.0 ? tot[0] / rz : 0.0;
+            rz = tot[0];
+            rr = tot[1];
+            its += 1.0;
+            step = (T)beta_d;
+            done = rr <= threshold;
+        }
+        __syncthreads();
+        T* t = dold; dold = dnew; dnew = t;
+        first = false;
+    }
+    for (unsigned c = cfirst; c < c1; c += cstep) {
+        T v[W];
+        if (NS >= 3) { ldv<T, W>(r + (c - c0), v); stv<T, W>(A.r + c, v); }
+        if (NS >= 4) { ldv<T, W>(x + (c - c0), v); stv<T, W>(A.x + c, v); }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        A.scal[S_BETA] = beta_d; A.scal[S_RZ] = rz; A.scal[S_RR] = rr; A.scal[S_ITERS] = its;
+        if (done) A.scal[S_DONE] = 1.0;
+    }
+}
+
 // flexible CG with m kept directions (Notay's FCG(m)):
 //   beta_j = -(z.q_j)/(d_j.q_j) for the kept directions j;  d = z + sum_j beta_j d_j;
 //   q = B d;  alpha = (d.r)/(d.q)
@@ -762,6 +1093,69 @@ cudaError_t pressure_rhs(const PressureWork<T>& W, const PoissonGrid& g, double 
     return cudaStreamSynchronize(s);
 }
 
+// Blocks, threads and shared arrays of k_pcg for a grid, or none (blocks 0: too large a chunk for
+// two shared arrays, or no cooperative launch).
+struct PcgPlan {
+    int blocks = 0, threads = 0, arrays = 0;
+    bool placed = false;    // groups' places in registers
+    unsigned chunk = 0;
+    size_t smem = 0;
+};
+template <typename T>
+PcgPlan pcg_plan(const PoissonGrid& g) {
+    PcgPlan p;
+    int dev = 0, sms = 0, coop = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
+        return p;
+    sms = std::min(sms, kPcgBlocksMax);
+    const unsigned n = (unsigned)g.nx * g.ny * g.nz, W = g.nz % VecW<T>::W == 0 ? VecW<T>::W : 1, groups = n / W;
+    // 512 groups a block in FP32, 256 in FP64 (64^3 FP32 10.7 against 11.2 us an iteration with 256;
+    // 20^3 FP64 11.6 against 13.9 with 512)
+    const unsigned least = sizeof(T) == 4 ? 512 : 256;
+    unsigned blocks = groups <= kPcgOneBlock ? 1u : std::min<unsigned>((unsigned)sms, (groups + least - 1) / least);
+    const unsigned chunk = (groups + blocks - 1) / blocks * W;
+    blocks = (n + chunk - 1) / chunk;
+    for (int a = 4; a >= 2; --a) {
+        const size_t smem = ((size_t)a * chunk + 2 * (size_t)g.nz) * sizeof(T);
+        if (smem > kPcgSmem) continue;
+        p.blocks = (int)blocks;
+        // a thread a group; in FP64, whose sums across a warp cost most, two where there are many
+        // (64^3 18.4 against 20.2 us an iteration)
+        const unsigned per = sizeof(T) == 8 && chunk / W > 512 ? 2 : 1;
+        p.threads = (int)std::min<unsigned>(kPcgThreadsMax, std::max<unsigned>(128u, (chunk / W / per + 31) / 32 * 32));
+        p.placed = chunk / W <= 4u * p.threads;
+        p.arrays = a; p.chunk = chunk; p.smem = smem;
+        return p;
+    }
+    return p;
+}
+
+template <typename T, int W, int NS, int G>
+cudaError_t launch_pcg_t(const PcgPlan& p, PcgArgs<T> A, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(k_pcg<T, W, NS, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPcgSmem);
+    int per_sm = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg<T, W, NS, G>, p.threads, p.smem);
+    if (e == cudaSuccess && per_sm < 1) e = cudaErrorCooperativeLaunchTooLarge;
+    if (e != cudaSuccess) return e;
+    void* args[] = {&A};
+    return cudaLaunchCooperativeKernel((const void*)k_pcg<T, W, NS, G>, dim3(p.blocks), dim3(p.threads), args, p.smem, s);
+}
+template <typename T, int W>
+cudaError_t launch_pcg_w(const PcgPlan& p, const PcgArgs<T>& A, cudaStream_t s) {
+    switch (p.arrays) {
+        case 4: return p.placed ? launch_pcg_t<T, W, 4, 4>(p, A, s) : launch_pcg_t<T, W, 4, 0>(p, A, s);
+        case 3: return p.placed ? launch_pcg_t<T, W, 3, 4>(p, A, s) : launch_pcg_t<T, W, 3, 0>(p, A, s);
+        default: return launch_pcg_t<T, W, 2, 0>(p, A, s);
+    }
+}
+template <typename T>
+cudaError_t launch_pcg(const PcgPlan& p, const PcgArgs<T>& A, cudaStream_t s) {
+    constexpr int V = VecW<T>::W;
+    return A.g.nz % V == 0 ? launch_pcg_w<T, V>(p, A, s) : launch_pcg_w<T, 1>(p, A, s);
+}
+
 template <typename T>
 cudaError_t pressure_pcg(const PressureWork<T>& W, const PoissonGrid& g, double bb, double rr0, double tol,
                          int max_iter, PressureReport* rep, cudaStream_t s) {
@@ -770,23 +1164,41 @@ cudaError_t pressure_pcg(const PressureWork<T>& W, const PoissonGrid& g, double 
     k_pcg_init<T><<<nb, nt, 0, s>>>(g, W.r, W.z, W.scal, tol * tol * bb, rr0, W.part, W.ticket);
     // iterations are enqueued in batches; the device flag turns the rest of a batch into
     // empty launches once the residual is below tolerance
+    PcgPlan plan = pcg_plan<T>(g);
     T* dold = W.d;
     T* dnew = W.d2;
     int launched = 0;
     double st[3] = {rr0 <= tol * tol * bb ? 1.0 : 0.0, 0.0, rr0};   // done, iterations, rr
     while (launched < max_iter && st[0] == 0.0) {
-        const int batch = std::min(kCgBatch, max_iter - launched);
-        for (int b = 0; b < batch; ++b) {
-            launch_direction<T>(W, g, dold, dnew, launched + b == 0, nullptr, W.part, W.ticket, s);
-            launch_update<T>(W, g, dnew, true, W.part + 2 * nb, W.ticket + 1, s);
-            std::swap(dold, dnew);
+        const int batch = std::min(plan.blocks ? kPcgIters : kCgBatch, max_iter - launched);
+        if (plan.blocks) {
+            cudaError_t e = cudaMemsetAsync(W.slots, 0, sizeof(unsigned long long), s);
+            const PcgArgs<T> A{g, W.p, W.r, W.z, dold, dnew, W.scal, W.slots + 1, (unsigned*)W.slots, plan.chunk, batch, launched == 0};
+            if (e == cudaSuccess) e = launch_pcg<T>(plan, A, s);
+            if (e == cudaErrorCooperativeLaunchTooLarge) {   // not all blocks fit at once: launch by launch
+                cudaGetLastError();
+                plan.blocks = 0;
+                continue;
+            }
+            if (e != cudaSuccess) return e;
+            if (batch & 1) std::swap(dold, dnew);
+            rep->launches += 1;
+        } else {
+            for (int b = 0; b < batch; ++b) {
+                launch_direction<T>(W, g, dold, dnew, launched + b == 0, nullptr, W.part, W.ticket, s);
+                launch_update<T>(W, g, dnew, true, W.part + 2 * nb, W.ticket + 1, s);
+                std::swap(dold, dnew);
+            }
+            rep->launches += 2 * batch;
         }
         launched += batch;
-        rep->launches += 2 * batch;
         double tail[4];
+        unsigned stuck = 0;
         cudaMemcpyAsync(tail, W.scal + S_RR, 4 * sizeof(double), cudaMemcpyDeviceToHost, s);
+        if (plan.blocks) cudaMemcpyAsync(&stuck, W.slots, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
         const cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return e;
+        if (stuck >= kPcgStuck) return cudaErrorLaunchTimeout;   // a meeting of k_pcg ran out
         st[0] = tail[S_DONE - S_RR]; st[1] = tail[S_ITERS - S_RR]; st[2] = tail[0];
     }
     rep->iterations = (int)st[1];
@@ -939,6 +1351,9 @@ cudaError_t subtract_gradient_p64(const double* p64, float* u, float* v, float* 
 
 // partial rows: the FCG dot kernel's kFcgMaxDirs + 1 and the direction kernel's 2 (the CG
 // kernels use fewer)
+// the arrival counter of k_pcg and its blocks' partial sums
+size_t pressure_slots() { return 1 + (size_t)kPcgBlocksMax * kPcgPartWords; }
+
 size_t pressure_partials() { return (size_t)kRedBlocks * (kFcgMaxDirs + 4); }
 
 #define FIA_PRESSURE_INST(T)                                                                                       \

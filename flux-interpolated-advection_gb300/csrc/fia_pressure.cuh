@@ -34,6 +34,7 @@ struct PressureWork {
     double* scal;               // kScalDoubles doubles (layout in fia_pressure.cu)
     double* sums;               // 4 doubles
     unsigned* ticket;           // 4 last-block counters (zero between kernels)
+    unsigned long long* slots;  // pressure_slots() words: where the blocks of k_pcg meet
 };
 
 struct PressureReport {
@@ -45,6 +46,7 @@ struct PressureReport {
 };
 
 size_t pressure_partials();
+size_t pressure_slots();
 
 // r = -b - B p (warm) or r = -b, p = 0 (cold), b = div(u) h, B = -A; |b|^2 and |r|^2 into
 // bb_rr_host[0..2) (synchronises the stream).
