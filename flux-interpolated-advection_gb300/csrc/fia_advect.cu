@@ -20,6 +20,7 @@
 //   k_gather     one thread per cell: rho' = (sum of the six signed face fluxes) / V.
 //                Deterministic, no atomics (the reference's per-thread += is racy).
 #include "fia_advect.cuh"
+#include "fia_weno_rec.cuh"
 
 #include <cmath>
 #include <vector>
@@ -324,100 +325,11 @@ __device__ __forceinline__ void piece_geom(const FaceGeom<T>& g, const T* px, co
     }
 }
 
-// weno6_3d_collapse at points that share x and z (the density quadrature points of a piece,
-// polygon_3D.cpp:286-453) and whose stencils start in two consecutive y rows: the z-pass of
-// the 6 x 7 (x, y) stencil rows is evaluated once into the thread's column zs (word
-// (7 ix + r) * stride, shared memory), and each point takes its y- and x-passes from it.  The
-// same evaluations on the same values as weno6_3d_collapse point by point, so the same results,
-// in 42 + 7 per point 1D evaluations instead of 43 per point.  point(m, y, w) gives point m in
-// [ya, yb]; acc += value * w in order.  A point whose row falls outside the column is evaluated
-// on its own.
-template <typename T, class Pt>
-__device__ void weno6_column(const T* __restrict__ a, const NodeField& F, T h, T px, T pz, T ya, T yb, int npts,
-                             const Pt& point, T& acc, T* zs, int stride) {
-    const T rx = (px - T(F.ox) * h) / h, rz = (pz - T(F.oz) * h) / h;
-    const T sx = snap_int(rx), sz = snap_int(rz);
-    const bool cxn = sx == rint(sx), czn = sz == rint(sz);
-    const int bx = cxn ? (int)sx : (int)floor(rx);
-    const int bz = czn ? (int)sz : (int)floor(rz);
-    auto row_of = [&](T py) {
-        const T ry = (py - T(F.oy) * h) / h;
-        const T sy = snap_int(ry);
-        return sy == rint(sy) ? (int)sy : (int)floor(ry);
-    };
-    const int by0 = row_of(ya);
-    const int nr = row_of(yb) > by0 ? 7 : 6;
-    T tx[6], tz[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        tx[i] = rx - T(bx - 2 + i);
-        tz[i] = rz - T(bz - 2 + i);
-    }
-    const WenoCoef<T> cx = weno_coef(tx), cz = weno_coef(tz);
-    int kk[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) kk[i] = clampi(bz - 2 + i, F.Mz - 1);
-    const int x0 = cxn ? 2 : 0, x1 = cxn ? 3 : 6;
-#pragma unroll 1
-    for (int ix = x0; ix < x1; ++ix) {
-        const int ii = clampi(bx - 2 + ix, F.Mx - 1);
-#pragma unroll 1
-        for (int r = 0; r < nr; ++r) {
-            const int jj = clampi(by0 - 2 + r, F.My - 1);
-            const T* row = a + (long long)F.Mz * ((long long)F.My * ii + jj);
-            T v;
-            if (czn) {
-                v = ldg(row + kk[2]);
-            } else {
-                T f[6];
-#pragma unroll
-                for (int iz = 0; iz < 6; ++iz) f[iz] = ldg(row + kk[iz]);
-                v = weno6_eval(f, cz);
-            }
-            zs[(7 * ix + r) * stride] = v;
-        }
-    }
-#pragma unroll 1
-    for (int m = 0; m < npts; ++m) {
-        T y, w;
-        point(m, y, w);
-        const T ry = (y - T(F.oy) * h) / h;
-        const T sy = snap_int(ry);
-        const bool cyn = sy == rint(sy);
-        const int by = cyn ? (int)sy : (int)floor(ry);
-        T val;
-        if (by < by0 || by - by0 > nr - 6) {
-            val = weno6_3d_collapse(a, F, h, px, y, pz);
-        } else {
-            T ty[6];
-#pragma unroll
-            for (int i = 0; i < 6; ++i) ty[i] = ry - T(by - 2 + i);
-            const WenoCoef<T> cy = weno_coef(ty);
-            const T* zb = zs + (by - by0) * stride;
-            T yv[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
-#pragma unroll 1
-            for (int ix = x0; ix < x1; ++ix) {
-                if (cyn) {
-                    yv[ix] = zb[(7 * ix + 2) * stride];
-                } else {
-                    T zv[6];
-#pragma unroll
-                    for (int iy = 0; iy < 6; ++iy) zv[iy] = zb[(7 * ix + iy) * stride];
-                    yv[ix] = weno6_eval(zv, cy);
-                }
-            }
-            val = cxn ? yv[2] : weno6_eval(yv, cx);
-        }
-        acc += val * w;
-    }
-}
-
-// The quadrature of one piece with centroid (cx, cy, cz) and y-normal ny (polygon_3D.cpp:257-487).
-// With a column zs (42 words at stride `stride`, see weno6_column) the WENO6 density points
-// share their z-pass.
+// The quadrature of one piece with centroid (cx, cy, cz) and y-normal ny (polygon_3D.cpp:257-487),
+// every value interpolated on its own.
 template <typename T>
 __device__ __forceinline__ T piece_quad(const PassDesc& d, T cx, T cy, T cz, T ny, const T* __restrict__ a,
-                                        const T* __restrict__ psi, T* zs = nullptr, int stride = 0) {
+                                        const T* __restrict__ psi) {
     if (ny == T(0)) return T(0);
     const T h = T(d.h);
     T F = T(0);
@@ -427,31 +339,7 @@ __device__ __forceinline__ T piece_quad(const PassDesc& d, T cx, T cy, T cz, T n
         const T ry = snap_int((cy - oy) / h);
         const int iy0 = (int)floor(ry);
         const T f = ry - T(iy0);
-        if (zs && d.interp == INTERP_WENO6 && !d.full_weno) {
-            // the same points, weights and order as below
-            const int k = d.k;
-            if (f < T(0.5)) {
-                const T lo = T(iy0) * h + oy, L = cy - lo;
-                auto pt = [&](int q, T& y, T& w) {
-                    y = (L / T(2)) * T(d.gx[q]) + (L / T(2)) + lo;
-                    w = ny * f * h * T(d.gw[q]);
-                };
-                weno6_column(a, d.A, h, cx, cz, lo, cy, k, pt, F, zs, stride);
-            } else {
-                const T lo0 = T(iy0) * h + oy, hi0 = (T(iy0) + T(0.5)) * h + oy, L0 = hi0 - lo0;
-                const T lo1 = (T(iy0) + T(0.5)) * h + oy, hi1 = (T(iy0) + f) * h + oy, L1 = hi1 - lo1;
-                auto pt = [&](int m, T& y, T& w) {
-                    if (m < k) {
-                        y = (L0 / T(2)) * T(d.gx[m]) + (L0 / T(2)) + lo0;
-                        w = ny * T(0.5) * h * T(d.gw[m]);
-                    } else {
-                        y = (L1 / T(2)) * T(d.gx[m - k]) + (L1 / T(2)) + lo1;
-                        w = ny * (f - T(0.5)) * h * T(d.gw[m - k]);
-                    }
-                };
-                weno6_column(a, d.A, h, cx, cz, lo0, hi1, 2 * k, pt, F, zs, stride);
-            }
-        } else if (f < T(0.5)) {
+        if (f < T(0.5)) {
             const T lo = T(iy0) * h + oy, L = cy - lo;
             for (int q = 0; q < d.k; ++q) {
                 const T yq = (L / T(2)) * T(d.gx[q]) + (L / T(2)) + lo;
@@ -862,14 +750,124 @@ __global__ void __launch_bounds__(128) k_clip64(PassDesc d, int fam, const doubl
 }
 
 constexpr int kQuad64Threads = 128;
+constexpr int kQuad64Group = 3;   // Gauss points of a half that share their y-stencil data
 
+// One record per node row and stencil base of a field (fia_weno_rec.cuh), of the advected field and
+// of psi alike.
+__global__ void k_records64(NodeField F, const double* __restrict__ field, WenoRec<double>* __restrict__ rec) {
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= weno_rec_count(F)) return;
+    const long long row = id / (F.Mz + 1);
+    const int b = (int)(id - row * (F.Mz + 1)) - 1;
+    double f[6];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) f[i] = __ldg(field + row * F.Mz + clampi(b - 2 + i, F.Mz - 1));
+    rec[id] = weno_record(f[2], f[1] - f[0], f[2] - f[1], f[3] - f[2], f[4] - f[3], f[5] - f[4]);
+}
+
+// stencil base and offset of a position (in cells from node 0) along one axis; a position within
+// rounding of a node sits on it
+__device__ __forceinline__ int base64(double r, double& s) {
+    const double sn = snap_int(r);
+    const int b = sn == rint(sn) ? (int)sn : (int)floor(r);
+    s = r - double(b);
+    return b;
+}
+
+// WENO6 of row (., j) at (x, z): 7 evaluations
+__device__ __forceinline__ double row64(const WenoRec<double>* __restrict__ rec, const NodeField& F, int bx, int b1, int j,
+                                        const WenoPos<double>& pz, const WenoPos<double>& px) {
+    double xv[6];
+#pragma unroll 1
+    for (int ix = 0; ix < 6; ++ix)
+        xv[ix] = weno_at(weno_unpack(ldg_rec(rec + ((long long)clampi(bx - 2 + ix, F.Mx - 1) * F.My + j) * (F.Mz + 1) + b1)), pz);
+    return weno_at(weno_data(xv), px);
+}
+
+// piece_quad with WENO6 from records: the z-pass of the 6 x 7 (x, y) stencil rows into the
+// thread's column zs, then, for each half of the cell below the centroid, the y-stencils' data
+// once for its Gauss points (as piece_quad32, fia_advect32.cu).  Bound by the FP64 pipe, and so by
+// its count of FP64 instructions: about 2400 a piece against 6500 with every 1D interpolant
+// formed from its samples; three passes of a 64^3 density step 51.1 -> 13.6 ms.
+__device__ __forceinline__ double piece_quad64(const PassDesc& d, double cx, double cy, double cz, double ny,
+                                               const WenoRec<double>* __restrict__ arec,
+                                               const WenoRec<double>* __restrict__ prec, const double* __restrict__ psi,
+                                               double* zs) {
+    const double h = d.h;
+    double sx, sz;
+    const int bx = base64((cx - d.A.ox * h) / h, sx);
+    const int b1 = clampi(base64((cz - d.A.oz * h) / h, sz) + 1, d.A.Mz);
+    const WenoPos<double> px = weno_pos(sx), pz = weno_pos(sz);
+    if (!d.use_integral) {
+        double sy;
+        const int by = base64((cy - d.P.oy * h) / h, sy);
+        if (fabs(sy) < 1e-9 && snap_int((cy - d.P.oy * h) / h) == double(by))   // a face at rest
+            return row64(prec, d.P, bx, b1, clampi(by, d.P.My - 1), pz, px) * ny;
+        return weno6_3d_collapse(psi, d.P, h, cx, cy, cz) * ny;
+    }
+    const double oy = (d.comp == 1) ? -0.5 * h : 0.0;
+    const double ry = snap_int((cy - oy) / h);
+    const int iy0 = (int)floor(ry);
+    const double f = ry - double(iy0);
+    const bool two = !(f < 0.5);
+#pragma unroll 1
+    for (int ix = 0; ix < 6; ++ix) {
+        const int row0 = clampi(bx - 2 + ix, d.A.Mx - 1) * d.A.My;
+#pragma unroll 1
+        for (int r = 0; r < 7; ++r) {
+            const int row = row0 + clampi(iy0 - 3 + r, d.A.My - 1);
+            zs[(7 * ix + r) * kQuad64Threads] =
+                weno_at(weno_unpack(ldg_rec(arec + (long long)row * (d.A.Mz + 1) + b1)), pz);
+        }
+    }
+    const int k = d.k;
+    double F = 0.0;
+#pragma unroll 1
+    for (int half = 0; half < (two ? 2 : 1); ++half) {
+        const double len = half ? f - 0.5 : (two ? 0.5 : f);   // of the interval, in cells
+        const double s0 = half ? 0.0 : 0.5;                    // its lower end past the third row of its stencil
+        const double wf = ny * len * h;
+#pragma unroll 1
+        for (int q0 = 0; q0 < k; q0 += kQuad64Group) {
+            const int n = min(kQuad64Group, k - q0);
+            double s[kQuad64Group], yv[kQuad64Group][6];
+#pragma unroll
+            for (int q = 0; q < kQuad64Group; ++q) s[q] = s0 + (0.5 * len) * (d.gx[q < n ? q0 + q : q0] + 1.0);
+#pragma unroll
+            for (int ix = 0; ix < 6; ++ix) {
+                double v[6];
+#pragma unroll
+                for (int i = 0; i < 6; ++i) v[i] = zs[(7 * ix + i + half) * kQuad64Threads];
+                const WenoData<double> w = weno_data(v);
+#pragma unroll
+                for (int q = 0; q < kQuad64Group; ++q)
+                    if (q < n) yv[q][ix] = weno_at(w, weno_pos(s[q]));
+            }
+#pragma unroll
+            for (int q = 0; q < kQuad64Group; ++q)
+                if (q < n) F += weno_at(weno_data(yv[q]), px) * (wf * d.gw[q0 + q]);
+        }
+    }
+    return F + row64(prec, d.P, bx, b1, clampi(iy0, d.P.My - 1), pz, px) * ny;
+}
+
+// a piece's flux takes the place of its centroid's x
 __global__ void __launch_bounds__(kQuad64Threads) k_quad64(PassDesc d, const double* __restrict__ a,
                                                            const double* __restrict__ psi, PieceStore64 ps,
                                                            long long npc) {
-    __shared__ double zcol[42 * kQuad64Threads];   // each thread's z-pass column (weno6_column)
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < npc; t += (long long)gridDim.x * blockDim.x) {
         const double4_32a p = ps.rec[t];
-        ps.flux[t] = piece_quad(d, p.x, p.y, p.z, p.w, a, psi, zcol + threadIdx.x, kQuad64Threads);
+        ps.rec[t].x = piece_quad(d, p.x, p.y, p.z, p.w, a, psi);
+    }
+}
+__global__ void __launch_bounds__(kQuad64Threads) k_quad64_weno(PassDesc d, const WenoRec<double>* __restrict__ arec,
+                                                                const WenoRec<double>* __restrict__ prec,
+                                                                const double* __restrict__ psi, PieceStore64 ps,
+                                                                long long npc) {
+    __shared__ double zcol[42 * kQuad64Threads];   // each thread's z-pass column
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < npc; t += (long long)gridDim.x * blockDim.x) {
+        const double4_32a p = ps.rec[t];
+        ps.rec[t].x = p.w == 0.0 ? 0.0 : piece_quad64(d, p.x, p.y, p.z, p.w, arec, prec, psi, zcol + threadIdx.x);
     }
 }
 
@@ -885,14 +883,14 @@ __global__ void k_facesum64(PassDesc d, int fam, PieceStore64 ps, double* __rest
     const bool multi = (r.y >> 30) & 1;
     double F = 0.0, V = 0.0;
     for (int q = 0; q < nf; ++q) {
-        F += ps.flux[(long long)r.x + q];
+        F += ps.rec[(long long)r.x + q].x;
         if (fvol) { const double4_32a p = ps.rec[(long long)r.x + q]; V += p.y * p.w; }
     }
     double Fr = -F, Vr = -V;
     if (multi) {
         Fr = 0.0; Vr = 0.0;
         for (int q = nf; q < nf + nr; ++q) {
-            Fr += ps.flux[(long long)r.x + q];
+            Fr += ps.rec[(long long)r.x + q].x;
             if (fvol) { const double4_32a p = ps.rec[(long long)r.x + q]; Vr += p.y * p.w; }
         }
     }
@@ -993,6 +991,12 @@ static cudaError_t launch_faces_from(const PassDesc& d, const T* a, const PassWo
     return cudaGetLastError();
 }
 
+// WENO6 from records: where the pass interpolates with it, unless every evaluation is wanted in
+// full or the records found no memory (fia_create)
+static bool weno_records64(const PassDesc& d, const PassWork<double>& w) {
+    return w.pieces64 && w.arec && w.prec && d.interp == INTERP_WENO6 && !d.full_weno;
+}
+
 // One face stage of the piece pipeline: clip (growing the store and clipping again when it is
 // too small), per-piece quadrature, per-face sums weighted into the face fluxes.
 static cudaError_t face_stage64(const PassDesc& d, const double* a, const PassWork<double>& w, const double* verts,
@@ -1026,7 +1030,11 @@ static cudaError_t face_stage64(const PassDesc& d, const double* a, const PassWo
     if (npc > 0) {
         const long long nb = std::min<long long>(blocks_for(npc, kQuad64Threads), 152LL * 16);
         prof_mark(w, 0, s);
-        k_quad64<<<(unsigned)nb, kQuad64Threads, 0, s>>>(d, a, w.psi, ps, (long long)npc);
+        if (weno_records64(d, w))
+            k_quad64_weno<<<(unsigned)nb, kQuad64Threads, 0, s>>>(d, (const WenoRec<double>*)w.arec,
+                                                                  (const WenoRec<double>*)w.prec, w.psi, ps, (long long)npc);
+        else
+            k_quad64<<<(unsigned)nb, kQuad64Threads, 0, s>>>(d, a, w.psi, ps, (long long)npc);
         prof_mark(w, 1, s);
     }
     for (int fam = 0; fam < 3; ++fam)
@@ -1068,10 +1076,9 @@ cudaError_t piece_store64_reserve(PieceStore64& p, long long pieces, long long f
     // ranges hold 31-bit starts
     if (pieces >= (1LL << 31)) pieces = (1LL << 31) - 1;
     if (pieces > p.cap) {
-        cudaFree(p.rec); cudaFree(p.flux);
-        p.rec = nullptr; p.flux = nullptr; p.cap = 0;
+        cudaFree(p.rec);
+        p.rec = nullptr; p.cap = 0;
         cudaError_t e = cudaMalloc(&p.rec, pieces * sizeof(double4_32a));
-        if (e == cudaSuccess) e = cudaMalloc(&p.flux, pieces * sizeof(double));
         if (e != cudaSuccess) return e;
         p.cap = pieces;
     }
@@ -1092,7 +1099,7 @@ cudaError_t piece_store64_reserve(PieceStore64& p, long long pieces, long long f
 }
 
 void piece_store64_free(PieceStore64& p) {
-    cudaFree(p.rec); cudaFree(p.flux); cudaFree(p.count); cudaFree(p.deferred); cudaFree(p.saved);
+    cudaFree(p.rec); cudaFree(p.count); cudaFree(p.deferred); cudaFree(p.saved);
     for (int f = 0; f < 3; ++f) cudaFree(p.range[f]);
     p = PieceStore64();
 }
@@ -1110,6 +1117,13 @@ cudaError_t run_pass(const PassDesc& d, const VelocityFields& vel, const T* a, c
                      const T* in, T* out, int mode, cudaStream_t s) {
     cudaError_t e = launch_psi<T>(d, a, w.psi, s);
     if (e != cudaSuccess) return e;
+    if constexpr (sizeof(T) == sizeof(double)) {
+        if (weno_records64(d, w)) {
+            if (d.use_integral)
+                k_records64<<<blocks_for(weno_rec_count(d.A), 256), 256, 0, s>>>(d.A, a, (WenoRec<double>*)w.arec);
+            k_records64<<<blocks_for(weno_rec_count(d.P), 256), 256, 0, s>>>(d.P, w.psi, (WenoRec<double>*)w.prec);
+        }
+    }
     if (!d.zero_velocity) {
         e = launch_backtrace<T>(d, vel, w.verts, s);
         if (e != cudaSuccess) return e;

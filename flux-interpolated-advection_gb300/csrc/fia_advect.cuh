@@ -7,8 +7,8 @@
 namespace fia {
 
 constexpr int kMaxGauss = 15;
-// bytes of a z-pass record of the FP32 form (fia_weno_rec.cuh): of the advected field, of psi
-constexpr int kRecBytes = 36, kPsiRecBytes = 32;
+// bytes of a z-pass record (fia_weno_rec.cuh): FP32 form, of the advected field and of psi; FP64 form
+constexpr int kRecBytes = 36, kPsiRecBytes = 32, kRecBytes64 = 64;
 
 // Triangulation of pieces above minimal_area bisects each triangle's longest edge
 // (facecutter.h:255-324).  Edges whose squared lengths agree to within this relative amount
@@ -80,8 +80,8 @@ void piece_store_free(PieceStore& p);
 // Pieces of the plain form's face pipeline (clip -> per-piece quadrature -> per-face sum),
 // as PieceStore: every face's pieces contiguous, in emission order, forward clip first.
 struct PieceStore64 {
-    double4_32a* rec = nullptr;      // (cx, cy, cz, ny): centroid (absolute), y component of the scaled normal
-    double* flux = nullptr;      // flux of each piece
+    double4_32a* rec = nullptr;      // (cx, cy, cz, ny): centroid (absolute), y component of the scaled normal;
+                                     //   after the quadrature the flux in the place of cx
     int2* range[3] = {nullptr, nullptr, nullptr};   // per face: start, nfwd | nrev << 15 | multi << 30
     unsigned* count = nullptr;   // device counters: [0] pieces appended, [1] faces listed for whole-face evaluation
     int* deferred = nullptr;     // those faces (family << 29 | face index), room for every face
@@ -108,7 +108,7 @@ struct PassWork {
     cudaEvent_t* prof_ev;   // 2 * prof_cap events, or null
     int* prof_n;            // pairs recorded so far
     int prof_cap;
-    void* arec = nullptr;           // FP32 form: z-pass records of the advected field and of psi (fia_weno_rec.cuh)
+    void* arec = nullptr;           // z-pass records of the advected field and of psi (fia_weno_rec.cuh)
     void* prec = nullptr;
     PieceStore* pieces = nullptr;   // FP32 form only
     PieceStore64* pieces64 = nullptr;   // FP64 form: the piece pipeline; null: one thread per face (k_faces)

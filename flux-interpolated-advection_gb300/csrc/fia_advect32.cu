@@ -287,15 +287,18 @@ __device__ __forceinline__ int piece_quad32(const PassDesc& d, const int* anc, f
     return two ? 49 + 14 * k : 49 + 7 * k;
 }
 
-// The same with linear interpolation (main passes with interpolation_method linear) or linear in
-// y with the nearest column (the error pass).
+// The same with every value interpolated on its own: linear interpolation (main passes with
+// interpolation_method linear), linear in y with the nearest column (the error pass), WENO6 where
+// the records found no memory.
 template <int METHOD, class L>
-__device__ __forceinline__ float linear_loc(const L& load, const NodeField& F, const int* anc, const float* q) {
-    return METHOD == INTERP_LINEAR ? lin3d_loc(load, F, anc, q) : lin1dy_loc(load, F, anc, q);
+__device__ __forceinline__ float plain_loc(const L& load, const NodeField& F, const int* anc, const float* q) {
+    if constexpr (METHOD == INTERP_WENO6) return weno6_3d_loc(load, F, anc, q);
+    else if constexpr (METHOD == INTERP_LINEAR) return lin3d_loc(load, F, anc, q);
+    else return lin1dy_loc(load, F, anc, q);
 }
 template <int METHOD>
-__device__ __forceinline__ void piece_quad32_linear(const PassDesc& d, const int* anc, float cx, float cy, float cz,
-                                                    float ny, const float* __restrict__ a, const PsiLoad& pl, Kahan& F) {
+__device__ __forceinline__ void piece_quad32_plain(const PassDesc& d, const int* anc, float cx, float cy, float cz,
+                                                   float ny, const float* __restrict__ a, const PsiLoad& pl, Kahan& F) {
     const PlainLoad al{a};
     float yp = cy;
     if (d.use_integral) {
@@ -309,12 +312,12 @@ __device__ __forceinline__ void piece_quad32_linear(const PassDesc& d, const int
             const float hl = second ? (cy - lo) * 0.5f : (two ? 0.25f : (cy - Y.ylo) * 0.5f);
             const float w = (second ? ny * (Y.f - 0.5f) : (two ? ny * 0.5f : ny * Y.f)) * d.gwf[q];
             const float qq[3] = {cx, hl * d.gxf[q] + hl + lo, cz};
-            F.add(linear_loc<METHOD>(al, d.A, anc, qq) * w);
+            F.add(plain_loc<METHOD>(al, d.A, anc, qq) * w);
         }
         yp = Y.ylo;
     }
     const float qp[3] = {cx, yp, cz};
-    F.add(linear_loc<METHOD>(pl, d.P, anc, qp) * (ny * d.invhf));
+    F.add(plain_loc<METHOD>(pl, d.P, anc, qp) * (ny * d.invhf));
 }
 
 __device__ __forceinline__ void corners(int fam, int i, int j, int k, int* ci, int* cj, int* ck) {
@@ -617,13 +620,13 @@ __global__ void __launch_bounds__(kQuadThreads, 4) k_quad32(PassDesc d, typename
 }
 
 template <int METHOD>
-__global__ void __launch_bounds__(kQuadThreads) k_quad32_linear(PassDesc d, const float* __restrict__ a,
-                                                                const float2* __restrict__ psi, PieceStore ps,
+__global__ void __launch_bounds__(kQuadThreads) k_quad32_plain(PassDesc d, const float* __restrict__ a,
+                                                               const float2* __restrict__ psi, PieceStore ps,
                                                                 long long npc, int run) {
     for_pieces(d, ps, npc, run, [&](const float4& p, const int* anc) {
         const float2 b = __ldg(psi + psi_node(d.P, anc[0], anc[1], anc[2]));
         Kahan F;
-        piece_quad32_linear<METHOD>(d, anc, p.x, p.y, p.z, p.w, a, PsiLoad{psi, b.x, b.y}, F);
+        piece_quad32_plain<METHOD>(d, anc, p.x, p.y, p.z, p.w, a, PsiLoad{psi, b.x, b.y}, F);
         return F.value();
     });
 }
@@ -785,16 +788,18 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
         const unsigned grid = (unsigned)std::min<long long>(ntile, 152 * 8);
         const int run = (int)std::max<long long>(1, std::min<long long>(8, ntile / (4 * grid)));
         prof_mark(w, 0, s);
-        if (d.interp == INTERP_WENO6 && d.comp < 0)
+        if (d.interp == INTERP_LINEAR)
+            k_quad32_plain<INTERP_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, run);
+        else if (d.interp != INTERP_WENO6)
+            k_quad32_plain<INTERP_1DY_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, run);
+        else if (!w.arec)
+            k_quad32_plain<INTERP_WENO6><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, run);
+        else if (d.comp < 0)
             k_quad32<WenoNewton><<<grid, kQuadThreads, 0, s>>>(d, newton_records(d.A, w.arec), (const float4*)w.prec, psi,
                                                                ps, (long long)npc, run, w.counters);
-        else if (d.interp == INTERP_WENO6)
+        else
             k_quad32<WenoSamples><<<grid, kQuadThreads, 0, s>>>(d, sample_records(d.A, w.arec), nullptr, psi, ps,
                                                                 (long long)npc, run, w.counters);
-        else if (d.interp == INTERP_LINEAR)
-            k_quad32_linear<INTERP_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, run);
-        else
-            k_quad32_linear<INTERP_1DY_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, run);
         prof_mark(w, 1, s);
     }
     for (int fam = 0; fam < 3; ++fam)
@@ -814,7 +819,7 @@ cudaError_t run_pass<float>(const PassDesc& d64, const VelocityFields& vel64, co
     float2* psi = (float2*)w.psi;
     const long long cols = (long long)d.A.Mx * d.A.Mz;
     k_psi32<<<nblk(cols, 128), 128, 0, s>>>(d, a, psi);
-    if (d.interp == INTERP_WENO6) {
+    if (d.interp == INTERP_WENO6 && w.arec) {
         // without the y-integral no point of the field itself is interpolated
         if (d.comp >= 0) {
             const WenoSamples::Records r = sample_records(d.A, w.arec);

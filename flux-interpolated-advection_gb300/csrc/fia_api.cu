@@ -33,7 +33,7 @@ struct fia_session {
     void* vel[3]; void* vel_next[3];
     void* cbuf;                  // correction field (pass 2 result)
     void* psi; void* verts; void* flux[3]; void* flux_rev[3];
-    void* arec; void* prec;      // FP32 form: z-pass records of the advected field and of psi
+    void* arec = nullptr; void* prec = nullptr;   // z-pass records of the advected field and of psi
     void* verts2 = nullptr;      // flux MacCormack: the vertices traced back (allocated on first use)
     // cell-volume correction (allocated on first use): per-face y n_y sums, cell volumes, the
     // right-hand side and the potential of its Poisson solve
@@ -974,8 +974,6 @@ fia_session* fia_create(int nx, int ny, int nz, double cell_length, int precisio
     A(s->rho, fb); A(s->rho_next, fb); A(s->pres, fb); A(s->cbuf, (size_t)big * 8); A(s->psi, pb);
     for (int c = 0; c < 3; ++c) { A(s->vel[c], fb); A(s->vel_next[c], fb); A(s->flux[c], pb); A(s->flux_rev[c], pb); }
     A(s->verts, 3 * fb);
-    s->arec = s->prec = nullptr;
-    if (precision == FIA_FP32C) { A(s->arec, (size_t)big * kRecBytes); A(s->prec, (size_t)big * kPsiRecBytes); }
     s->verts_bytes = fb;
     for (int q = 0; q < 5; ++q) A(s->pw[q], fb);
     { void* t2; A(t2, 4 * sizeof(unsigned)); s->ticket = (unsigned*)t2; }
@@ -994,6 +992,17 @@ fia_session* fia_create(int nx, int ny, int nz, double cell_length, int precisio
         ok = piece_store_reserve(s->pieces, 10 * big + 1024, big) == cudaSuccess;
     }
     if (ok && precision == FIA_FP64) ok = piece_store64_reserve(s->pieces64, 10 * big + 1024, big) == cudaSuccess;
+    if (ok) {
+        // the z-pass records; a session that finds no memory for them interpolates without
+        const size_t ab = (size_t)big * (precision == FIA_FP64 ? kRecBytes64 : kRecBytes);
+        const size_t rb = (size_t)big * (precision == FIA_FP64 ? kRecBytes64 : kPsiRecBytes);
+        if (cudaMalloc(&s->arec, ab) != cudaSuccess) s->arec = nullptr;
+        if (!s->arec || cudaMalloc(&s->prec, rb) != cudaSuccess) {
+            cudaFree(s->arec);
+            s->arec = s->prec = nullptr;
+            cudaGetLastError();
+        }
+    }
     if (!ok) {
         g_last_error = "fia_create: device allocation failed";
         fia_destroy(s);
@@ -1040,6 +1049,7 @@ void fia_destroy(fia_session* s) {
     unet::net_destroy(s->net);
     piece_store_free(s->pieces);
     piece_store64_free(s->pieces64);
+    cudaFree(s->arec); cudaFree(s->prec);
     if (s->p64) cudaFree(s->p64);
     if (s->solid) cudaFree(s->solid);
     for (void* p : s->allocations) cudaFree(p);

@@ -19,7 +19,7 @@ namespace fia {
 // One 1D WENO6 evaluation as a real call.  Inlined, the face kernel held some sixty copies
 // of weno6_eval (the unrolled z-passes of a stencil), more code than the instruction cache
 // holds; ncu showed most warps waiting on instruction fetch.  Arguments travel in registers.
-__device__ __noinline__ float weno6_f(float f0, float f1, float f2, float f3, float f4, float f5, WenoCoef<float> w) {
+static __device__ __noinline__ float weno6_f(float f0, float f1, float f2, float f3, float f4, float f5, WenoCoef<float> w) {
     const float f[6] = {f0, f1, f2, f3, f4, f5};
     return weno6_eval<float, true>(f, w);
 }
@@ -29,7 +29,7 @@ __device__ __forceinline__ float weno6_call(const float* f, const WenoCoef<float
 // Two evaluations with the same coefficients in one call: the two dependency chains (the
 // weights end in a serial max / reciprocal / normalise tail) interleave, which a call per
 // evaluation prevents, at half the calls.  Each result equals weno6_f's.
-__device__ __noinline__ float2 weno6_f2(float a0, float a1, float a2, float a3, float a4, float a5, float b0, float b1,
+static __device__ __noinline__ float2 weno6_f2(float a0, float a1, float a2, float a3, float a4, float a5, float b0, float b1,
                                         float b2, float b3, float b4, float b5, WenoCoef<float> w) {
     const float fa[6] = {a0, a1, a2, a3, a4, a5}, fb[6] = {b0, b1, b2, b3, b4, b5};
     return make_float2(weno6_eval<float, true>(fa, w), weno6_eval<float, true>(fb, w));

@@ -8,7 +8,7 @@
 //
 // Two arithmetics.
 //
-// WenoNewton (density).  For six samples f0..f5 and a position s in [0, 1) past f2, the three
+// WenoNewton (density, and every field of the FP64 form).  For six samples f0..f5 and a position s in [0, 1) past f2, the three
 // cubic candidates in Newton form around f2 share their linear term:
 //   P_i = f2 + s D2 + m G_i,   m = s (s - 1) / 6,
 //   G_0 = 3 S1 + (s + 1) T0,  G_1 = 3 S1 + (s + 1) (S2 - S1),  G_2 = 3 S2 + (s - 2) T2
@@ -33,13 +33,20 @@
 namespace fia {
 
 // 1/x for the weights' quotients.  FP32: the hardware approximation (1 ulp) without the scaling
-// of subnormal operands, which weno_indicators keeps away.  FP64: IEEE.
+// of subnormal operands, which weno_indicators keeps away.  FP64: the hardware's seed (20 bits) and
+// two Newton steps x += x (1 - a x), correct to about one unit in the last place: four FP64
+// instructions, of which an IEEE division takes about ten.
 __device__ __forceinline__ float weno_rcp(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ double weno_rcp(double x) { return 1.0 / x; }
+__device__ __forceinline__ double weno_rcp(double a) {
+    double x;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(a));
+    x = fma(x, fma(-a, x, 1.0), x);
+    return fma(x, fma(-a, x, 1.0), x);
+}
 
 // what depends on the position alone
 template <typename T>
@@ -163,6 +170,13 @@ __host__ __device__ __forceinline__ long long weno_rec_count(const NodeField& F)
 template <typename T>
 __device__ __forceinline__ WenoData<T> weno_unpack(const WenoRec<T>& r) {
     return WenoData<T>{r.f, r.d, r.s1, r.s2, r.t0, r.t2, r.q0, (T(1) - r.q0) - r.q2, r.q2};
+}
+
+// FP64 records: eight doubles
+__device__ __forceinline__ WenoRec<double> ldg_rec(const WenoRec<double>* p) {
+    const double2* q = reinterpret_cast<const double2*>(p);
+    const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3);
+    return WenoRec<double>{a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y};
 }
 
 struct WenoNewton {

@@ -1,4 +1,4 @@
-"""The per-piece quadrature of the chosen form at the edges of its stencils and point groups: grids
+"""The per-piece quadrature of both forms at the edges of its stencils and point groups: grids
 smaller than the six-node stencil along each axis (every z-record clamped), Gauss rules around
 the group of three points, and WENO6 psi points off the node rows (use_integral 0).
 
@@ -42,6 +42,30 @@ def test_fp32_weno_pass_small_grids(shape, comp, k, integral):
     keep = np.argsort(d)[:-4]
     assert np.linalg.norm(d[keep]) < 2e-6 * np.linalg.norm(ref)
     assert np.linalg.norm(d) < 5e-4 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("shape", [(2, 2, 2), (3, 7, 2), (9, 2, 5), (12, 9, 33)])
+@pytest.mark.parametrize("comp", [-1, 0, 1, 2])
+@pytest.mark.parametrize("k,integral,zero", [(1, 1, 0), (5, 1, 0), (15, 1, 0), (3, 0, 0), (3, 0, 1)])
+def test_fp64_weno_pass_small_grids(shape, comp, k, integral, zero):
+    """the plain form at its parity bound, 1e-10"""
+    n = max(shape)
+    h = 1.0 / n
+    nx, ny, nz = shape
+    u, v, w = scenes.fourier_velocity(n, seed=3)
+    u = u.reshape(n + 1, n, n)[:nx + 1, :ny, :nz].ravel()
+    v = v.reshape(n, n + 1, n)[:nx, :ny + 1, :nz].ravel()
+    w = w.reshape(n, n, n + 1)[:nx, :ny, :nz + 1].ravel()
+    f = (u, v, w)[comp] if comp >= 0 else scenes.gaussian_blobs(n, seed=4).reshape(n, n, n)[:nx, :ny, :nz].ravel()
+    dt = 1.7 * h
+    ref, _, _, _ = O.flux_pass(shape, h, u, v, w, comp, f, dt, 0, 1, integral, zero, (0.5, 0.5), k)
+    g = fia.Grid3D(*shape, h)
+    for name, a in (("u", u), ("v", v), ("w", w)):
+        g.set(name, a)
+    got, st = g.debug_flux_pass(comp, f, dt, 0, 1, integral, zero, (0.5, 0.5), k)
+    g.close()
+    assert st == 0
+    assert np.linalg.norm(got - ref) < 1e-10 * np.linalg.norm(ref)
 
 
 def test_fp32_weno_weights_keep_their_range():
