@@ -357,18 +357,12 @@ __device__ __forceinline__ int range_bits(int nfwd, int nrev, bool multi) {
 //               when an iso-line crosses a piece more than twice), pieces appended
 //               contiguously per face (warp prefix sum + one atomic per warp), y-normal sums;
 //               a face the shared pool cannot hold goes to a list
-//  k_clip32_deferred  the listed faces, clipped in local memory, appended the same way
+//  k_clip32_deferred  the listed faces, in a larger shared pool or else in local memory, appended
+//               the same way
 //  k_quad32     one thread per piece: quadrature + WENO6 (uniform work per thread, no clip
 //               code, so fewer registers and no divergence from the piece count);
 //  k_facesum32  one thread per face: compensated sum of its pieces in emission order.
-__device__ __forceinline__ void face_of(int fam, const NodeField& A, long long id, int& i, int& j, int& k) {
-    const int Fy = A.My + (fam == 1), Fz = A.Mz + (fam == 2);
-    k = (int)(id % Fz);
-    j = (int)((id / Fz) % Fy);
-    i = (int)(id / ((long long)Fz * Fy));
-}
-
-// face_of for the tags of the piece store (face ids below 2^29): two 32-bit divisions
+// lattice index of face id of family fam (ids are below 2^29): two 32-bit divisions
 __device__ __forceinline__ void face_of32(int fam, const NodeField& A, unsigned id, int& i, int& j, int& k) {
     const unsigned Fy = A.My + (fam == 1), Fz = A.Mz + (fam == 2);
     const unsigned t = id / Fz;
@@ -382,7 +376,7 @@ __device__ __forceinline__ void face_of32(int fam, const NodeField& A, unsigned 
 __device__ __forceinline__ void face_geometry(const PassDesc& d, int fam, long long id, const float* __restrict__ disp,
                                               LocalFace& g) {
     int i, j, k;
-    face_of(fam, d.A, id, i, j, k);
+    face_of32(fam, d.A, (unsigned)id, i, j, k);
     int ci[4], cj[4], ck[4];
     corners(fam, i, j, k, ci, cj, ck);
     g.anc[0] = i; g.anc[1] = j; g.anc[2] = k;
@@ -416,36 +410,55 @@ __device__ __forceinline__ void warp_counters(unsigned long long pc, unsigned fc
     }
 }
 
-// fast = 0 sends every face to the list (the local-memory clipper alone)
-__global__ void __launch_bounds__(kClipThreads, 4) k_clip32(PassDesc d, int fam, const float* __restrict__ disp,
-                                                            PieceStore ps, unsigned* status,
-                                                            unsigned long long* counters, int fast) {
+// Both clips of a face into a pool; false: it does not fit.
+template <class Pool>
+__device__ __forceinline__ bool clip_both(const PassDesc& d, const LocalFace& g, const Pool& P, int& npieces, bool& multi,
+                                          int& nst, int& nfwd, float& N, float& Nr) {
+    Kahan ny;
+    if (!clip32_fast(d, g, npieces, multi, nst, ny, P)) return false;
+    nfwd = nst;
+    N = ny.value();
+    Nr = -N;
+    if (multi) {
+        ny = Kahan();
+        int np2 = 0;
+        bool m2 = false;
+        if (!clip32_fast(d, reversed_face(g), np2, m2, nst, ny, P)) return false;
+        Nr = ny.value();
+    }
+    return true;
+}
+
+// The face families of one launch: blocks [first[f], first[f + 1]) hold family f.  One launch for
+// the three instead of one each leaves one partly filled last wave, not three: a MacCormack
+// step on 70 x 97 x 51 cells took 3.50 ms before this and the larger pool below, 2.97 with both.
+struct FamilyBlocks {
+    unsigned first[4];
+    __device__ __forceinline__ int family(unsigned b) const { return b < first[1] ? 0 : (b < first[2] ? 1 : 2); }
+    __device__ __forceinline__ unsigned start(int fam) const { return fam == 0 ? first[0] : (fam == 1 ? first[1] : first[2]); }
+};
+__device__ __forceinline__ long long family_faces(const PassDesc& d, int fam) {
+    return (long long)(d.A.Mx + (fam == 0)) * (d.A.My + (fam == 1)) * (d.A.Mz + (fam == 2));
+}
+
+// fast = 0 sends every face to the list
+__global__ void __launch_bounds__(kClipThreads, kClipBlocks) k_clip32(PassDesc d, FamilyBlocks fb,
+                                                                      const float* __restrict__ disp, PieceStore ps,
+                                                                      unsigned* status, unsigned long long* counters,
+                                                                      int fast) {
     extern __shared__ float clip_smem[];
     const FastPool P{clip_smem + threadIdx.x};
-    const int Fx = d.A.Mx + (fam == 0), Fy = d.A.My + (fam == 1), Fz = d.A.Mz + (fam == 2);
-    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long nface = (long long)Fx * Fy * Fz;
+    const int fam = fb.family(blockIdx.x);
+    const long long id = (long long)(blockIdx.x - fb.start(fam)) * blockDim.x + threadIdx.x;
+    const long long nface = family_faces(d, fam);
     const int lane = threadIdx.x & 31;
     int npieces = 0, nst = 0, nfwd = 0;
     bool multi = false, ok = false;
     if (id < nface) {
         LocalFace g;
         face_geometry(d, fam, id, disp, g);
-        Kahan ny;
-        ok = fast != 0 && clip32_fast(d, g, npieces, multi, nst, ny, P);
         float N = 0.f, Nr = 0.f;
-        if (ok) {
-            nfwd = nst;
-            N = ny.value();
-            Nr = -N;
-            if (multi) {
-                ny = Kahan();
-                int np2 = 0;
-                bool m2 = false;
-                ok = clip32_fast(d, reversed_face(g), np2, m2, nst, ny, P);
-                Nr = ny.value();
-            }
-        }
+        ok = fast != 0 && clip_both(d, g, P, npieces, multi, nst, nfwd, N, Nr);
         if (ok) {
             normal_of(ps, fam)[id] = make_float2(N, Nr);
         } else {
@@ -459,11 +472,7 @@ __global__ void __launch_bounds__(kClipThreads, 4) k_clip32(PassDesc d, int fam,
     if (ok) {
         if (start + cnt <= ps.cap) {
             const int tag = (fam << 29) | (int)id;
-            for (int q = 0; q < cnt; ++q) {
-                const int e = kFastR - 1 - q;
-                ps.rec[start + q] = make_float4(P.at(e, 0), P.at(e, 1), P.at(e, 2), P.at(e, 3));
-                ps.face[start + q] = tag;
-            }
+            for (int q = 0; q < cnt; ++q) { ps.rec[start + q] = P.piece(q); ps.face[start + q] = tag; }
         }
         // a range beyond the capacity is kept as it is: the host sees the count, grows the
         // store and runs the pass again
@@ -472,48 +481,60 @@ __global__ void __launch_bounds__(kClipThreads, 4) k_clip32(PassDesc d, int fam,
     warp_counters((unsigned long long)npieces, ok ? 1u : 0u, (ok && multi) ? 1u : 0u, 0u, lane, status, counters);
 }
 
-// The faces k_clip32 listed (all families), clipped by clip32 in local memory; grid-stride
-// over the list length the clip kernels left in ps.count[1].
-__global__ void __launch_bounds__(128) k_clip32_deferred(PassDesc d, const float* __restrict__ disp, PieceStore ps,
-                                                         unsigned* status, unsigned long long* counters) {
+// The faces k_clip32 listed (all families): with a larger pool, or else by clip32 in local
+// memory; grid-stride over the list length the clip kernels left in ps.count[1].
+__global__ void __launch_bounds__(kDeferThreads) k_clip32_deferred(PassDesc d, const float* __restrict__ disp, PieceStore ps,
+                                                                   unsigned* status, unsigned long long* counters,
+                                                                   int fast) {
+    __shared__ float pool[DeferPool::kWords * kDeferThreads];
+    const DeferPool P{pool + threadIdx.x};
     const long long nd = (long long)ps.count[1];
     const int lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x == 0 && nd > 0) atomicAdd(&counters[4], (unsigned long long)nd);
-    for (long long base = (long long)blockIdx.x * blockDim.x; base < nd; base += (long long)gridDim.x * blockDim.x) {
-        const long long t = base + threadIdx.x;
-        const bool valid = t < nd;
+    // a short list is spread over the warps: the faces of one would wait for each other
+    const long long warps = (long long)gridDim.x * (kDeferThreads / 32);
+    const int per = (int)min(32LL, (nd + warps - 1) / warps);
+    for (long long base = ((long long)blockIdx.x * (kDeferThreads / 32) + (threadIdx.x >> 5)) * per; base < nd;
+         base += warps * per) {
+        const long long t = base + lane;
+        const bool valid = lane < per && t < nd;
         const int tag = valid ? ps.deferred[t] : 0;
         const int fam = tag >> 29;
         const long long id = tag & ((1 << 29) - 1);
         unsigned st = 0;
-        int npieces = 0, nmulti = 0, nfwd = 0;
-        bool multi = false;
+        int npieces = 0, cnt = 0, nfwd = 0;
+        bool multi = false, pooled = false;
         PieceSink sink;
         if (valid) {
             LocalFace g;
             face_geometry(d, fam, id, disp, g);
-            clip32(d, g, st, npieces, multi, sink);
-            nfwd = sink.n;
-            const float N = sink.ny.value();
-            float Nr = -N;
-            if (multi) {
-                int np2 = 0;
-                bool m2 = false;
-                sink.ny = Kahan();
-                clip32(d, reversed_face(g), st, np2, m2, sink);
-                Nr = sink.ny.value();
-                ++nmulti;
+            float N = 0.f, Nr = 0.f;
+            pooled = fast != 0 && clip_both(d, g, P, npieces, multi, cnt, nfwd, N, Nr);
+            if (!pooled) {
+                npieces = 0;
+                multi = false;
+                clip32(d, g, st, npieces, multi, sink);
+                nfwd = sink.n;
+                N = sink.ny.value();
+                Nr = -N;
+                if (multi) {
+                    int np2 = 0;
+                    bool m2 = false;
+                    sink.ny = Kahan();
+                    clip32(d, reversed_face(g), st, np2, m2, sink);
+                    Nr = sink.ny.value();
+                }
+                cnt = sink.n;
             }
             normal_of(ps, fam)[id] = make_float2(N, Nr);
         }
-        const int cnt = sink.n;
         const long long start = warp_slots(ps.count, cnt, lane);
         if (valid) {
             if (start + cnt <= ps.cap)
-                for (int q = 0; q < cnt; ++q) { ps.rec[start + q] = sink.p[q]; ps.face[start + q] = tag; }
+                for (int q = 0; q < cnt; ++q) { ps.rec[start + q] = pooled ? P.piece(q) : sink.p[q]; ps.face[start + q] = tag; }
             range_of(ps, fam)[id] = make_int2((int)start, range_bits(nfwd, cnt - nfwd, multi));
         }
-        warp_counters((unsigned long long)npieces, valid ? 1u : 0u, (unsigned)nmulti, st, lane, status, counters);
+        warp_counters((unsigned long long)npieces, valid ? 1u : 0u, (valid && multi) ? 1u : 0u, st, lane, status, counters);
     }
 }
 
@@ -635,11 +656,16 @@ __global__ void __launch_bounds__(kQuadThreads) k_quad32_plain(PassDesc d, const
 // MacCormack scheme accumulate into one (flux, y-normal sum) pair per face
 // With fvol: (M, Mr) = sums of y n_y of the face's pieces in cells (y relative to the face
 // anchor), the same weighting, for the cell volumes of the cell-volume correction.
-__global__ void k_facesum32(PassDesc d, int fam, PieceStore ps, float2* __restrict__ flux, float2* __restrict__ flux_rev,
-                            unsigned* status, float wgt, int acc, float2* __restrict__ fvol) {
-    const long long nface = (long long)(d.A.Mx + (fam == 0)) * (d.A.My + (fam == 1)) * (d.A.Mz + (fam == 2));
-    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= nface) return;
+struct FaceSums {
+    float2 *flux[3], *flux_rev[3], *fvol[3];
+};
+__global__ void k_facesum32(PassDesc d, FamilyBlocks fb, PieceStore ps, FaceSums fs, unsigned* status, float wgt, int acc) {
+    const int fam = fb.family(blockIdx.x);
+    const long long id = (long long)(blockIdx.x - fb.start(fam)) * blockDim.x + threadIdx.x;
+    if (id >= family_faces(d, fam)) return;
+    float2* const flux = fam == 0 ? fs.flux[0] : (fam == 1 ? fs.flux[1] : fs.flux[2]);
+    float2* const flux_rev = fam == 0 ? fs.flux_rev[0] : (fam == 1 ? fs.flux_rev[1] : fs.flux_rev[2]);
+    float2* const fvol = fam == 0 ? fs.fvol[0] : (fam == 1 ? fs.fvol[1] : fs.fvol[2]);
     const int2 r = range_of(ps, fam)[id];
     const int nf = r.y & 0x7fff, nr = (r.y >> 15) & 0x7fff;
     const bool multi = (r.y >> 30) & 1;
@@ -729,6 +755,13 @@ __global__ void k_gather32(PassDesc d, const float2* __restrict__ fx, const floa
 }
 
 inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
+// blocks of t threads over the faces of the three families (faces at rest: the y-faces)
+inline FamilyBlocks family_blocks(const long long* nface, bool rest, int t) {
+    FamilyBlocks fb;
+    fb.first[0] = 0;
+    for (int f = 0; f < 3; ++f) fb.first[f + 1] = fb.first[f] + (rest && f != 1 ? 0u : nblk(nface[f], t));
+    return fb;
+}
 
 }  // namespace
 
@@ -768,11 +801,9 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
             k_rest_clip32<<<1, 32, 0, s>>>(d, 1, ps);
             k_rest_fill32<<<nblk(nface[1], 256), 256, 0, s>>>(d, 1, ps, w.status, w.counters);
         } else {
-            for (int fam = 0; fam < 3; ++fam)
-                if (!rest || fam == 1)
-                    k_clip32<<<nblk(nface[fam], kClipThreads), kClipThreads, kClipSmem, s>>>(d, fam, disp, ps, w.status,
-                                                                                             w.counters, ps.clip_fast);
-            k_clip32_deferred<<<152 * 8, 128, 0, s>>>(d, disp, ps, w.status, w.counters);
+            const FamilyBlocks fb = family_blocks(nface, rest, kClipThreads);
+            k_clip32<<<fb.first[3], kClipThreads, kClipSmem, s>>>(d, fb, disp, ps, w.status, w.counters, ps.clip_fast);
+            k_clip32_deferred<<<152 * 4, kDeferThreads, 0, s>>>(d, disp, ps, w.status, w.counters, ps.clip_fast);
         }
         cudaError_t e = cudaMemcpyAsync(&npc, ps.count, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -802,11 +833,14 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
                                                                 (long long)npc, run, w.counters);
         prof_mark(w, 1, s);
     }
-    for (int fam = 0; fam < 3; ++fam)
-        if (!rest || fam == 1)
-            k_facesum32<<<nblk(nface[fam], 256), 256, 0, s>>>(d, fam, ps, (float2*)w.flux[fam], (float2*)w.flux_rev[fam],
-                                                              w.status, wgt, acc,
-                                                              d.volumes ? (float2*)w.fvol[fam] : nullptr);
+    FaceSums fs;
+    for (int fam = 0; fam < 3; ++fam) {
+        fs.flux[fam] = (float2*)w.flux[fam];
+        fs.flux_rev[fam] = (float2*)w.flux_rev[fam];
+        fs.fvol[fam] = d.volumes ? (float2*)w.fvol[fam] : nullptr;
+    }
+    const FamilyBlocks fb = family_blocks(nface, rest, 256);
+    k_facesum32<<<fb.first[3], 256, 0, s>>>(d, fb, ps, fs, w.status, wgt, acc);
     return cudaGetLastError();
 }
 

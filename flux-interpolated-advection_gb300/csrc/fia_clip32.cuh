@@ -16,9 +16,21 @@ namespace fia {
 struct CVf { float p0, p1, c0, c1; };
 __host__ __device__ __forceinline__ float cvc(const CVf& v, int dim) { return dim ? v.c1 : v.c0; }
 
+// Sums of products written out (one product rounded, the others fused), so that every clipper in
+// every kernel rounds alike.
+__host__ __device__ __forceinline__ float clip_mul(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+// a b - c d
+__host__ __device__ __forceinline__ float cross2(float a, float b, float c, float d) { return fmaf(a, b, -clip_mul(c, d)); }
+
 __host__ __device__ __forceinline__ float bilinf(const float* v, float xi, float eta) {
     const float a = v[1] - v[0], b = v[3] - v[0], c = (v[0] - v[1]) + (v[2] - v[3]);
-    return v[0] + xi * a + eta * b + (xi * eta) * c;
+    return fmaf(clip_mul(xi, eta), c, fmaf(eta, b, fmaf(xi, a, v[0])));
 }
 
 struct LocalFace {
@@ -70,18 +82,20 @@ struct ArrayVerts {
 // on the far side of the iso-line that bounds it, and the error pass's nearest-cell
 // interpolation (1Dy-linear) then read psi of the wrong column.  Relative to the first vertex
 // the products are of the sliver's own size and its centroid is accurate to FP32 rounding.
+// The terms of the first vertex's two edges vanish.
 template <class V>
 __host__ __device__ __forceinline__ void centroid_v(const V& v, int num, float& cx, float& cy, float& area) {
     const float x0 = v.x(0), y0 = v.y(0);
     float a = 0.f, sx = 0.f, sy = 0.f;
-    for (int n = 0; n < num; ++n) {
-        const int m = (n + 1 == num) ? 0 : n + 1;
-        const float xn = v.x(n) - x0, yn = v.y(n) - y0, xm = v.x(m) - x0, ym = v.y(m) - y0;
-        const float c = xn * ym - xm * yn;
-        a += c; sx += c * (xn + xm); sy += c * (yn + ym);
+    float xn = v.x(1) - x0, yn = v.y(1) - y0;
+    for (int m = 2; m < num; ++m) {
+        const float xm = v.x(m) - x0, ym = v.y(m) - y0;
+        const float c = cross2(xn, ym, xm, yn);
+        a += c; sx = fmaf(c, xn + xm, sx); sy = fmaf(c, yn + ym, sy);
+        xn = xm; yn = ym;
     }
     a = fabsf(0.5f * a);
-    if (a != 0.f) { const float s = 1.0f / (6.0f * a); cx = x0 + sx * s; cy = y0 + sy * s; }
+    if (a != 0.f) { const float s = 1.0f / (6.0f * a); cx = x0 + clip_mul(sx, s); cy = y0 + clip_mul(sy, s); }
     else {
         sx = 0.f; sy = 0.f;
         for (int n = 0; n < num; ++n) { sx += v.x(n) - x0; sy += v.y(n) - y0; }
@@ -104,7 +118,7 @@ __host__ __device__ __forceinline__ bool piece_geom_v(const LocalFace& g, const 
         const float x0 = bilinf(g.x, v.x(0), v.y(0)), z0 = bilinf(g.z, v.x(0), v.y(0));
         const float ax = bilinf(g.x, v.x(1), v.y(1)) - x0, az = bilinf(g.z, v.x(1), v.y(1)) - z0;
         const float bx = bilinf(g.x, v.x(2), v.y(2)) - x0, bz = bilinf(g.z, v.x(2), v.y(2)) - z0;
-        ny = 0.5f * (az * bx - ax * bz);
+        ny = 0.5f * cross2(az, bx, ax, bz);
     } else {
         float acc = 0.f;
         float x0 = bilinf(g.x, v.x(0), v.y(0)) - cx, z0 = bilinf(g.z, v.x(0), v.y(0)) - cz;
@@ -113,7 +127,7 @@ __host__ __device__ __forceinline__ bool piece_geom_v(const LocalFace& g, const 
             float x1, z1;
             if (n + 1 == num) { x1 = xs; z1 = zs; }
             else { x1 = bilinf(g.x, v.x(n + 1), v.y(n + 1)) - cx; z1 = bilinf(g.z, v.x(n + 1), v.y(n + 1)) - cz; }
-            acc += z0 * x1 - x0 * z1;
+            acc += cross2(z0, x1, x0, z1);
             x0 = x1; z0 = z1;
         }
         ny = acc * 0.5f;
@@ -182,9 +196,9 @@ constexpr int kPool32 = 144, kMaxV32 = 32, kStack32 = 48;
 __host__ __device__ __forceinline__ float cross_point(const CVf& a, const CVf& b, float v0, float v1, float iso, int dim, CVf& X) {
     const float inv = 1.0f / (v1 - v0);
     const float t0 = v1 * inv, t1 = -v0 * inv;
-    X.p0 = t0 * a.p0 + t1 * b.p0;
-    X.p1 = t0 * a.p1 + t1 * b.p1;
-    const float other = snap_int(t0 * cvc(a, 1 - dim) + t1 * cvc(b, 1 - dim));
+    X.p0 = fmaf(t0, a.p0, clip_mul(t1, b.p0));
+    X.p1 = fmaf(t0, a.p1, clip_mul(t1, b.p1));
+    const float other = snap_int(fmaf(t0, cvc(a, 1 - dim), clip_mul(t1, cvc(b, 1 - dim))));
     if (dim == 0) { X.c0 = iso; X.c1 = other; } else { X.c1 = iso; X.c0 = other; }
     return t1;
 }
@@ -281,15 +295,33 @@ static __host__ __device__ void clip32(const PassDesc& d, const LocalFace& g, un
 // out word-major ([word][thread]): a warp's access to one word of its threads' slots is one
 // conflict-free wavefront however far apart the threads' polygons are, where the same pool
 // in local memory costs a line per thread and, with 36 warps per SM, is written back to
-// DRAM (about 360 bytes per face).  The pool grows upward from slot 0 and the face's pieces
-// downward from the top slot.  It is clip32 -- the same cuts, pieces, emission order and
-// arithmetic -- except that a face needing more room (about 0.2% of the faces of a developed
-// flow at CFL 2), cutting a polygon an odd number of times, or holding a piece above the
+// DRAM (about 360 bytes per face).
+//
+// Bound by the serial chain of cuts of each lane's own face (about 24 of 32 lanes in step) and the
+// shared-memory latency on it, which the resident warps hide: a pool of 15 slots and 12 words lets six
+// CTAs stay on an SM.  The clip launches of two density steps at 128^3: 5.90 ms with one cut per
+// crossing edge and byte lists of moved vertices, 3.21 ms now.  The same step, all launches, with
+// other pools: 22 slots, 18 words, four CTAs 5.76 ms; 18, 15, five 5.53; 15, 12, six 5.50; 14, 12, six
+// 5.52 (the smaller the pool, the more faces go to the list).
+//
+// A polygon is a list of up to eight 4-bit vertex numbers in one word: a cut adds two vertices and
+// moves none, and the lists of its parts are shifts of the parent's.  A cut that crosses two
+// edges (a line crosses nearly every polygon so) finds them from the vertices' sides as a bit
+// mask, then computes both crossing points at once, not edge by edge as each lane comes to its
+// own.  The range of a polygon's colours is taken once a colour: after a cut at an iso-line the
+// part below it needs no further cut in that colour, and the part above it is next cut at the
+// next line, up to the parent's last.  Vertices grow upward from slot 0 (those of finished
+// polygons are dropped with them), the face's pieces downward from the top slot.
+//
+// It is clip32 -- the same cuts, pieces, emission order and arithmetic -- except that a face
+// needing more room, cutting a polygon an odd number of times, or holding a piece above the
 // triangulation area returns false and is clipped again by clip32 in local memory.
-constexpr int kFastR = 26, kFastS = 6, kClipThreads = 128;
+constexpr int kFastR = 15, kFastS = 12, kClipThreads = 128, kClipBlocks = 6;   // CTAs per SM
 constexpr int kFastWords = 4 * kFastR + kFastS;
-constexpr int kClipSmem = kFastWords * kClipThreads * (int)sizeof(float);   // 56,320 B: 4 CTAs per SM
-static_assert(4 * (kClipSmem + 1024) <= 233472, "four clip CTAs per SM");
+constexpr int kClipSmem = kFastWords * kClipThreads * (int)sizeof(float);   // 36,864 B
+static_assert(kClipBlocks * (kClipSmem + 1024) <= 233472, "clip CTAs per SM");
+constexpr int kFastVerts = 16;       // 4-bit vertex numbers
+constexpr int kFastIso = 30000;      // iso values of a stack entry are 16-bit
 
 #ifndef __CUDA_ARCH__
 // host builds of the clipper (the host check of the shared-pool clipper) stop on a slot outside
@@ -300,13 +332,18 @@ static_assert(4 * (kClipSmem + 1024) <= 233472, "four clip CTAs per SM");
 }
 #endif
 
-struct FastPool {
+// R vertex slots and S stack words of each of STRIDE threads; polygons of eight (32-bit lists) or
+// fifteen vertices (64-bit lists)
+template <int R, int S, int STRIDE, typename List>
+struct ClipPool {
+    static constexpr int kR = R, kS = S, kWords = 4 * R + S, kNum = sizeof(List) == 4 ? 8 : 15;
+    typedef List list;
     float* w;   // this thread's word 0
     __host__ __device__ __forceinline__ float& at(int e, int c) const {
 #ifndef __CUDA_ARCH__
-        if (e < 0 || e >= kFastR || c < 0 || c > 3) fast_pool_range_error(e, c);
+        if (e < 0 || e >= R || c < 0 || c > 3) fast_pool_range_error(e, c);
 #endif
-        return w[(4 * e + c) * kClipThreads];
+        return w[(4 * e + c) * STRIDE];
     }
     __host__ __device__ __forceinline__ CVf get(int e) const { return CVf{at(e, 0), at(e, 1), at(e, 2), at(e, 3)}; }
     __host__ __device__ __forceinline__ void put(int e, const CVf& v) const {
@@ -314,26 +351,62 @@ struct FastPool {
     }
     __host__ __device__ __forceinline__ unsigned& stk(int i) const {
 #ifndef __CUDA_ARCH__
-        if (i < 0 || i >= kFastS) fast_pool_range_error(kFastR + i, -1);
+        if (i < 0 || i >= S) fast_pool_range_error(R + i, -1);
 #endif
-        return reinterpret_cast<unsigned*>(w)[(4 * kFastR + i) * kClipThreads];
+        return reinterpret_cast<unsigned*>(w)[(4 * R + i) * STRIDE];
+    }
+    // piece q of the face (stored downward from the top slot)
+    __host__ __device__ __forceinline__ float4 piece(int q) const {
+        const int e = R - 1 - q;
+        return make_float4(at(e, 0), at(e, 1), at(e, 2), at(e, 3));
     }
 };
-struct PoolVerts {
-    FastPool P;
-    int s;
-    __host__ __device__ __forceinline__ float x(int n) const { return P.at(s + n, 0); }
-    __host__ __device__ __forceinline__ float y(int n) const { return P.at(s + n, 1); }
+typedef ClipPool<kFastR, kFastS, kClipThreads, unsigned> FastPool;
+// The faces k_clip32 lists get a larger pool before the local-memory clipper, whose launch cost
+// 54 us at 128^3 and at 16^3 alike (one face's serial chain through local frames); with this pool 19.
+constexpr int kDeferThreads = 64;
+typedef ClipPool<36, 28, kDeferThreads, unsigned long long> DeferPool;
+
+// a polygon: vertex n is nibble n of v
+template <typename List>
+struct FastPoly {
+    List v;
+    int num;
+    __host__ __device__ __forceinline__ int id(int n) const { return (int)(v >> (4 * n)) & 15; }
+    __host__ __device__ __forceinline__ void add(int i) { v |= (List)i << (4 * num); ++num; }
+    // vertices [n, n + count) of another polygon, not all a list holds
+    __host__ __device__ __forceinline__ void add(const FastPoly& p, int n, int count) {
+        v |= ((p.v >> (4 * n)) & (((List)1 << (4 * count)) - 1)) << (4 * num);
+        num += count;
+    }
 };
-__host__ __device__ __forceinline__ unsigned stack_word(int start, int num, int dim) {
-    return (unsigned)start | ((unsigned)num << 8) | ((unsigned)dim << 16);
+template <class Pool>
+struct PoolVerts {
+    Pool P;
+    FastPoly<typename Pool::list> p;
+    __host__ __device__ __forceinline__ float x(int n) const { return P.at(p.id(n), 0); }
+    __host__ __device__ __forceinline__ float y(int n) const { return P.at(p.id(n), 1); }
+};
+__host__ __device__ __forceinline__ int lowest_bit(unsigned m) {
+#ifdef __CUDA_ARCH__
+    return __ffs((int)m) - 1;
+#else
+    return __builtin_ctz(m);
+#endif
 }
 
+// what comes next for a polygon: its range in colour 0, cuts in colour 0, its range in colour 1,
+// cuts in colour 1, emission
+enum FastStage : int { FS_RANGE0 = 0, FS_CUT0 = 1, FS_RANGE1 = 2, FS_CUT1 = 3, FS_EMIT = 4 };
+
 // One clip of a face (facecutter.h:59-224) in the shared pool.  nst pieces are stored so far
-// (slot kFastR - 1 - q holds piece q as cx, cy, cz, ny); ny sums the y-normals of this clip.
+// (slot R - 1 - q holds piece q as cx, cy, cz, ny); ny sums the y-normals of this clip.
+template <class Pool>
 static __host__ __device__ bool clip32_fast(const PassDesc& d, const LocalFace& g, int& npieces, bool& multi, int& nst, Kahan& ny,
-                            const FastPool& P) {
-    if (4 > kFastR - nst) return false;
+                            const Pool& P) {
+    constexpr int R = Pool::kR, S = Pool::kS, kNum = Pool::kNum, kEntry = sizeof(typename Pool::list) == 4 ? 3 : 4;
+    typedef FastPoly<typename Pool::list> Poly;
+    if (4 > R - nst) return false;
     const float xi[4] = {0.f, 1.f, 1.f, 0.f}, eta[4] = {0.f, 0.f, 1.f, 1.f};
     float col0[4], col1[4];
 #pragma unroll
@@ -344,99 +417,124 @@ static __host__ __device__ bool clip32_fast(const PassDesc& d, const LocalFace& 
     if (!colours_finite(col0, col1, g.y)) return false;    // flagged by clip32
 #pragma unroll
     for (int q = 0; q < 4; ++q) P.put(q, CVf{xi[q], eta[q], col0[q], col1[q]});
-    P.stk(0) = stack_word(0, 4, 0);
-    int sp = 1;
     const float minA = d.minimal_area_f;
-    while (sp > 0) {
-        --sp;
-        const unsigned e = P.stk(sp);
-        const int pstart = (int)(e & 0xffu), num = (int)((e >> 8) & 0xffu), dim = (int)(e >> 16);
-        const int cc = 2 + dim;
-        float mn = P.at(pstart, cc), mx = mn;
-        for (int n = 1; n < num; ++n) { const float c = P.at(pstart + n, cc); mn = fminf(mn, c); mx = fmaxf(mx, c); }
-        int start = (int)ceilf(mn), end = (int)floorf(mx);
-        if (mn - float(start) == 0.f) start += 1;
-        if (mx - float(end) == 0.f) end -= 1;
-        bool cut = false;
-        if (start <= end) {
-            const float iso = float(start);
-            // the crossings bound what the cut writes: the parts away from vertex 0 (at most
-            // num - 1 + ncross vertices) from pstart + num, the part holding vertex 0 (at most
-            // num + ncross) from b0, after them
-            int ncross = 0;
-            bool sprev = (P.at(pstart + num - 1, cc) - iso) < 0.f;
-            for (int n = 0; n < num; ++n) {
-                const bool sn = (P.at(pstart + n, cc) - iso) < 0.f;
-                ncross += sn != sprev ? 1 : 0;
-                sprev = sn;
-            }
-            const int b0 = pstart + 2 * num - 1 + ncross;
-            if (b0 + num + ncross > kFastR - nst) return false;
-            int h0 = 0, h1 = 0, slot = 0, wpos = pstart + num, p1start = wpos, nchild = 0;
-            const CVf V0 = P.get(pstart);
-            CVf A = V0;
-            P.put(b0 + h0++, V0);
-            for (int n = 0; n < num; ++n) {
-                const CVf B = (n + 1 == num) ? V0 : P.get(pstart + n + 1);
-                const float v0 = cvc(A, dim) - iso, v1 = cvc(B, dim) - iso;
-                if ((v0 < 0.f) != (v1 < 0.f)) {
-                    cut = true;
-                    CVf X;
-                    const float t1 = cross_point(A, B, v0, v1, iso, dim, X);
-                    if (slot == 0) {
-                        P.put(b0 + h0++, X);
-                        slot = 1; h1 = 0; p1start = wpos;
-                        if (t1 < 1.0f) P.put(p1start + h1++, X);
-                    } else {
-                        P.put(p1start + h1++, X);
-                        // the part is complete: pushed where it lands after the parent is dropped
-                        if (sp >= kFastS) return false;
-                        P.stk(sp++) = stack_word(p1start - num, h1, dim);
-                        ++nchild;
-                        wpos = p1start + h1;
-                        slot = 0;
-                        if (t1 < 1.0f) P.put(b0 + h0++, X);
-                    }
+    Poly p{0x3210u, 4};
+    int stage = FS_RANGE0, iso = 0, end = 0, top = 4, sp = 0;   // top: vertex slots in use; sp: stack words
+    auto push = [&](const Poly& q, int st, int is, int en) {
+        P.stk(sp) = (unsigned)q.v;
+        P.stk(sp + 1) = (unsigned)q.num | (unsigned)st << 4 | (unsigned)top << 8;
+        P.stk(sp + 2) = ((unsigned)is & 0xffffu) | (unsigned)en << 16;
+        if constexpr (kEntry == 4) P.stk(sp + 3) = (unsigned)(q.v >> 32);
+        sp += kEntry;
+    };
+    for (;;) {
+        // the current polygon, cut until it is a piece
+        while (stage != FS_EMIT) {
+            const int dim = stage >> 1, cc = 2 + dim;
+            if (!(stage & 1)) {
+                float mn = P.at(p.id(0), cc), mx = mn;
+                typename Pool::list ids = p.v;
+                for (int n = 1; n < p.num; ++n) {
+                    ids >>= 4;
+                    const float c = P.at((int)(ids & 15u), cc);
+                    mn = fminf(mn, c); mx = fmaxf(mx, c);
                 }
-                if (n < num - 1) {
-                    if (slot == 0) P.put(b0 + h0++, B);
-                    else P.put(p1start + h1++, B);
-                }
-                A = B;
+                if (!(mn > -(float)kFastIso && mx < (float)kFastIso)) return false;
+                iso = (int)ceilf(mn); end = (int)floorf(mx);
+                if (mn - float(iso) == 0.f) iso += 1;
+                if (mx - float(end) == 0.f) end -= 1;
+                stage += iso <= end ? 1 : 2;
+                continue;
             }
-            if (nchild > 1) multi = true;
-            if (cut) {
-                if (slot != 0 || sp >= kFastS) return false;
-                // drop the parent: the parts move down by num, the part of vertex 0 follows them
-                for (int q = pstart + num; q < wpos; ++q) P.put(q - num, P.get(q));
-                for (int q = 0; q < h0; ++q) P.put(wpos - num + q, P.get(b0 + q));
-                P.stk(sp++) = stack_word(wpos - num, h0, dim);
+            // sides of the vertices and crossed edges (bit n: edge n -> n + 1)
+            const float fiso = float(iso);
+            unsigned side = 0;
+            typename Pool::list ids = p.v;
+            for (int n = 0; n < p.num; ++n, ids >>= 4) side |= (P.at((int)(ids & 15u), cc) - fiso < 0.f ? 1u : 0u) << n;
+            unsigned cross = side ^ ((side >> 1) | ((side & 1u) << (p.num - 1)));
+            int left = 0;
+            for (unsigned c = cross; c; c &= c - 1u) ++left;
+            if (left == 0 || (left & 1)) return false;
+            // each of the parts gets at most the parent's vertices and its crossings
+            if (top + left > kFastVerts || top + left > R - nst) return false;
+            const bool two = left == 2;
+            if (!two) {
+                if (p.num + left > kNum) return false;
+                multi = true;
+            }
+            Poly p0{0, 0}, child{0, 0};
+            int done = 0;    // parent's vertices taken so far
+            while (left > 0) {
+                // the next two crossings: away from vertex 0's part, and back
+                const int e1 = lowest_bit(cross);
+                cross &= cross - 1u;
+                const int e2 = lowest_bit(cross);
+                cross &= cross - 1u;
+                left -= 2;
+                if (p.num - (e2 - e1) + 2 > kNum || e2 - e1 + 2 > kNum) return false;
+                const CVf A = P.get(p.id(e1)), B = P.get(p.id(e1 + 1));
+                const CVf C = P.get(p.id(e2)), D = P.get(p.id(e2 + 1 == p.num ? 0 : e2 + 1));
+                CVf X, Y;
+                const float t1 = cross_point(A, B, cvc(A, dim) - fiso, cvc(B, dim) - fiso, fiso, dim, X);
+                const float u1 = cross_point(C, D, cvc(C, dim) - fiso, cvc(D, dim) - fiso, fiso, dim, Y);
+                P.put(top, X);
+                P.put(top + 1, Y);
+                p0.add(p, done, e1 + 1 - done);
+                p0.add(top);
+                if (u1 < 1.0f) p0.add(top + 1);
+                child = Poly{0, 0};
+                if (t1 < 1.0f) child.add(top);
+                child.add(p, e1 + 1, e2 - e1);
+                child.add(top + 1);
+                done = e2 + 1;
+                top += 2;
+                if (left > 0 || !two) {
+                    if (sp + kEntry > S) return false;
+                    push(child, stage - 1, 0, 0);    // its range is taken again
+                }
+            }
+            if (done < p.num) p0.add(p, done, p.num - done);
+            if (two) {
+                // the part below the line is done with this colour; the one above goes on at the
+                // next line
+                if (sp + kEntry > S) return false;
+                const bool low0 = side & 1u;
+                const int above = iso + 1 <= end ? stage : stage + 1;
+                push(child, low0 ? above : stage + 1, iso + 1, end);
+                stage = low0 ? stage + 1 : above;
+                ++iso;
+            } else {
+                stage -= 1;
+            }
+            p = p0;
+        }
+        if (p.num >= 3) {
+            const PoolVerts<Pool> V{P, p};
+            float cx, cy, area;
+            centroid_v(V, p.num, cx, cy, area);
+            if (area > minA) return false;      // triangulated by clip32
+            if (area != 0.f) {
+                ++npieces;
+                float4 pc;
+                if (piece_geom_v(g, V, p.num, cx, cy, pc)) {
+                    ny.add(pc.w);
+                    const int slotp = R - 1 - nst;
+                    if (slotp < top) return false;
+                    P.at(slotp, 0) = pc.x; P.at(slotp, 1) = pc.y; P.at(slotp, 2) = pc.z; P.at(slotp, 3) = pc.w;
+                    ++nst;
+                }
             }
         }
-        if (!cut) {
-            if (dim == 0) {
-                if (sp >= kFastS) return false;
-                P.stk(sp++) = stack_word(pstart, num, 1);
-            } else if (num >= 3) {
-                const PoolVerts V{P, pstart};
-                float cx, cy, area;
-                centroid_v(V, num, cx, cy, area);
-                if (area > minA) return false;      // triangulated by clip32
-                if (area != 0.f) {
-                    ++npieces;
-                    float4 pc;
-                    if (piece_geom_v(g, V, num, cx, cy, pc)) {
-                        ny.add(pc.w);
-                        const int slotp = kFastR - 1 - nst;
-                        if (slotp < pstart) return false;   // the polygon above pstart is spent
-                        P.at(slotp, 0) = pc.x; P.at(slotp, 1) = pc.y; P.at(slotp, 2) = pc.z; P.at(slotp, 3) = pc.w;
-                        ++nst;
-                    }
-                }
-            }
-        }
+        if (sp == 0) return true;
+        sp -= kEntry;
+        const unsigned m = P.stk(sp + 1), w = P.stk(sp + 2);
+        p = Poly{P.stk(sp), (int)(m & 15u)};
+        if constexpr (kEntry == 4) p.v |= (typename Pool::list)P.stk(sp + 3) << 32;
+        stage = (int)(m >> 4) & 15;
+        top = (int)(m >> 8);
+        iso = (int)(short)(w & 0xffffu);
+        end = (int)(short)(w >> 16);
     }
-    return true;
 }
 
 // the upper cell's vertex order (v0, v3, v2, v1)
