@@ -223,7 +223,8 @@ constexpr int kQuadThreads = 128;
 // Density: bound by the L1 data path (86% busy; issue slots 64%, 16 warps per SM by registers): a
 // piece reads 42 + 6 records of 32 bytes, and the lanes of a warp spread over several cells.  One
 // launch on the main pass at 128^3 (18.6M pieces): 4.99 ms evaluating every 1D interpolant from its
-// samples, 2.22 ms now; a density step's launches at 256^3: 44.5 -> 21.4 ms.  Measured beside it:
+// samples, 2.12 ms now; a density step's launches at 256^3: 44.5 -> 21.0 ms.  Measured beside it, with
+// 2.58 and 21.3 ms at that time:
 // five CTAs per SM 2.88 against 2.58 ms a step (spills), three 2.84; the records as two planes of
 // 16 bytes 2.50 (but 21.8 against 21.3 ms at 256^3); the pieces of a warp's faces interleaved
 // in the store 2.67, with planes 2.48 and 21.7.

@@ -18,7 +18,7 @@
 // samples only, so a jump outside them does not reach it.  The differences and the q_i are functions of the
 // samples only (WENO6_interpolation_3d.cpp:70-123; equal in exact arithmetic, and a little closer
 // to it in FP32: 3.1e-7 against 3.8e-7 of a 128^3 density step).  17 arithmetic instructions and
-// two 16-byte loads from a record, against about 62 and six 4-byte loads from the samples.
+// one 32-byte load from a record, against about 62 and six 4-byte loads from the samples.
 //
 // WenoSamples (velocity).  weno6_eval's own arithmetic (fia_device.cuh), bit for bit, from
 // records that hold the samples and their reciprocal indicators.  The pressure of the projection
@@ -172,11 +172,25 @@ __device__ __forceinline__ WenoData<T> weno_unpack(const WenoRec<T>& r) {
     return WenoData<T>{r.f, r.d, r.s1, r.s2, r.t0, r.t2, r.q0, (T(1) - r.q0) - r.q2, r.q2};
 }
 
+// 32 bytes of a record in one load (p 32-byte aligned: records are multiples of 32 bytes from the
+// base of an allocation): half the requests of two 16-byte loads.  The quadrature of a density step
+// at 128^3 takes 2.50 ms, 2.61 with two; of a velocity step on 120 x 161 x 77 cells 7.25, 7.39.
+__device__ __forceinline__ void ldg32(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+__device__ __forceinline__ void ldg32(const double* p, double& a, double& b, double& c, double& d) {
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p));
+}
+
 // FP64 records: eight doubles
 __device__ __forceinline__ WenoRec<double> ldg_rec(const WenoRec<double>* p) {
-    const double2* q = reinterpret_cast<const double2*>(p);
-    const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2), d = __ldg(q + 3);
-    return WenoRec<double>{a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y};
+    const double* q = reinterpret_cast<const double*>(p);
+    WenoRec<double> r;
+    ldg32(q, r.f, r.d, r.s1, r.s2);
+    ldg32(q + 4, r.t0, r.t2, r.q0, r.q2);
+    return r;
 }
 
 struct WenoNewton {
@@ -202,8 +216,9 @@ struct WenoNewton {
         const float4* __restrict__ r;
         int stride;    // Mz + 1
         __device__ __forceinline__ Raw load(int row, int b1) const {
-            const float4* p = r + 2LL * (row * stride + b1);
-            return Raw{__ldg(p), __ldg(p + 1)};
+            Raw w;
+            ldg32(r + 2LL * (row * stride + b1), w.a, w.b);
+            return w;
         }
     };
     // of psi: the record's f is the pair's high word, the differences are the pairs'; the value is
@@ -213,8 +228,8 @@ struct WenoNewton {
         PsiLoad load;
         int stride, b1;
         __device__ __forceinline__ Data data(int row) const {
-            const float4* p = r + 2LL * (row * stride + b1);
-            Raw w{__ldg(p), __ldg(p + 1)};
+            Raw w;
+            ldg32(r + 2LL * (row * stride + b1), w.a, w.b);
             const float lo = __ldg(&load.a[row * (stride - 1) + (b1 > 0 ? b1 - 1 : 0)].y);
             w.a.x = (w.a.x - load.hi0) + (lo - load.lo0);
             return w.data();
@@ -276,7 +291,10 @@ struct WenoSamples {
         int stride;
         __device__ __forceinline__ Raw load(int row, int b1) const {
             const int i = row * stride + b1;
-            return Raw{__ldg(r + 2LL * i), __ldg(r + 2LL * i + 1), __ldg(r2 + i)};
+            Raw w;
+            ldg32(r + 2LL * i, w.a, w.b);
+            w.c = __ldg(r2 + i);
+            return w;
         }
     };
     // psi relative to the face's base pair: the samples depend on the face, so their data are
