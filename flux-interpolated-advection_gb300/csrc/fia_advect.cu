@@ -4,7 +4,7 @@
 // move_substances_3d.cpp:585-841, and its velocity counterpart
 // advect_velocity_flux_advection_3d.cpp:252-576) becomes four kernels:
 //
-//   k_psi        one thread per (x,z) column: psi = running y-integral of the field
+//   k_psi_inc, k_psi_scan  psi = running y-integral of the field: the cells' increments, their sums
 //                (calc_psi_3D.cpp:10-308, :311-537)
 //   k_backtrace  one thread per UNIQUE cell vertex: x' = x - dt u(x), pin rule, clamp
 //                (calc_backtraced_face_3D.cpp:9-160).  The reference backtraces every
@@ -103,41 +103,92 @@ PassDesc desc32(const PassDesc& d) {
 }
 
 // ------------------------------------------------------------------------------------
-// psi: one thread per column (i,k); psi(.,0,.) = 0, psi(.,j,.) = psi(.,j-1,.) + incr(j-1)
+// psi(.,0,.) = 0, psi(.,j,.) = psi(.,j-1,.) + incr(j-1): the cells' increments, then their sums
 // ------------------------------------------------------------------------------------
-template <typename T>
-__global__ void k_psi(PassDesc d, const T* __restrict__ a, T* __restrict__ psi) {
+// The increment of cell (i, c, k) goes to psi row c + 1; a thread takes kPsiRun cells of a column.
+// WENO6: cell c spans [c + oy - 1/2, c + oy + 1/2] cells, k Gauss points per half, at offsets from
+// the nodes that no cell changes; the stencil data of its second half (base c) serve the first half
+// of cell c + 1.  Bound by the FP64 pipe.  The psi of a 64^3 plain-form step took 2.0 ms of 22.4 as one
+// thread per column (4096 chains of 64 cells, every point from its samples), 0.13 now.
+constexpr int kPsiRun = 4, kPsiThreads = 128;
+template <typename T, int MODE>
+__global__ void __launch_bounds__(kPsiThreads) k_psi_inc(PassDesc d, const T* __restrict__ a, T* __restrict__ psi) {
+    __shared__ WenoPos<T> pos[2 * kMaxGauss];
+    const T h = T(d.h);
+    if constexpr (MODE == PSI_WENO6) {
+        if (threadIdx.x < 2 * d.k) {
+            const int half = (int)threadIdx.x >= d.k, q = threadIdx.x - half * d.k;
+            // from node c - 1 in the first half, from node c in the second
+            const T y = T(0.25) * (T(1) + T(d.gx[q]));
+            pos[threadIdx.x] = weno_pos(half ? y : y + T(0.5));
+        }
+        __syncthreads();
+    }
     const int Mx = d.A.Mx, My = d.A.My, Mz = d.A.Mz;
+    const int runs = (My + kPsiRun - 1) / kPsiRun;
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= (long long)Mx * runs * Mz) return;
+    const int k = (int)(id % Mz);
+    const long long t = id / Mz;
+    const int j0 = (int)(t % runs) * kPsiRun, i = (int)(t / runs);
+    const int j1 = min(j0 + kPsiRun, My);
+    if constexpr (MODE == PSI_WENO6) {
+        const T* col = a + idx3(d.A, i, 0, k);
+        T f[6];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) f[m] = ldg(col + (long long)clampi(j0 - 3 + m, My - 1) * Mz);
+        WenoData<T> w = weno_data(f);
+#pragma unroll 1
+        for (int j = j0; j < j1; ++j) {
+            T inc = T(0);
+#pragma unroll 1
+            for (int q = 0; q < d.k; ++q) inc += weno_at(w, pos[q]) * T(d.gw[q]);
+#pragma unroll
+            for (int m = 0; m < 5; ++m) f[m] = f[m + 1];
+            f[5] = ldg(col + (long long)clampi(j + 3, My - 1) * Mz);
+            w = weno_data(f);
+#pragma unroll 1
+            for (int q = 0; q < d.k; ++q) inc += weno_at(w, pos[d.k + q]) * T(d.gw[q]);
+            psi[idx3(d.P, i, j + 1, k)] = inc * (h / T(2));
+        }
+    } else {
+        const T px = (T(i) + T(d.A.ox)) * h, pz = (T(k) + T(d.A.oz)) * h;
+        for (int j = j0; j < j1; ++j) {
+            const T y0 = ((T(j) + T(0.25)) + T(d.A.oy) - T(0.5)) * h;
+            const T y1 = ((T(j) + T(0.75)) + T(d.A.oy) - T(0.5)) * h;
+            psi[idx3(d.P, i, j + 1, k)] =
+                lin3d(a, d.A, h, px, y0, pz) * (h / T(2)) + lin3d(a, d.A, h, px, y1, pz) * (h / T(2));
+        }
+    }
+}
+// one thread per (x, z) column, the increments loaded kScanAhead at a time (PLAIN: formed from the field)
+constexpr int kScanAhead = 16, kScanThreads = 64;
+template <typename T, bool PLAIN>
+__global__ void __launch_bounds__(kScanThreads) k_psi_scan(PassDesc d, const T* __restrict__ a, T* __restrict__ psi) {
+    const int My = d.A.My, Mz = d.A.Mz;
     const long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= (long long)Mx * Mz) return;
+    if (col >= (long long)d.A.Mx * Mz) return;
     const int i = (int)(col / Mz), k = (int)(col % Mz);
     const T h = T(d.h);
-    const T px = (T(i) + T(d.A.ox)) * h, pz = (T(k) + T(d.A.oz)) * h;
+    T* P = psi + idx3(d.P, i, 0, k);
+    const T* A = a + idx3(d.A, i, 0, k);
     T acc = T(0);
-    psi[idx3(d.P, i, 0, k)] = T(0);
-    for (int j = 1; j <= My; ++j) {
-        if (d.psi_mode == PSI_PLAIN) {
-            acc = acc + ldg(a + idx3(d.A, i, j - 1, k)) * h;
-        } else if (d.psi_mode == PSI_WENO6) {
-            // cell j-1 spans [(j-1+oy-.5)h, (j+oy-.5)h]; k Gauss points per half
-            const T ylo = (T(j) - T(1.0) + T(d.A.oy) - T(0.5)) * h;
-            const T ymid = (T(j) - T(0.5) + T(d.A.oy) - T(0.5)) * h;
-            const T yhi = (T(j) + T(d.A.oy) - T(0.5)) * h;
-            for (int half = 0; half < 2; ++half) {
-                const T lo = half ? ymid : ylo, hi = half ? yhi : ymid;
-                const T L = hi - lo;
-                for (int q = 0; q < d.k; ++q) {
-                    const T py = (L / T(2)) * T(d.gx[q]) + (L / T(2)) + lo;
-                    acc += weno6_1dy(a, d.A, h, px, py, pz) * (h / T(2)) * T(d.gw[q]);
-                }
-            }
-        } else {
-            const T y0 = ((T(j - 1) + T(0.25)) + T(d.A.oy) - T(0.5)) * h;
-            const T y1 = ((T(j - 1) + T(0.75)) + T(d.A.oy) - T(0.5)) * h;
-            const T a0 = lin3d(a, d.A, h, px, y0, pz), a1 = lin3d(a, d.A, h, px, y1, pz);
-            acc = acc + a0 * (h / T(2)) + a1 * (h / T(2));
+    *P = T(0);
+    auto at = [&](int j) { return PLAIN ? ldg(A + (long long)(j - 1) * Mz) * h : P[(long long)j * Mz]; };
+    int j = 1;
+    for (; j + kScanAhead - 1 <= My; j += kScanAhead) {
+        T v[kScanAhead];
+#pragma unroll
+        for (int m = 0; m < kScanAhead; ++m) v[m] = at(j + m);
+#pragma unroll
+        for (int m = 0; m < kScanAhead; ++m) {
+            acc = acc + v[m];
+            P[(long long)(j + m) * Mz] = acc;
         }
-        psi[idx3(d.P, i, j, k)] = acc;
+    }
+    for (; j <= My; ++j) {
+        acc = acc + at(j);
+        P[(long long)j * Mz] = acc;
     }
 }
 
@@ -964,7 +1015,12 @@ static inline unsigned blocks_for(long long n, int t) { return (unsigned)((n + t
 template <typename T>
 cudaError_t launch_psi(const PassDesc& d, const T* a, T* psi, cudaStream_t s) {
     const long long cols = (long long)d.A.Mx * d.A.Mz;
-    k_psi<T><<<blocks_for(cols, 128), 128, 0, s>>>(d, a, psi);
+    const unsigned inc = blocks_for(cols * ((d.A.My + kPsiRun - 1) / kPsiRun), kPsiThreads);
+    if (d.psi_mode == PSI_WENO6) k_psi_inc<T, PSI_WENO6><<<inc, kPsiThreads, 0, s>>>(d, a, psi);
+    else if (d.psi_mode == PSI_LINEAR) k_psi_inc<T, PSI_LINEAR><<<inc, kPsiThreads, 0, s>>>(d, a, psi);
+    const unsigned scan = blocks_for(cols, kScanThreads);
+    if (d.psi_mode == PSI_PLAIN) k_psi_scan<T, true><<<scan, kScanThreads, 0, s>>>(d, a, psi);
+    else k_psi_scan<T, false><<<scan, kScanThreads, 0, s>>>(d, a, psi);
     return cudaGetLastError();
 }
 

@@ -26,47 +26,123 @@ namespace fia {
 
 namespace {
 
+inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
+
 // ---------------------------------------------------------------------------------
-// psi as hi/lo pairs, one thread per (x,z) column
+// psi as hi/lo pairs: the cells' increments, then their running sums along y
 // ---------------------------------------------------------------------------------
-__global__ void k_psi32(PassDesc d, const float* __restrict__ a, float2* __restrict__ psi) {
+// The increment of cell (i, c, k) goes to psi row c + 1 as a (sum, compensation) pair.  A thread
+// takes kPsiRun cells of a column.  WENO6: cell c spans [c + oy - 1/2, c + oy + 1/2], so its points
+// lie below node c in the first half and above it in the second, at offsets that no cell changes:
+// the coefficients are formed once a block, and the stencil data of the second half serve the first
+// half of the next cell too.  The three psi of a density step at 128^3 took 360 us as one thread
+// a column, which evaluated every point from its samples and summed as it went (16384 threads, each a
+// chain of 128 cells): 78 us now, 30 of them these increments (bound by FP32 issue).  Runs of 8 cells
+// measure the same there, and 3% of a whole step more at 16^3.
+constexpr int kPsiRun = 4, kPsiThreads = 128;
+template <int MODE>
+__global__ void __launch_bounds__(kPsiThreads) k_psi_inc32(PassDesc d, const float* __restrict__ a,
+                                                           float2* __restrict__ psi) {
+    __shared__ WenoCoef<float> coef[2 * kMaxGauss];
+    const float hf = d.hf, oy = d.A.oyf;
+    if constexpr (MODE == PSI_WENO6) {
+        if (threadIdx.x < 2 * d.k) {
+            const int half = (int)threadIdx.x >= d.k, q = threadIdx.x - half * d.k;
+            const float y = ((oy - 0.5f) + 0.5f * float(half)) + 0.25f * (1.0f + d.gxf[q]);
+            int by;
+            float sy, t[6];
+            locate(0, y, oy, by, sy);
+#pragma unroll
+            for (int i = 0; i < 6; ++i) t[i] = sy + float(2 - i);
+            coef[threadIdx.x] = weno_coef(t);
+        }
+        __syncthreads();
+    }
     const int Mx = d.A.Mx, My = d.A.My, Mz = d.A.Mz;
-    const long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (col >= (long long)Mx * Mz) return;
-    const int i = (int)(col / Mz), k = (int)(col % Mz);
-    const PlainLoad L{a};
-    const float hf = d.hf;
-    float hi = 0.f, lo = 0.f;
-    psi[idx3(d.P, i, 0, k)] = make_float2(0.f, 0.f);
-    const float oy = d.A.oyf;
-    for (int j = 1; j <= My; ++j) {
-        Kahan inc;
-        if (d.psi_mode == PSI_PLAIN) {
-            inc.add(__ldg(a + idx3(d.A, i, j - 1, k)) * hf);
-        } else if (d.psi_mode == PSI_WENO6) {
-            // cell j-1 spans [j-1+oy-.5, j+oy-.5] in cells; anchor (i, j-1, k)
-            const int anc[3] = {i, j - 1, k};
-            for (int half = 0; half < 2; ++half) {
-                const float lo_y = (oy - 0.5f) + 0.5f * float(half);
-                for (int q = 0; q < d.k; ++q) {
-                    const float qq[3] = {d.A.oxf, lo_y + 0.25f * (1.0f + d.gxf[q]), d.A.ozf};
-                    inc.add(weno6_1dy_loc(L, d.A, anc, qq) * (0.5f * hf) * d.gwf[q]);
-                }
-            }
-        } else {
-            const int anc[3] = {i, j - 1, k};
-            const float q0[3] = {d.A.oxf, 0.25f + oy - 0.5f, d.A.ozf};
-            const float q1[3] = {d.A.oxf, 0.75f + oy - 0.5f, d.A.ozf};
+    const int runs = (My + kPsiRun - 1) / kPsiRun;
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= (long long)Mx * runs * Mz) return;
+    const int k = (int)(id % Mz);
+    const long long t = id / Mz;
+    const int j0 = (int)(t % runs) * kPsiRun, i = (int)(t / runs);
+    const int j1 = min(j0 + kPsiRun, My);
+    if constexpr (MODE == PSI_WENO6) {
+        const float* col = a + idx3(d.A, i, 0, k);
+        float f[6];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) f[m] = __ldg(col + (long long)clampi(j0 - 3 + m, My - 1) * Mz);
+        Weno6Data w = weno6_data(f);
+#pragma unroll 1
+        for (int j = j0; j < j1; ++j) {
+            Kahan inc;
+#pragma unroll 1
+            for (int q = 0; q < d.k; ++q) inc.add(weno6_at(w, coef[q]) * (0.5f * hf) * d.gwf[q]);
+#pragma unroll
+            for (int m = 0; m < 5; ++m) f[m] = f[m + 1];
+            f[5] = __ldg(col + (long long)clampi(j + 3, My - 1) * Mz);
+            w = weno6_data(f);
+#pragma unroll 1
+            for (int q = 0; q < d.k; ++q) inc.add(weno6_at(w, coef[d.k + q]) * (0.5f * hf) * d.gwf[q]);
+            psi[idx3(d.P, i, j + 1, k)] = make_float2(inc.s, inc.c);
+        }
+    } else {
+        const PlainLoad L{a};
+        const float q0[3] = {d.A.oxf, 0.25f + oy - 0.5f, d.A.ozf};
+        const float q1[3] = {d.A.oxf, 0.75f + oy - 0.5f, d.A.ozf};
+        for (int j = j0; j < j1; ++j) {
+            const int anc[3] = {i, j, k};
+            Kahan inc;
             inc.add(lin3d_loc(L, d.A, anc, q0) * (0.5f * hf));
             inc.add(lin3d_loc(L, d.A, anc, q1) * (0.5f * hf));
+            psi[idx3(d.P, i, j + 1, k)] = make_float2(inc.s, inc.c);
         }
+    }
+}
+// The running sums, one thread per (x, z) column; the cells' increments are loaded kScanAhead at a
+// time (PLAIN: formed from the field).
+constexpr int kScanAhead = 16, kScanThreads = 64;
+template <bool PLAIN>
+__global__ void __launch_bounds__(kScanThreads) k_psi_scan32(PassDesc d, const float* __restrict__ a,
+                                                             float2* __restrict__ psi) {
+    const int My = d.A.My, Mz = d.A.Mz;
+    const long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (col >= (long long)d.A.Mx * Mz) return;
+    const int i = (int)(col / Mz), k = (int)(col % Mz);
+    float2* P = psi + idx3(d.P, i, 0, k);
+    const float* A = a + idx3(d.A, i, 0, k);
+    float hi = 0.f, lo = 0.f;
+    *P = make_float2(0.f, 0.f);
+    auto add = [&](int j, float2 v) {
+        Kahan inc;
+        if (PLAIN) inc.add(v.x * d.hf);
+        else inc = Kahan{v.x, v.y};
         // (hi, lo) += inc
         float s, e;
         two_sum(hi, inc.s, s, e);
         e += lo + inc.c;
         two_sum(s, e, hi, lo);
-        psi[idx3(d.P, i, j, k)] = make_float2(hi, lo);
+        P[(long long)j * Mz] = make_float2(hi, lo);
+    };
+    auto at = [&](int j) {
+        return PLAIN ? make_float2(__ldg(A + (long long)(j - 1) * Mz), 0.f) : P[(long long)j * Mz];
+    };
+    int j = 1;
+    for (; j + kScanAhead - 1 <= My; j += kScanAhead) {
+        float2 v[kScanAhead];
+#pragma unroll
+        for (int m = 0; m < kScanAhead; ++m) v[m] = at(j + m);
+#pragma unroll
+        for (int m = 0; m < kScanAhead; ++m) add(j + m, v[m]);
     }
+    for (; j <= My; ++j) add(j, at(j));
+}
+void psi32(const PassDesc& d, const float* a, float2* psi, cudaStream_t s) {
+    const long long cols = (long long)d.A.Mx * d.A.Mz;
+    const unsigned inc = nblk(cols * ((d.A.My + kPsiRun - 1) / kPsiRun), kPsiThreads);
+    if (d.psi_mode == PSI_WENO6) k_psi_inc32<PSI_WENO6><<<inc, kPsiThreads, 0, s>>>(d, a, psi);
+    else if (d.psi_mode == PSI_LINEAR) k_psi_inc32<PSI_LINEAR><<<inc, kPsiThreads, 0, s>>>(d, a, psi);
+    if (d.psi_mode == PSI_PLAIN) k_psi_scan32<true><<<nblk(cols, kScanThreads), kScanThreads, 0, s>>>(d, a, psi);
+    else k_psi_scan32<false><<<nblk(cols, kScanThreads), kScanThreads, 0, s>>>(d, a, psi);
 }
 
 // ---------------------------------------------------------------------------------
@@ -755,7 +831,6 @@ __global__ void k_gather32(PassDesc d, const float2* __restrict__ fx, const floa
     else out[id] = out[id] + val;
 }
 
-inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 // blocks of t threads over the faces of the three families (faces at rest: the y-faces)
 inline FamilyBlocks family_blocks(const long long* nface, bool rest, int t) {
     FamilyBlocks fb;
@@ -852,8 +927,7 @@ cudaError_t run_pass<float>(const PassDesc& d64, const VelocityFields& vel64, co
     VelocityFields vel = vel64;
     vel.fu = field32(vel64.fu); vel.fv = field32(vel64.fv); vel.fw = field32(vel64.fw);
     float2* psi = (float2*)w.psi;
-    const long long cols = (long long)d.A.Mx * d.A.Mz;
-    k_psi32<<<nblk(cols, 128), 128, 0, s>>>(d, a, psi);
+    psi32(d, a, psi, s);
     if (d.interp == INTERP_WENO6 && w.arec) {
         // without the y-integral no point of the field itself is interpolated
         if (d.comp >= 0) {
@@ -938,8 +1012,7 @@ void piece_store_free(PieceStore& p) {
 template <>
 cudaError_t launch_psi<float>(const PassDesc& d64, const float* a, float* psi, cudaStream_t s) {
     const PassDesc d = desc32(d64);
-    const long long cols = (long long)d.A.Mx * d.A.Mz;
-    k_psi32<<<nblk(cols, 128), 128, 0, s>>>(d, a, (float2*)psi);
+    psi32(d, a, (float2*)psi, s);
     return cudaGetLastError();
 }
 
