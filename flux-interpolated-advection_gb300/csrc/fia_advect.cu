@@ -21,6 +21,7 @@
 //                Deterministic, no atomics (the reference's per-thread += is racy).
 #include "fia_advect.cuh"
 #include "fia_weno_rec.cuh"
+#include "fia_trace.cuh"
 
 #include <cmath>
 #include <vector>
@@ -222,6 +223,7 @@ __device__ __forceinline__ double jitter_unit(long long id, int axis, unsigned s
     return (double)(x >> 11) * (2.0 / 9007199254740992.0) - 1.0;
 }
 
+// one thread a vertex: linear interpolation, and WENO6 without the collapse (PassDesc::full_weno)
 template <typename T>
 __global__ void k_backtrace(PassDesc d, const T* __restrict__ u, const T* __restrict__ v,
                             const T* __restrict__ w, NodeField fu, NodeField fv, NodeField fw,
@@ -241,11 +243,9 @@ __global__ void k_backtrace(PassDesc d, const T* __restrict__ u, const T* __rest
         pinned = (vi <= 1 || vi >= d.N[d.comp]);
     }
     if (!pinned) {
-        // at the rest position WENO6 collapses along the axes on which the vertex lies on a node
-        // plane of the component's lattice (weno6_3d_collapse)
-        const T vx = interp_c(d, d.interp, u, fu, h, p[0], p[1], p[2]);
-        const T vy = interp_c(d, d.interp, v, fv, h, p[0], p[1], p[2]);
-        const T vz = interp_c(d, d.interp, w, fw, h, p[0], p[1], p[2]);
+        const T vx = interp(d.interp, u, fu, h, p[0], p[1], p[2]);
+        const T vy = interp(d.interp, v, fv, h, p[0], p[1], p[2]);
+        const T vz = interp(d.interp, w, fw, h, p[0], p[1], p[2]);
         const T dt = T(d.dt);
         p[0] -= vx * dt; p[1] -= vy * dt; p[2] -= vz * dt;
         if (d.vertex_jitter != 0.0)
@@ -260,6 +260,35 @@ __global__ void k_backtrace(PassDesc d, const T* __restrict__ u, const T* __rest
         if (p[c] > hi) p[c] = hi;
     }
     verts[3 * id + 0] = p[0]; verts[3 * id + 1] = p[1]; verts[3 * id + 2] = p[2];
+}
+
+// The same with WENO6 collapsed on the node planes, a tile of vertices and one velocity component a
+// block (fia_trace.cuh).
+template <int N>
+__global__ void __launch_bounds__(kTraceThreads) k_trace64(PassDesc d, const double* __restrict__ u,
+                                                           const double* __restrict__ v, const double* __restrict__ w,
+                                                           NodeField fu, NodeField fv, NodeField fw,
+                                                           double* __restrict__ verts, TraceTiles tiles) {
+    extern __shared__ double trace_sm[];
+    const int c = blockIdx.y;
+    const double* a = c == 0 ? u : (c == 1 ? v : w);
+    const NodeField F = c == 0 ? fu : (c == 1 ? fv : fw);
+    const double off[3] = {F.ox, F.oy, F.oz}, h = d.h;
+    const int L[3] = {d.A.Mx + 1, d.A.My + 1, d.A.Mz + 1};
+    const double q[3] = {d.comp == 0 ? -0.5 : 0.0, d.comp == 1 ? -0.5 : 0.0, d.comp == 2 ? -0.5 : 0.0};
+    const double e = c == d.comp ? 0.5 * h : 0.0;
+    const double lo = -e, hi = h * double(c == 0 ? d.N[0] : (c == 1 ? d.N[1] : d.N[2])) + e;
+    const int Np = d.comp == 0 ? d.N[0] : (d.comp == 1 ? d.N[1] : d.N[2]);
+    trace_tile<N, TraceCoef64>(a, F, off, L, q, tiles, trace_sm, [&](int i, int j, int k, double val) {
+        const int vi = d.comp == 0 ? i : (d.comp == 1 ? j : k);
+        const long long id = ((long long)i * L[1] + j) * L[2] + k;
+        double p = double(c == 0 ? i : (c == 1 ? j : k)) * h - e;
+        if (!(d.comp >= 0 && (vi <= 1 || vi >= Np))) {
+            p -= val * d.dt;
+            if (d.vertex_jitter != 0.0) p += d.vertex_jitter * jitter_unit(id, c, d.jitter_seed) * h;
+        }
+        verts[3 * id + c] = p < lo ? lo : (p > hi ? hi : p);
+    });
 }
 
 // Second trace of the flux MacCormack scheme (calc_backtraced_face_3D.cpp:9-128, time
@@ -1026,6 +1055,20 @@ cudaError_t launch_psi(const PassDesc& d, const T* a, T* psi, cudaStream_t s) {
 
 template <typename T>
 cudaError_t launch_backtrace(const PassDesc& d, const VelocityFields& vel, T* verts, cudaStream_t s) {
+    if constexpr (sizeof(T) == sizeof(double)) {
+        // as in the chosen form: 8 x 8 tiles, 4 x 4 where those would leave SMs without a block
+        if (d.interp == INTERP_WENO6 && !d.full_weno) {
+            const int L[3] = {d.A.Mx + 1, d.A.My + 1, d.A.Mz + 1};
+            const TraceTiles t8 = trace_tiles(L, 8, 16), t4 = trace_tiles(L, 4, 16);
+            const bool big = 3 * trace_blocks(L, 8, t8) >= 152 * 2;
+            const TraceTiles t = big ? t8 : t4;
+            const dim3 g(trace_blocks(L, big ? 8 : 4, t), 3);
+            const double *u = (const double*)vel.u, *v = (const double*)vel.v, *w = (const double*)vel.w;
+            if (big) k_trace64<8><<<g, kTraceThreads, trace_smem(8, t, 8), s>>>(d, u, v, w, vel.fu, vel.fv, vel.fw, verts, t);
+            else k_trace64<4><<<g, kTraceThreads, trace_smem(4, t, 8), s>>>(d, u, v, w, vel.fu, vel.fv, vel.fw, verts, t);
+            return cudaGetLastError();
+        }
+    }
     const long long n = (long long)(d.A.Mx + 1) * (d.A.My + 1) * (d.A.Mz + 1);
     k_backtrace<T><<<blocks_for(n, 128), 128, 0, s>>>(d, (const T*)vel.u, (const T*)vel.v, (const T*)vel.w,
                                                       vel.fu, vel.fv, vel.fw, verts);
