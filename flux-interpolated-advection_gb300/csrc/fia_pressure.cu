@@ -14,7 +14,9 @@
 #include "fia_pressure.cuh"
 
 #include <algorithm>
+#include <type_traits>
 #include <cmath>
+#include <cstdint>
 
 namespace fia {
 
@@ -111,6 +113,34 @@ __device__ double block_total(const double* part, int nblocks, int q) {
     }
     __syncthreads();
     return tot;
+}
+
+// The same for NV rows at once (each in block_total's order): row after row, the last block's loads,
+// shuffles and barriers are waited for NV times.
+template <int NV>
+__device__ __forceinline__ void block_totals(const double* part, int nblocks, double (&tot)[NV]) {
+    __shared__ double sh[NV][33];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double s[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) s[q] = 0.0;
+    for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) s[q] += __ldcg(part + b + nblocks * q);
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        s[q] = warp_sum(s[q]);
+        if (lane == 0) sh[q][wid] = s[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        double t = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[threadIdx.x][w];
+        sh[threadIdx.x][32] = t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NV; ++q) tot[q] = sh[q][32];
 }
 
 // ---------------------------------------------------------------------------------
@@ -415,12 +445,12 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_direction_apply(PoissonGrid 
     }
     block_dots<T, 2>(acc, part);
     if (last_block(ticket)) {
-        const double t = block_total(part, gridDim.x, 0);
-        const double tr = rres ? block_total(part, gridDim.x, 1) : 0.0;
+        double t[2];
+        block_totals<2>(part, gridDim.x, t);   // without rres the second is zero
         if (threadIdx.x == 0) {
-            const double num = rres ? tr : scal[S_RZ];
-            scal[S_ALPHA] = t != 0.0 ? num / t : 0.0;
-            scal[S_DQ] = t;
+            const double num = rres ? t[1] : scal[S_RZ];
+            scal[S_ALPHA] = t[0] != 0.0 ? num / t[0] : 0.0;
+            scal[S_DQ] = t[0];
             *ticket = 0;
         }
     }
@@ -481,16 +511,16 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update(PoissonGrid g, double
     }
     block_dots<T, 2>(acc, part);
     if (last_block(ticket)) {
-        const double trz = block_total(part, gridDim.x, 0);
-        const double trr = block_total(part, gridDim.x, 1);
+        double t[2];
+        block_totals<2>(part, gridDim.x, t);
         if (threadIdx.x == 0) {
             if (jacobi) {
-                scal[S_BETA] = scal[S_RZ] != 0.0 ? trz / scal[S_RZ] : 0.0;
-                scal[S_RZ] = trz;
+                scal[S_BETA] = scal[S_RZ] != 0.0 ? t[0] / scal[S_RZ] : 0.0;
+                scal[S_RZ] = t[0];
             }
-            scal[S_RR] = trr;
+            scal[S_RR] = t[1];
             scal[S_ITERS] += 1.0;
-            if (trr <= scal[S_THRESH]) scal[S_DONE] = 1.0;
+            if (t[1] <= scal[S_THRESH]) scal[S_DONE] = 1.0;
             *ticket = 0;
         }
     }
@@ -837,38 +867,78 @@ struct DirSet {
     int n;
 };
 
-template <typename T, int W>
+// The number NQ of kept directions is a template argument: tested inside the loop it keeps each
+// vector's load behind the test.  Bound by HBM: 67 MB a vector at 256^3, ten vectors with eight
+// directions (floor 99 us).  Copied to the thread's own shared slots, two groups of all vectors are in
+// flight (kDotsSmem; 2 CTAs per SM): 134 us, 139 with the loads in registers, a few at a time.
+constexpr int kDotsStages = 2;
+template <typename T, int W, int NQ>
+constexpr int kDotsSmem = W * sizeof(T) == 16 ? kDotsStages * (NQ + 2) * kRedThreads * 16 : 0;
+template <typename T, int W, int NQ>
 __global__ void __launch_bounds__(kRedThreads) k_fcgm_dots(unsigned n, double* __restrict__ scal, const T* __restrict__ z,
                                                             const T* __restrict__ r, DirSet<T> qs, double* part,
                                                             unsigned* ticket) {
     if (scal[S_DONE] != 0.0) return;
-    const unsigned ngr = n / W;
-    DotAcc<T> acc[kFcgMaxDirs + 1];   // z.q_j, then z.r
-    for (unsigned gi = blockIdx.x * blockDim.x + threadIdx.x; gi < ngr; gi += gridDim.x * blockDim.x) {
-        const unsigned c0 = gi * W;
-        T zv[W], v[W];
-        ldv<T, W>(z + c0, zv);
-        ldv<T, W>(r + c0, v);
+    const unsigned ngr = n / W, step = gridDim.x * blockDim.x, g0 = blockIdx.x * blockDim.x + threadIdx.x;
+    DotAcc<T> acc[NQ + 1];   // z.q_j, then z.r
+    auto vec = [&](int v) { return v == 0 ? z : (v == 1 ? r : qs.v[v < 2 ? 0 : v - 2]); };
+    auto add = [&](const T (&zv)[W], const T (&v)[W], int j) {
 #pragma unroll
-        for (int e = 0; e < W; ++e) acc[kFcgMaxDirs].add(zv[e], v[e]);
+        for (int e = 0; e < W; ++e) acc[j].add(zv[e], v[e]);
+    };
+    if constexpr (W * sizeof(T) == 16) {
+        extern __shared__ __align__(16) unsigned char dots_smem[];
+        unsigned char* mine = dots_smem + threadIdx.x * 16;
+        const uint32_t base = (uint32_t)__cvta_generic_to_shared(mine);
+        auto slot = [](int stage, int v) { return (stage * (NQ + 2) + v) * (kRedThreads * 16); };
+        auto issue = [&](unsigned gi, int stage) {
+            if (gi < ngr)
 #pragma unroll
-        for (int j = 0; j < kFcgMaxDirs; ++j) {
-            if (j >= qs.n) break;
-            ldv<T, W>(qs.v[j] + c0, v);
+                for (int v = 0; v < NQ + 2; ++v)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(base + slot(stage, v)),
+                                 "l"(vec(v) + (size_t)gi * W)
+                                 : "memory");
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
 #pragma unroll
-            for (int e = 0; e < W; ++e) acc[j].add(zv[e], v[e]);
+        for (int k = 0; k < kDotsStages; ++k) issue(g0 + k * step, k);
+        int stage = 0;
+        for (unsigned gi = g0; gi < ngr; gi += step) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kDotsStages - 1) : "memory");
+            T zv[W], v[W];
+            ldv<T, W>(reinterpret_cast<const T*>(mine + slot(stage, 0)), zv);
+#pragma unroll
+            for (int j = 0; j < NQ; ++j) {
+                ldv<T, W>(reinterpret_cast<const T*>(mine + slot(stage, 2 + j)), v);
+                add(zv, v, j);
+            }
+            ldv<T, W>(reinterpret_cast<const T*>(mine + slot(stage, 1)), v);
+            add(zv, v, NQ);
+            issue(gi + kDotsStages * step, stage);
+            stage = stage + 1 == kDotsStages ? 0 : stage + 1;
+        }
+    } else {
+        for (unsigned gi = g0; gi < ngr; gi += step) {
+            T zv[W], v[W];
+            ldv<T, W>(z + gi * W, zv);
+#pragma unroll
+            for (int j = 0; j <= NQ; ++j) {
+                ldv<T, W>((j < NQ ? qs.v[j < NQ ? j : 0] : r) + gi * W, v);
+                add(zv, v, j);
+            }
         }
     }
-    block_dots<T, kFcgMaxDirs + 1>(acc, part);
+    block_dots<T, NQ + 1>(acc, part);
     if (last_block(ticket)) {
-        double t[kFcgMaxDirs + 1];
-        for (int j = 0; j <= kFcgMaxDirs; ++j) t[j] = (j < qs.n || j == kFcgMaxDirs) ? block_total(part, gridDim.x, j) : 0.0;
+        double t[NQ + 1];
+        block_totals<NQ + 1>(part, gridDim.x, t);
         if (threadIdx.x == 0) {
-            for (int j = 0; j < qs.n; ++j) {
+#pragma unroll
+            for (int j = 0; j < NQ; ++j) {
                 const double dq = scal[S_DQJ + qs.slot[j]];
                 scal[S_BETAJ + qs.slot[j]] = dq != 0.0 ? -t[j] / dq : 0.0;
             }
-            scal[S_RZ] = t[kFcgMaxDirs];
+            scal[S_RZ] = t[NQ];
             *ticket = 0;
         }
     }
@@ -876,116 +946,89 @@ __global__ void __launch_bounds__(kRedThreads) k_fcgm_dots(unsigned n, double* _
 
 // d_new = z + sum_j beta_j d_j (streamed once; the stencil kernel below then reads d_new
 // instead of recomputing it for each neighbour)
-template <typename T, int W>
+template <typename T, int W, int NQ>
 __global__ void __launch_bounds__(kRedThreads) k_fcgm_combine(unsigned n, const double* __restrict__ scal,
                                                                const T* __restrict__ z, DirSet<T> ds,
                                                                T* __restrict__ dnew) {
     if (scal[S_DONE] != 0.0) return;
     const unsigned ngr = n / W;
-    T beta[kFcgMaxDirs];
+    T beta[NQ + 1];
 #pragma unroll
-    for (int j = 0; j < kFcgMaxDirs; ++j) beta[j] = j < ds.n ? (T)scal[S_BETAJ + ds.slot[j]] : T(0);
+    for (int j = 0; j < NQ; ++j) beta[j] = (T)scal[S_BETAJ + ds.slot[j]];
     for (unsigned gi = blockIdx.x * blockDim.x + threadIdx.x; gi < ngr; gi += gridDim.x * blockDim.x) {
         const unsigned c0 = gi * W;
-        T o[W];
+        T o[W], b[NQ + 1][W];
         ldv<T, W>(z + c0, o);
 #pragma unroll
-        for (int j = 0; j < kFcgMaxDirs; ++j) {
-            if (j >= ds.n) break;
-            T b[W];
-            ldv<T, W>(ds.v[j] + c0, b);
+        for (int j = 0; j < NQ; ++j) ldv<T, W>(ds.v[j] + c0, b[j]);
 #pragma unroll
-            for (int e = 0; e < W; ++e) o[e] += beta[j] * b[e];
-        }
+        for (int j = 0; j < NQ; ++j)
+#pragma unroll
+            for (int e = 0; e < W; ++e) o[e] += beta[j] * b[j][e];
         stv<T, W>(dnew + c0, o);
     }
 }
 
-// q = B d for d = z + sum_j beta_j d_j (with ds.n = 0 and dnew null: d = z, already combined);
-// d.q and d.r; the last block sets alpha = d.r / d.q
-template <typename T, int W>
-__global__ void __launch_bounds__(kRedThreads) k_fcgm_direction(PoissonGrid g, double* __restrict__ scal,
-                                                                 const T* __restrict__ z, DirSet<T> ds,
-                                                                 T* __restrict__ dnew, T* __restrict__ qnew, int newslot,
-                                                                 const T* __restrict__ rres, double* part,
-                                                                 unsigned* ticket) {
+// q = B d;  d.q and d.r; the last block sets alpha = d.r / d.q.  The neighbours outside the grid
+// are read at the cell itself and not added, so that a group's loads wait for no test: 55 us at 256^3,
+// 117 with each behind its test (floor 30: d, r and q).
+template <typename T, int W, bool SOLID>
+__global__ void __launch_bounds__(kRedThreads) k_fcgm_apply(PoissonGrid g, double* __restrict__ scal,
+                                                             const T* __restrict__ d, T* __restrict__ qnew, int newslot,
+                                                             const T* __restrict__ rres, double* part, unsigned* ticket) {
     if (scal[S_DONE] != 0.0) return;
     const unsigned n = (unsigned)g.nx * g.ny * g.nz, ngr = n / W;
     const unsigned sx = (unsigned)g.ny * g.nz, sy = (unsigned)g.nz;
-    T beta[kFcgMaxDirs];
-#pragma unroll
-    for (int j = 0; j < kFcgMaxDirs; ++j) beta[j] = j < ds.n ? (T)scal[S_BETAJ + ds.slot[j]] : T(0);
-    auto dvec = [&](unsigned o0, T (&o)[W]) {
-        ldv<T, W>(z + o0, o);
-#pragma unroll
-        for (int j = 0; j < kFcgMaxDirs; ++j) {
-            if (j >= ds.n) break;
-            T b[W];
-            ldv<T, W>(ds.v[j] + o0, b);
-#pragma unroll
-            for (int e = 0; e < W; ++e) o[e] += beta[j] * b[e];
-        }
-    };
-    auto d1 = [&](unsigned o) -> T {
-        T v = z[o];
-        for (int j = 0; j < ds.n; ++j) v += beta[j] * ds.v[j][o];
-        return v;
-    };
+    const int pin = g.pin;
+    auto solid = [&](unsigned o) { return SOLID && g.solid[o] != 0; };
     DotAcc<T> acc[2];
     for (unsigned gi = blockIdx.x * blockDim.x + threadIdx.x; gi < ngr; gi += gridDim.x * blockDim.x) {
         const unsigned c0 = gi * W;
         const Cell k = decode(c0, g.ny, g.nz);
-        T dc[W], s[W];
+        const bool in[6] = {k.ix > 0, k.ix < g.nx - 1, k.iy > 0, k.iy < g.ny - 1, k.iz > 0, k.iz + W < g.nz};
+        const unsigned at[4] = {in[0] ? c0 - sx : c0, in[1] ? c0 + sx : c0, in[2] ? c0 - sy : c0, in[3] ? c0 + sy : c0};
+        T dc[W], rv[W], nv[4][W], s[W];
         int dg[W];
-        dvec(c0, dc);
+        ldv<T, W>(d + c0, dc);
+#pragma unroll
+        for (int m = 0; m < 4; ++m) ldv<T, W>(d + at[m], nv[m]);
+        const T zl = d[in[4] ? c0 - 1 : c0], zr = d[in[5] ? c0 + W : c0];
+        ldv<T, W>(rres + c0, rv);
 #pragma unroll
         for (int e = 0; e < W; ++e) { s[e] = T(0); dg[e] = 0; }
-        auto side = [&](bool ok, unsigned o0) {
-            if (!ok) return;
-            T nv[W];
-            dvec(o0, nv);
 #pragma unroll
-            for (int e = 0; e < W; ++e) {
-                const unsigned o = o0 + e;
-                if (g.solid && g.solid[o]) continue;
-                ++dg[e];
-                if ((int)o != g.pin) s[e] += nv[e];
-            }
-        };
-        side(k.ix > 0, c0 - sx);
-        side(k.ix < g.nx - 1, c0 + sx);
-        side(k.iy > 0, c0 - sy);
-        side(k.iy < g.ny - 1, c0 + sy);
+        for (int m = 0; m < 4; ++m)
+#pragma unroll
+            for (int e = 0; e < W; ++e)
+                if (in[m] && !solid(at[m] + e)) {
+                    ++dg[e];
+                    if ((int)(at[m] + e) != pin) s[e] += nv[m][e];
+                }
+        T qv[W];
 #pragma unroll
         for (int e = 0; e < W; ++e) {
             const unsigned c = c0 + e;
-            if (e > 0 || k.iz > 0) {
-                const unsigned o = c - 1;
-                if (!(g.solid && g.solid[o])) { ++dg[e]; if ((int)o != g.pin) s[e] += e > 0 ? dc[e - 1] : d1(o); }
+            if ((e > 0 || in[4]) && !solid(c - 1)) {
+                ++dg[e];
+                if ((int)(c - 1) != pin) s[e] += e > 0 ? dc[e > 0 ? e - 1 : 0] : zl;
             }
-            if (e < W - 1 || k.iz + W < g.nz) {
-                const unsigned o = c + 1;
-                if (!(g.solid && g.solid[o])) { ++dg[e]; if ((int)o != g.pin) s[e] += e < W - 1 ? dc[e + 1] : d1(o); }
+            if ((e < W - 1 || in[5]) && !solid(c + 1)) {
+                ++dg[e];
+                if ((int)(c + 1) != pin) s[e] += e < W - 1 ? dc[e < W - 1 ? e + 1 : 0] : zr;
             }
-        }
-        T qv[W], rv[W];
-        ldv<T, W>(rres + c0, rv);
-#pragma unroll
-        for (int e = 0; e < W; ++e) {
-            qv[e] = excluded(g, c0 + e) ? T(0) : T(dg[e]) * dc[e] - s[e];
+            qv[e] = (int)c == pin || solid(c) ? T(0) : T(dg[e]) * dc[e] - s[e];
             acc[0].add(dc[e], qv[e]);
             acc[1].add(dc[e], rv[e]);
         }
-        if (dnew) stv<T, W>(dnew + c0, dc);
         stv<T, W>(qnew + c0, qv);
     }
     block_dots<T, 2>(acc, part);
     if (last_block(ticket)) {
-        const double t = block_total(part, gridDim.x, 0);
-        const double tr = block_total(part, gridDim.x, 1);
+        double t[2];
+        block_totals<2>(part, gridDim.x, t);
         if (threadIdx.x == 0) {
-            scal[S_ALPHA] = t != 0.0 ? tr / t : 0.0;
-            scal[S_DQJ + newslot] = t;
+            scal[S_ALPHA] = t[0] != 0.0 ? t[1] / t[0] : 0.0;
+            scal[S_DQJ + newslot] = t[0];
             *ticket = 0;
         }
     }
@@ -1242,7 +1285,6 @@ template <typename T>
 cudaError_t fcg_iteration(const PressureWork<T>& W, const PoissonGrid& g, const FcgBuffers<T>& B, int it, int m,
                           cudaStream_t s) {
     const unsigned n = (unsigned)g.nx * g.ny * g.nz;
-    const int nb = kRedBlocks, nt = kRedThreads;
     m = std::max(1, std::min(m, kFcgMaxDirs));
     const int ring = m + 1, newslot = it % ring;
     DirSet<T> qs, ds;
@@ -1252,20 +1294,39 @@ cudaError_t fcg_iteration(const PressureWork<T>& W, const PoissonGrid& g, const 
         qs.v[j] = B.q[sl]; qs.slot[j] = sl;
         ds.v[j] = B.d[sl]; ds.slot[j] = sl;
     }
-    constexpr int V = VecW<T>::W;
-    DirSet<T> none = ds;
-    none.n = 0;
-    if (g.nz % V == 0) {
-        k_fcgm_dots<T, V><<<nb, nt, 0, s>>>(n, W.scal, W.z, W.r, qs, W.part, W.ticket);
-        k_fcgm_combine<T, V><<<nb, nt, 0, s>>>(n, W.scal, W.z, ds, B.d[newslot]);
-        k_fcgm_direction<T, V><<<nb, nt, 0, s>>>(g, W.scal, B.d[newslot], none, (T*)nullptr, B.q[newslot], newslot,
-                                                 W.r, W.part + (kFcgMaxDirs + 1) * nb, W.ticket + 1);
-    } else {
-        k_fcgm_dots<T, 1><<<nb, nt, 0, s>>>(n, W.scal, W.z, W.r, qs, W.part, W.ticket);
-        k_fcgm_combine<T, 1><<<nb, nt, 0, s>>>(n, W.scal, W.z, ds, B.d[newslot]);
-        k_fcgm_direction<T, 1><<<nb, nt, 0, s>>>(g, W.scal, B.d[newslot], none, (T*)nullptr, B.q[newslot], newslot,
-                                                 W.r, W.part + (kFcgMaxDirs + 1) * nb, W.ticket + 1);
-    }
+    const int nb = kRedBlocks, nt = kRedThreads;
+    const T* dn = B.d[newslot];
+    T* qn = B.q[newslot];
+    double* part = W.part + (kFcgMaxDirs + 1) * nb;
+    cudaError_t err = cudaSuccess;
+    auto run = [&](auto w, auto nq) {
+        constexpr int V = decltype(w)::value, NQ = decltype(nq)::value;
+        constexpr int sm = kDotsSmem<T, V, NQ>;
+        if (sm > 0 && err == cudaSuccess)
+            err = cudaFuncSetAttribute(k_fcgm_dots<T, V, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        if (err != cudaSuccess) return;
+        k_fcgm_dots<T, V, NQ><<<nb, nt, sm, s>>>(n, W.scal, W.z, W.r, qs, W.part, W.ticket);
+        k_fcgm_combine<T, V, NQ><<<nb, nt, 0, s>>>(n, W.scal, W.z, ds, B.d[newslot]);
+        if (g.solid) k_fcgm_apply<T, V, true><<<nb, nt, 0, s>>>(g, W.scal, dn, qn, newslot, W.r, part, W.ticket + 1);
+        else k_fcgm_apply<T, V, false><<<nb, nt, 0, s>>>(g, W.scal, dn, qn, newslot, W.r, part, W.ticket + 1);
+    };
+    auto dirs = [&](auto w) {
+        static_assert(kFcgMaxDirs == 8, "one case a count");
+        switch (qs.n) {
+            case 0: run(w, std::integral_constant<int, 0>()); break;
+            case 1: run(w, std::integral_constant<int, 1>()); break;
+            case 2: run(w, std::integral_constant<int, 2>()); break;
+            case 3: run(w, std::integral_constant<int, 3>()); break;
+            case 4: run(w, std::integral_constant<int, 4>()); break;
+            case 5: run(w, std::integral_constant<int, 5>()); break;
+            case 6: run(w, std::integral_constant<int, 6>()); break;
+            case 7: run(w, std::integral_constant<int, 7>()); break;
+            default: run(w, std::integral_constant<int, 8>());
+        }
+    };
+    if (g.nz % VecW<T>::W == 0) dirs(std::integral_constant<int, VecW<T>::W>());
+    else dirs(std::integral_constant<int, 1>());
+    if (err != cudaSuccess) return err;
     launch_update<T>(W, g, B.d[newslot], false, W.part, W.ticket + 2, s, B.q[newslot]);
     return cudaGetLastError();
 }
