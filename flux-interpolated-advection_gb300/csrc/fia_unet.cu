@@ -160,6 +160,18 @@ __device__ __forceinline__ float load_scalar(const Src& s, int x, int y, int z) 
     return ((const float*)s.p)[vox(s.dims, x, y, z) * s.cstride + s.coff];
 }
 
+// The pooled input of a layer, once: staged by the convolutions themselves, each halo voxel was
+// averaged by every CTA whose halo holds it (2.8 times, and once per share of the output channels),
+// eight loads at a time.  The three pooled layers at 256^3 took 147 us; pooling and layers take 80.
+__global__ void k_pool(Src src, int d0, int d1, int d2, uint4* __restrict__ out) {
+    const int nu = src.C >> 3;
+    const unsigned n = (unsigned)d0 * d1 * d2 * nu;
+    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned v = i / nu, t = v / (unsigned)d2;
+        out[i] = load_unit(src, (int)(t / (unsigned)d1), (int)(t % (unsigned)d1), (int)(v - t * (unsigned)d2), (int)(i - v * nu) * 8);
+    }
+}
+
 // Stages the halo brick of the convolution input (channels-last, swizzled 16-byte units).
 __device__ void stage_units(const ConvArgs& a, uint4* sm, int bx, int by, int bz) {
     const int ncu = a.cin >> 3;
@@ -292,25 +304,37 @@ __global__ void __launch_bounds__(kConvThreads) k_conv2(ConvArgs a) {
         const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
         const int j = lane >> 3, i = lane & 7;
         const int m = i + ((j & 1) << 3), ku = j >> 1;
-        for (int tap = 0; tap < 27; ++tap) {
-            int dx, dy, dz;
-            tap_offsets(tap, dx, dy, dz);
-            uint32_t addr[MT];
+        // the weights of kAhead steps (a tap and 16 channels each) are in flight; loaded at their own
+        // step, each was waited for (64 -> 64 at 16^3: 25 us; a training step at 64^3 11% less)
+        constexpr int kAhead = NTL <= 2 ? 6 : (NTL <= 4 ? 3 : (NTL <= 6 ? 2 : 1));
+        const int steps = 27 * nc16;
+        const uint2* wt = a.wfrag + (size_t)n0 * 32 + lane;
+        uint2 wb[kAhead][NTL];
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                const int hv = ((mt + dx) * HY + (warp + dy)) * HZ + m + dz;
-                addr[mt] = sbase + (uint32_t)(hv * ncp + ku) * 16u;
-            }
-            const uint2* wt = a.wfrag + ((size_t)tap * nc16 * NT + n0) * 32 + lane;
-            for (int c16 = 0; c16 < nc16; ++c16) {
+        for (int p = 0; p < kAhead; ++p)
+#pragma unroll
+            for (int n = 0; n < NTL; ++n) wb[p][n] = __ldg(wt + ((size_t)min(p, steps - 1) * NT + n) * 32);
+        int dx = 0, dy = 0, dz = 0, c16 = 0;
+        for (int s0 = 0; s0 < steps; s0 += kAhead) {
+#pragma unroll
+            for (int p = 0; p < kAhead; ++p) {
+                if (s0 + p >= steps) break;
                 uint32_t A[MT][4];
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) ldsm_x4(A[mt], addr[mt] + c16 * 32);
+                for (int mt = 0; mt < MT; ++mt) {
+                    const int hv = ((mt + dx) * HY + (warp + dy)) * HZ + m + dz;
+                    ldsm_x4(A[mt], sbase + (uint32_t)(hv * ncp + ku) * 16u + c16 * 32);
+                }
 #pragma unroll
-                for (int n = 0; n < NTL; ++n) {
-                    const uint2 b = __ldg(wt + (c16 * NT + n) * 32);
+                for (int n = 0; n < NTL; ++n)
 #pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) mma_bf16(acc[mt][n], A[mt], b.x, b.y);
+                    for (int mt = 0; mt < MT; ++mt) mma_bf16(acc[mt][n], A[mt], wb[p][n].x, wb[p][n].y);
+#pragma unroll
+                for (int n = 0; n < NTL; ++n)
+                    wb[p][n] = __ldg(wt + ((size_t)min(s0 + p + kAhead, steps - 1) * NT + n) * 32);
+                if (++c16 == nc16) {
+                    c16 = 0;
+                    if (++dz == 3) { dz = 0; if (++dy == 3) { dy = 0; ++dx; } }
                 }
             }
         }
@@ -397,6 +421,13 @@ __global__ void __launch_bounds__(kConvThreads) k_conv2(ConvArgs a) {
 // epilogue reads the accumulators with tcgen05.ld (warps w, w + 4, ...: TMEM lanes 32 (w mod 4)
 // .. + 31 = rows, splitting the 16-column blocks), applies ReLU and stores BF16 channels-last.
 //
+// PLANES (several x-planes, all 27 taps resident): a plane p of the halo serves tile t with dx = p - t,
+// so one MMA with the weights of up to three dx side by side (N = 48 for 16 channels) feeds the
+// accumulators of three tiles from one read of the plane; each accumulator still takes its taps in
+// their order.  Bound by the MMAs (half of the cycles) and, between them, by each CTA's own chain of
+// staging, MMAs and epilogue, which 2 to 4 CTAs per SM overlap.  16 -> 16 at 128^3: 81 us with two
+// planes and an MMA per tile and tap, 72 with four planes (floor 20: its input and output).
+//
 // Every wait is bounded; on a timeout the kernel sets bit 0 of *status, skips the epilogue
 // and still frees its tensor memory.
 // ---------------------------------------------------------------------------------
@@ -404,7 +435,9 @@ constexpr int TCY = 16, TCZ = 8, HCY = TCY + 2, HCZ = TCZ + 2;
 constexpr int kTcThreadsMax = 512;
 constexpr int kTcWaitLimit = 1 << 22;
 constexpr size_t kTcSmemBudget = 110 * 1024;   // two CTAs per SM
-constexpr int kTcSmemMax = 112 * 1024;
+constexpr size_t kTcSmemBudget1 = 225 * 1024;  // one
+constexpr int kTcSmemMax = kTcSmemBudget1;
+constexpr size_t kTcSmemSmall = 56 * 1024;     // four: 256 threads each
 
 __host__ __device__ constexpr int tc_hvp(int txc) { return ((txc + 2) * HCY * HCZ) | 1; }
 
@@ -427,7 +460,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mb, uint32_t parity) {
     return false;
 }
 
-template <int TXC, int NU, int THREADS>
+template <int TXC, int NU, int THREADS, bool PLANES>
 __global__ void __launch_bounds__(THREADS) k_conv_tc(ConvArgs a, int n_out, int tpc, unsigned* status) {
     extern __shared__ __align__(1024) unsigned char tsm[];
     __shared__ __align__(8) uint64_t bar_full[2], bar_empty[2];
@@ -477,23 +510,87 @@ __global__ void __launch_bounds__(THREADS) k_conv_tc(ConvArgs a, int n_out, int 
     // the first two chunks load while the halo is staged
     if (tid == 32) for (int c = 0; c < min(2, nchunks); ++c) issue_chunk(c);
     // halo: plain and upsampled BF16 by cp.async (zero fill outside the grid), the rest computed
-    const int total = ((TXC + 2) * HCY * HCZ) * nu;
-    for (int i = tid; i < total; i += THREADS) {
-        const int hv = i / nu, u = i - hv * nu;
-        const int hz = hv % HCZ, hy = (hv / HCZ) % HCY, hx = hv / (HCZ * HCY);
-        const int x = bx + hx - 1, y = by + hy - 1, z = bz + hz - 1;
-        const bool in = x >= 0 && y >= 0 && z >= 0 && x < a.dims[0] && y < a.dims[1] && z < a.dims[2];
-        const int c = u << 3;
-        const uint32_t off = (uint32_t)(u * hvp + hv) * 16u;
-        uint4* dptr = reinterpret_cast<uint4*>(tsm + off);
-        if (c < a.s0.C) stage_one(a.s0, x, y, z, c, in, halo + off, dptr);
-        else stage_one(a.s1, x, y, z, c - a.s0.C, in, halo + off, dptr);
+    // A thread keeps one unit and z-offset of the lines (x, y) of the halo and goes from line to line,
+    // so that its source, channel and z-bounds are formed once (at 256^3 the 48 -> 16 layer 352 -> 285
+    // us, the 16 -> 16 layers 89 -> 81, against one sequence over all units, each taken apart by
+    // divisions).
+    constexpr int kLine = HCZ * NU, kLines = (TXC + 2) * HCY, kStep = THREADS / kLine;
+    if (tid < kLine * kStep) {
+        const int l0 = tid / kLine, i = tid - l0 * kLine, hz = i / nu, u = i - hz * nu, z = bz + hz - 1;
+        int c = u << 3;
+        const bool second = c >= a.s0.C;
+        if (second) c -= a.s0.C;
+        const Src& src = second ? a.s1 : a.s0;
+        const int kind = src.kind, up = kind == SRC_BF16_UP ? 1 : 0;
+        const bool zin = z >= 0 && z < a.dims[2];
+        const uint32_t dst0 = halo + (uint32_t)(u * hvp + hz) * 16u;
+        if (kind == SRC_BF16 || kind == SRC_BF16_UP) {
+            const __nv_bfloat16* base = (const __nv_bfloat16*)src.p + src.coff + c;
+            const long long sy = (long long)src.dims[2] * src.cstride, sx = sy * src.dims[1];
+            const __nv_bfloat16* bzp = base + (zin ? (long long)(z >> up) * src.cstride : 0);
+            int hx = 0, hy = l0;
+            while (hy >= HCY) { hy -= HCY; ++hx; }
+            for (int l = l0; l < kLines; l += kStep) {
+                const int x = bx + hx - 1, y = by + hy - 1;
+                const bool in = zin && x >= 0 && y >= 0 && x < a.dims[0] && y < a.dims[1];
+                const __nv_bfloat16* gp = in ? bzp + (x >> up) * sx + (y >> up) * sy : base;
+                cp_async16(dst0 + (uint32_t)l * (HCZ * 16u), gp, in ? 16 : 0);
+                hy += kStep;
+                while (hy >= HCY) { hy -= HCY; ++hx; }
+            }
+        } else {
+            for (int l = l0; l < kLines; l += kStep) {
+                const int hx = l / HCY, x = bx + hx - 1, y = by + l - hx * HCY - 1;
+                const bool in = zin && x >= 0 && y >= 0 && x < a.dims[0] && y < a.dims[1];
+                *reinterpret_cast<uint4*>(tsm + (dst0 - halo) + (size_t)l * (HCZ * 16)) =
+                    in ? load_unit(src, x, y, z, c) : make_uint4(0, 0, 0, 0);
+            }
+        }
     }
     cp_async_wait_all();
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
 
-    if (tid == 32) {
+    if constexpr (PLANES) {
+        if (tid == 0) {
+            if (!mbar_wait((uint32_t)__cvta_generic_to_shared(&bar_full[0]), 0u)) failed = 1;
+            else {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t adesc0 = umma_sdesc(halo, (uint32_t)hvp * 16u, HCZ * 16u);
+                const uint64_t bdesc0 = umma_sdesc(wbuf0, 3u * (uint32_t)n_out * 16u, 128u);
+                // tiles [t0, t1) of plane p, each with its dx = p - t
+                auto mma = [&](int p, int t0, int t1, int dydz, int hvt, int ks, uint32_t acc) {
+                    const uint64_t ad = adesc0 + (uint64_t)(2 * ks * hvp + hvt + p * HCY * HCZ);
+                    const uint64_t bd = bdesc0 + (uint64_t)(((dydz * NU + 2 * ks) * 3 + 2 - (p - t0)) * n_out);
+                    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                                 ::"r"(tbase + (uint32_t)(t0 * n_out)), "l"(ad), "l"(bd),
+                                   "r"(umma_idesc((t1 - t0) * n_out)), "r"(acc)
+                                 : "memory");
+                };
+#pragma unroll 1
+                for (int p = 0; p < TXC + 2; ++p) {
+                    const int t0 = max(0, p - 2), t1 = min(TXC, p + 1);
+#pragma unroll 1
+                    for (int dydz = 0; dydz < 9; ++dydz) {
+                        const int hvt = (dydz / 3) * HCZ + dydz % 3;
+#pragma unroll
+                        for (int ks = 0; ks < NU / 2; ++ks) {
+                            if (ks == 0 && dydz == 0 && p < TXC) {   // tile p starts here
+                                if (t0 < p) mma(p, t0, p, dydz, hvt, ks, 1u);
+                                mma(p, p, p + 1, dydz, hvt, ks, 0u);
+                            } else {
+                                mma(p, t0, t1, dydz, hvt, ks, 1u);
+                            }
+                        }
+                    }
+                }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                             ::"r"((uint32_t)__cvta_generic_to_shared(&bar_empty[0]))
+                             : "memory");
+            }
+        }
+    } else if (tid == 32) {
         // producer: the remaining chunks, each once the MMAs of the chunk two before are done
         for (int c = 2; c < nchunks; ++c) {
             if (!mbar_wait((uint32_t)__cvta_generic_to_shared(&bar_empty[c & 1]), (uint32_t)((c >> 1) - 1) & 1u)) {
@@ -742,12 +839,14 @@ __global__ void k_pack(const float* __restrict__ W, int cin, int cout, int trans
 }
 
 // forward weights for k_conv_tc: unit (tap, u, n) = W[tap][8u .. 8u+7][n] as BF16, n < nout
-// (columns n >= cout are zero)
-__global__ void k_pack_tc(const float* __restrict__ W, int cin, int cout, int nout, uint4* __restrict__ out) {
+// (columns n >= cout are zero); planes: units in the order (dy dz, u, dx descending, n)
+__global__ void k_pack_tc(const float* __restrict__ W, int cin, int cout, int nout, int planes, uint4* __restrict__ out) {
     const int nu = cin / 8;
     const int total = 27 * nu * nout;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-        const int n = e % nout, u = (e / nout) % nu, tap = e / (nout * nu);
+        const int n = e % nout, t = e / nout;
+        const int u = planes ? (t / 3) % nu : t % nu;
+        const int tap = planes ? 9 * (2 - t % 3) + t / (3 * nu) : t / nu;
         if (n >= cout) { out[e] = make_uint4(0, 0, 0, 0); continue; }
         const float* w = W + ((size_t)tap * cin + 8 * u) * cout + n;
         out[e] = make_uint4(pack_bf16(w[0], w[(size_t)cout]), pack_bf16(w[2 * (size_t)cout], w[3 * (size_t)cout]),
@@ -855,32 +954,65 @@ __device__ __forceinline__ void pro1(int i, int nc, int& j0, float& w0, int& j1,
     j1 = max(0, min(nc - 1, j1));
 }
 
-// z = omega r / diag + (1/scale) P y   (0 on excluded cells); omega_on = 0 drops the first term
+// a x + b y, the second product rounded (written out so that both group widths round alike)
+__device__ __forceinline__ float lerp(float a, float x, float b, float y) { return fmaf(a, x, __fmul_rn(b, y)); }
+
+// z = omega r / diag + (1/scale) P y   (0 on excluded cells); omega_on = 0 drops the first term.
+// W = 4 (rows of a multiple of four cells): a group's cells share the four coarse rows and read 16
+// coarse values, not 32, with the row's weights formed once: 63 us at 256^3, 130 with one cell a thread
+// (floor 21: r, y and z).
+template <int W>
 __global__ void k_combine(PoissonGrid g, const float* __restrict__ r, const float* __restrict__ y, int c0, int c1,
                           int c2, const float* __restrict__ omega, int omega_on, const double* rr, double n_free,
                           float* __restrict__ z) {
     const float sc = rms_scale(rr, n_free);
     const float inv = sc > 0.f ? 1.f / sc : 0.f;
     const float om = omega_on ? *omega : 0.f;
-    const unsigned n = (unsigned)g.nx * g.ny * g.nz;
-    for (unsigned c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-        if (excl(g, c)) { z[c] = 0.f; continue; }
-        const unsigned t = c / (unsigned)g.nz;
+    const unsigned n = (unsigned)g.nx * g.ny * g.nz / W;
+    for (unsigned gi = blockIdx.x * blockDim.x + threadIdx.x; gi < n; gi += gridDim.x * blockDim.x) {
+        const unsigned c = gi * W, t = c / (unsigned)g.nz;
         const int iz = (int)(c - t * (unsigned)g.nz), iy = (int)(t % (unsigned)g.ny), ix = (int)(t / (unsigned)g.ny);
-        int xa, xb, ya, yb, za, zb;
-        float wxa, wxb, wya, wyb, wza, wzb;
+        float rv[W], zv[W];
+        if constexpr (W == 4) {
+            const float4 v = *reinterpret_cast<const float4*>(r + c);
+            rv[0] = v.x; rv[1] = v.y; rv[2] = v.z; rv[3] = v.w;
+        } else {
+            rv[0] = r[c];
+        }
+        int xa, xb, ya, yb;
+        float wxa, wxb, wya, wyb;
         pro1(ix, c0, xa, wxa, xb, wxb);
         pro1(iy, c1, ya, wya, yb, wyb);
-        pro1(iz, c2, za, wza, zb, wzb);
-        auto Y = [&](int x, int yy, int zz) { return y[((unsigned)x * c1 + yy) * c2 + zz]; };
-        const float p = wxa * (wya * (wza * Y(xa, ya, za) + wzb * Y(xa, ya, zb)) + wyb * (wza * Y(xa, yb, za) + wzb * Y(xa, yb, zb))) +
-                        wxb * (wya * (wza * Y(xb, ya, za) + wzb * Y(xb, ya, zb)) + wyb * (wza * Y(xb, yb, za) + wzb * Y(xb, yb, zb)));
-        const int d = bdiag(g, ix, iy, iz);
-        const float jac = d > 0 ? r[c] / (float)d : 0.f;
-        z[c] = om * jac + inv * p;
+        const float* row[4] = {y + ((unsigned)xa * c1 + ya) * c2, y + ((unsigned)xa * c1 + yb) * c2,
+                               y + ((unsigned)xb * c1 + ya) * c2, y + ((unsigned)xb * c1 + yb) * c2};
+        // the group's coarse columns: W = 4 (iz a multiple of 4) iz/2 - 1 .. iz/2 + 2, clamped
+        constexpr int NC = W == 4 ? 4 : 2;
+        float Y[4][NC];
+        int za[W], zb[W];
+        float wza[W], wzb[W];
+#pragma unroll
+        for (int e = 0; e < W; ++e) pro1(iz + e, c2, za[e], wza[e], zb[e], wzb[e]);
+#pragma unroll
+        for (int m = 0; m < NC; ++m) {
+            const int col = W == 4 ? (m < 2 ? (m == 0 ? za[0] : zb[0]) : (m == 2 ? zb[W == 4 ? 2 : 0] : zb[W - 1]))
+                                   : (m == 0 ? za[0] : zb[0]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) Y[q][m] = row[q][col];
+        }
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+            constexpr int kFirst[4] = {0, 1, 1, 2};   // za, zb of cell e are columns kFirst[e], kFirst[e] + 1
+            const int a = W == 4 ? kFirst[e] : 0, b = a + 1;
+            const float p = lerp(wxa, lerp(wya, lerp(wza[e], Y[0][a], wzb[e], Y[0][b]), wyb, lerp(wza[e], Y[1][a], wzb[e], Y[1][b])),
+                                 wxb, lerp(wya, lerp(wza[e], Y[2][a], wzb[e], Y[2][b]), wyb, lerp(wza[e], Y[3][a], wzb[e], Y[3][b])));
+            const int d = bdiag(g, ix, iy, iz + e);
+            const float jac = d > 0 ? rv[e] / (float)d : 0.f;
+            zv[e] = excl(g, c + e) ? 0.f : lerp(inv, p, om, jac);
+        }
+        if constexpr (W == 4) *reinterpret_cast<float4*>(z + c) = make_float4(zv[0], zv[1], zv[2], zv[3]);
+        else z[c] = zv[0];
     }
 }
-
 // weight of coarse cell m in the prolongation to fine cell i along one axis: 3/4 for the two
 // children (2m, 2m+1), 1/4 for the next fine cells out (2m-1, 2m+2); at the ends of the axis
 // the clamped neighbour adds its 1/4 to the end cell (fine 0 -> coarse 0, fine 2nc-1 ->
@@ -1059,6 +1191,13 @@ constexpr int kRedBlocks = 304;
 // a training pair with the Poisson problem it belongs to (solid mask copy, pinned cell)
 struct Pair { float* r; float* p; unsigned char* solid; int pin; double denom; };
 
+struct TcConfig {
+    int txc, tpc;   // x-planes of a CTA (0: not k_conv_tc), taps of a weight chunk
+    size_t smem;
+    bool planes;    // plane by plane, the weights packed for it
+};
+constexpr bool tc_planes(int txc, int nu, int tpc) { return txc > 1 && nu <= 6 && tpc == 27; }
+
 struct Net {
     int fine[3];
     int dims[4][3];
@@ -1070,7 +1209,9 @@ struct Net {
     unsigned* tc_status;  // bit 0: a k_conv_tc wait ran out
     bool use_tc;
     size_t tc_budget;     // shared memory per k_conv_tc CTA
+    TcConfig tc[kLayers]; // how k_conv_tc runs a layer
     void* act[kTensors];
+    void* pool[kLayers];   // pooled inputs (IN_POOL layers)
     float* grad[kTensors];
     float* temp;       // backward data output of concat / pool inputs
     float* z;          // fine-grid preconditioner output (training)
@@ -1088,6 +1229,15 @@ namespace {
 #define UCK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return e_; } while (0)
 
 int grid_for(long long n) { return (int)std::max(1LL, std::min<long long>(4 * 152, (n + 255) / 256)); }
+
+void combine(const PoissonGrid& g, const float* r, const float* y, const int* dims, const float* omega, int omega_on,
+             const double* rr, double n_free, float* z, cudaStream_t s) {
+    const long long nf = (long long)g.nx * g.ny * g.nz;
+    if (g.nz % 4 == 0)
+        k_combine<4><<<grid_for(nf / 4), 256, 0, s>>>(g, r, y, dims[0], dims[1], dims[2], omega, omega_on, rr, n_free, z);
+    else
+        k_combine<1><<<grid_for(nf), 256, 0, s>>>(g, r, y, dims[0], dims[1], dims[2], omega, omega_on, rr, n_free, z);
+}
 
 void* dalloc(Net* n, size_t bytes) {
     void* p = nullptr;
@@ -1133,37 +1283,50 @@ cudaError_t launch_conv2_t(ConvArgs a, int nsplit, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <int TXC, int NU, int THREADS>
+template <int TXC, int NU, int THREADS, bool PLANES>
 cudaError_t launch_conv_tc_k(const ConvArgs& a, int n_out, int tpc, size_t smem, unsigned* status, cudaStream_t s) {
     static bool attr = false;
     if (!attr) {
-        UCK(cudaFuncSetAttribute(k_conv_tc<TXC, NU, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemMax));
+        UCK(cudaFuncSetAttribute(k_conv_tc<TXC, NU, THREADS, PLANES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kTcSmemMax));
         attr = true;
     }
     const dim3 grid((a.dims[2] + TCZ - 1) / TCZ, (a.dims[1] + TCY - 1) / TCY, (a.dims[0] + TXC - 1) / TXC);
-    k_conv_tc<TXC, NU, THREADS><<<grid, THREADS, smem, s>>>(a, n_out, tpc, status);
+    k_conv_tc<TXC, NU, THREADS, PLANES><<<grid, THREADS, smem, s>>>(a, n_out, tpc, status);
     return cudaGetLastError();
 }
 
-// 256 threads where the CTA is small enough for many CTAs per SM, else 512 (measured at
-// 256^3: the 16 -> 16 layers 92 us with 256 threads, 130 with 512; the 48 -> 16 layer 379 us
-// with 256, 352 with 512)
+// 256 threads where the CTA is small enough for four CTAs per SM, else 512 (a projection at 256^3:
+// 104 ms; 108 with 512 threads for the four-plane CTAs too).  Several planes with all taps at once
+// go plane by plane.
 template <int TXC, int NU>
 cudaError_t launch_conv_tc_t(const ConvArgs& a, int n_out, int tpc, size_t smem, unsigned* status, cudaStream_t s) {
-    if (smem <= 40 * 1024) return launch_conv_tc_k<TXC, NU, 256>(a, n_out, tpc, smem, status, s);
-    return launch_conv_tc_k<TXC, NU, kTcThreadsMax>(a, n_out, tpc, smem, status, s);
+    constexpr bool kPlanes = tc_planes(TXC, NU, 27);
+    if (kPlanes && tpc == 27) {
+        if (smem <= kTcSmemSmall) return launch_conv_tc_k<TXC, NU, 256, kPlanes>(a, n_out, tpc, smem, status, s);
+        return launch_conv_tc_k<TXC, NU, kTcThreadsMax, kPlanes>(a, n_out, tpc, smem, status, s);
+    }
+    if constexpr (TXC > 2) return cudaErrorInvalidValue;
+    else {
+        if (smem <= kTcSmemSmall) return launch_conv_tc_k<TXC, NU, 256, false>(a, n_out, tpc, smem, status, s);
+        return launch_conv_tc_k<TXC, NU, kTcThreadsMax, false>(a, n_out, tpc, smem, status, s);
+    }
 }
 
 template <int TXC>
 cudaError_t launch_conv_tc_nu(const ConvArgs& a, int n_out, int tpc, size_t smem, unsigned* status, cudaStream_t s) {
-    switch (a.cin / 8) {
-        case 2: return launch_conv_tc_t<TXC, 2>(a, n_out, tpc, smem, status, s);
-        case 4: return launch_conv_tc_t<TXC, 4>(a, n_out, tpc, smem, status, s);
-        case 6: return launch_conv_tc_t<TXC, 6>(a, n_out, tpc, smem, status, s);
-        case 8: return launch_conv_tc_t<TXC, 8>(a, n_out, tpc, smem, status, s);
-        case 10: return launch_conv_tc_t<TXC, 10>(a, n_out, tpc, smem, status, s);
-        case 14: return launch_conv_tc_t<TXC, 14>(a, n_out, tpc, smem, status, s);
-        default: return cudaErrorInvalidValue;
+    if constexpr (TXC == 4) {
+        return a.cin == 16 ? launch_conv_tc_t<4, 2>(a, n_out, tpc, smem, status, s) : cudaErrorInvalidValue;
+    } else {
+        switch (a.cin / 8) {
+            case 2: return launch_conv_tc_t<TXC, 2>(a, n_out, tpc, smem, status, s);
+            case 4: return launch_conv_tc_t<TXC, 4>(a, n_out, tpc, smem, status, s);
+            case 6: return launch_conv_tc_t<TXC, 6>(a, n_out, tpc, smem, status, s);
+            case 8: return launch_conv_tc_t<TXC, 8>(a, n_out, tpc, smem, status, s);
+            case 10: return launch_conv_tc_t<TXC, 10>(a, n_out, tpc, smem, status, s);
+            case 14: return launch_conv_tc_t<TXC, 14>(a, n_out, tpc, smem, status, s);
+            default: return cudaErrorInvalidValue;
+        }
     }
 }
 
@@ -1177,28 +1340,41 @@ size_t conv_tc_smem(int txc, int cin, int n_out, int tpc) {
 // multiple of 16 up to 64, or the single FP32 output channel of the last layer, computed as 16
 // with zero weights) and its tiles make at least one wave.  Configurations, best first: all
 // 27 taps in one or two weight chunks (no refill wait, both loads overlap the halo staging),
-// two x-planes per CTA before one; then 9-, 3- and 1-tap chunks; each within 110 KB of shared
-// memory (two CTAs per SM).  Returns false (nothing launched) otherwise.
+// two x-planes per CTA before one; then 9- and 3-tap chunks; each within 110 KB of shared
+// memory (two CTAs per SM).  Where only single taps would fit, one CTA per SM with up to 225 KB: each
+// refill of a one-tap buffer is waited for (80 -> 32 at 64^3: 120 us, 102 so), and 112 input channels
+// did not fit at all (112 -> 48 at 32^3 by mma.sync: 131 us, 31 so).  Four planes for 16 input channels,
+// whose halo leaves room for four CTAs, where they make four waves.
+// txc = 0: the layer does not qualify.
 int tc_nout(int cout) { return cout == 1 ? 16 : cout; }
 
-bool try_conv_tc(const ConvArgs& a, int cout, size_t budget, unsigned* status, cudaStream_t s, cudaError_t* err) {
-    if (!a.wtc || a.cin % 16 || cout != a.cout_real) return false;
-    const bool f32_single = a.out_kind == OUT_F32 && cout == 1;
-    if (!f32_single && (a.out_kind != OUT_BF16 || cout % 16 || cout > 64)) return false;
+TcConfig tc_config(const int* dims, int cin, int cout, size_t budget) {
+    TcConfig c{};
+    if (cin % 16 || !(cout == 1 || (cout % 16 == 0 && cout <= 64))) return c;
     const int n_out = tc_nout(cout);
-    const long long tiles1 = (long long)((a.dims[2] + TCZ - 1) / TCZ) * ((a.dims[1] + TCY - 1) / TCY) * a.dims[0];
-    if (tiles1 < 152) return false;
-    static const int order[][2] = {{2, 27}, {2, 14}, {1, 27}, {1, 14}, {2, 9}, {1, 9}, {2, 3}, {1, 3}, {2, 1}, {1, 1}};
+    const long long tiles1 = (long long)((dims[2] + TCZ - 1) / TCZ) * ((dims[1] + TCY - 1) / TCY) * dims[0];
+    if (tiles1 < 152) return c;
+    static const int order[][2] = {{4, 27}, {2, 27}, {2, 14}, {1, 27}, {1, 14}, {2, 9}, {1, 9}, {2, 3}, {1, 3}, {0, 0},
+                                   {2, 27}, {2, 14}, {2, 9}, {1, 27}, {1, 14}, {1, 9}, {2, 3}, {1, 3}, {0, 0},
+                                   {2, 1}, {1, 1}};
+    bool one = false;
     for (const auto& o : order) {
         const int txc = o[0], tpc = o[1];
+        if (txc == 0) { one = !one && budget == kTcSmemBudget; continue; }
+        if (txc == 4 && (cin != 16 || tiles1 / 4 < 4 * 152)) continue;
         if (txc == 2 && tiles1 / 2 < 2 * 152) continue;
-        const size_t sm = conv_tc_smem(txc, a.cin, n_out, tpc);
-        if (sm > budget) continue;
-        *err = txc == 2 ? launch_conv_tc_nu<2>(a, n_out, tpc, sm, status, s)
-                        : launch_conv_tc_nu<1>(a, n_out, tpc, sm, status, s);
-        return true;
+        const size_t sm = conv_tc_smem(txc, cin, n_out, tpc);
+        if (sm > (one ? kTcSmemBudget1 : budget)) continue;
+        c.txc = txc; c.tpc = tpc; c.smem = sm; c.planes = tc_planes(txc, cin / 8, tpc);
+        break;
     }
-    return false;
+    return c;
+}
+cudaError_t launch_conv_tc(const ConvArgs& a, const TcConfig& c, int cout, unsigned* status, cudaStream_t s) {
+    const int n = tc_nout(cout);
+    return c.txc == 4   ? launch_conv_tc_nu<4>(a, n, c.tpc, c.smem, status, s)
+           : c.txc == 2 ? launch_conv_tc_nu<2>(a, n, c.tpc, c.smem, status, s)
+                        : launch_conv_tc_nu<1>(a, n, c.tpc, c.smem, status, s);
 }
 
 // Chooses the brick (MT) and the n-tile split for a convolution with cout_padded output
@@ -1271,7 +1447,7 @@ void layer_sources(const Net* n, int l, ConvArgs& a) {
     switch (d.mode) {
         case IN_SCALAR: a.s0 = make_src(SRC_F32, n->act[d.in0], 1, 1, 0, n->dims[lev]); break;
         case IN_PLAIN: a.s0 = make_src(SRC_BF16, n->act[d.in0], d.shape.cin, d.shape.cin, 0, n->dims[lev]); break;
-        case IN_POOL: a.s0 = make_src(SRC_BF16_POOL, n->act[d.in0], d.shape.cin, d.shape.cin, 0, n->dims[lev - 1]); break;
+        case IN_POOL: a.s0 = make_src(SRC_BF16, n->pool[l], d.shape.cin, d.shape.cin, 0, n->dims[lev]); break;
         case IN_UPCAT: {
             const int cu = kTensorC[d.in0], cs = kTensorC[d.in1];
             a.s0 = make_src(SRC_BF16_UP, n->act[d.in0], cu, cu, 0, n->dims[lev + 1]);
@@ -1288,14 +1464,19 @@ cudaError_t forward(Net* n, cudaStream_t s) {
         const LayerDef& d = kDefs[l];
         ConvArgs a;
         layer_sources(n, l, a);
+        if (d.mode == IN_POOL) {
+            const Src src = make_src(SRC_BF16_POOL, n->act[d.in0], d.shape.cin, d.shape.cin, 0, n->dims[d.shape.level - 1]);
+            const int* pd = n->dims[d.shape.level];
+            k_pool<<<grid_for(nvox(pd) * (d.shape.cin / 8)), 256, 0, s>>>(src, pd[0], pd[1], pd[2], (uint4*)n->pool[l]);
+            ++n->launches;
+        }
         a.wfrag = n->wf[l];
         a.relu = d.shape.relu;
         a.cout_real = d.shape.cout;
         if (d.out == T_Y) { a.out_kind = OUT_F32; a.out = n->act[T_Y]; a.out_cstride = 1; a.out_coff = 0; }
         else { a.out_kind = OUT_BF16; a.out = n->act[d.out]; a.out_cstride = d.shape.cout; a.out_coff = 0; }
         a.wtc = n->use_tc ? n->wt[l] : nullptr;
-        cudaError_t e = cudaSuccess;
-        if (try_conv_tc(a, d.shape.cout, n->tc_budget, n->tc_status, s, &e)) UCK(e);
+        if (a.wtc && n->tc[l].txc) UCK(launch_conv_tc(a, n->tc[l], d.shape.cout, n->tc_status, s));
         else UCK(launch_conv(a, std::max(8, d.shape.cout), s));
         ++n->launches;
     }
@@ -1368,7 +1549,8 @@ cudaError_t pack_all(Net* n, cudaStream_t s) {
             k_pack<<<grid_for((long long)frag_count(sh.cin, sh.cout, true)), 256, 0, s>>>(W, sh.cin, sh.cout, 1, n->wb[l]);
         if (n->wt[l])
             k_pack_tc<<<grid_for(27LL * (sh.cin / 8) * tc_nout(sh.cout)), 256, 0, s>>>(W, sh.cin, sh.cout,
-                                                                                    tc_nout(sh.cout), n->wt[l]);
+                                                                                    tc_nout(sh.cout),
+                                                                                    n->tc[l].planes ? 1 : 0, n->wt[l]);
     }
     return cudaGetLastError();
 }
@@ -1402,7 +1584,11 @@ Net* net_create(int nx, int ny, int nz, cudaStream_t s) {
     n->tc_budget = kTcSmemBudget;
     if (const char* e = std::getenv("FIA_TC_SMEM_KB")) {
         const long kb = std::strtol(e, nullptr, 10);
-        if (kb >= 16 && kb * 1024 <= kTcSmemMax) n->tc_budget = (size_t)kb * 1024;
+        if (kb >= 16 && kb <= 112) n->tc_budget = (size_t)kb * 1024;
+    }
+    for (int l = 0; l < kLayers; ++l) {
+        const LayerShape& sh = kDefs[l].shape;
+        n->tc[l] = n->wt[l] ? tc_config(n->dims[sh.level], sh.cin, sh.cout, n->tc_budget) : TcConfig{};
     }
     size_t tmax = 0;
     for (int t = 0; t < kTensors; ++t) {
@@ -1413,6 +1599,7 @@ Net* net_create(int nx, int ny, int nz, cudaStream_t s) {
     }
     for (int l = 0; l < kLayers; ++l) {
         const LayerDef& d = kDefs[l];
+        n->pool[l] = d.mode == IN_POOL ? A((size_t)nvox(n->dims[d.shape.level]) * d.shape.cin * 2 + 64) : nullptr;
         if (d.mode == IN_POOL || d.mode == IN_UPCAT)
             tmax = std::max(tmax, (size_t)nvox(n->dims[d.shape.level]) * d.shape.cin);
     }
@@ -1448,11 +1635,9 @@ cudaError_t net_get_weights(Net* n, float* host, long long count) {
 
 cudaError_t net_grid_op(Net* n, const PoissonGrid& g, int op, const float* in, float* out, cudaStream_t s) {
     const int* d0 = n->dims[0];
-    const long long nf = (long long)g.nx * g.ny * g.nz;
     if (op == 0) k_restrict<<<grid_for(nvox(d0)), 256, 0, s>>>(g, in, out, d0[0], d0[1], d0[2], nullptr, 0.0);
     else if (op == 1)
-        k_combine<<<grid_for(nf), 256, 0, s>>>(g, in, in, d0[0], d0[1], d0[2], n->w + num_parameters() - 1, 0,
-                                               nullptr, 0.0, out);
+        combine(g, in, in, d0, n->w + num_parameters() - 1, 0, nullptr, 0.0, out, s);
     else if (op == 2) k_prolong_adj<<<grid_for(nvox(d0)), 256, 0, s>>>(g, in, d0[0], d0[1], d0[2], out);
     else return cudaErrorInvalidValue;
     UCK(cudaGetLastError());
@@ -1513,9 +1698,7 @@ cudaError_t net_apply(Net* n, const PoissonGrid& g, const float* r, float* z, co
     n->launches = 0;
     k_restrict<<<grid_for(nvox(d0)), 256, 0, s>>>(g, r, (float*)n->act[T_X0], d0[0], d0[1], d0[2], rr, n_free);
     UCK(forward(n, s));
-    k_combine<<<grid_for((long long)g.nx * g.ny * g.nz), 256, 0, s>>>(g, r, (const float*)n->act[T_Y], d0[0], d0[1],
-                                                                      d0[2], n->w + num_parameters() - 1, 1, rr,
-                                                                      n_free, z);
+    combine(g, r, (const float*)n->act[T_Y], d0, n->w + num_parameters() - 1, 1, rr, n_free, z, s);
     n->launches += 2;
     return cudaGetLastError();
 }
@@ -1566,12 +1749,10 @@ cudaError_t net_loss(Net* n, const PoissonGrid& g0, int pair, bool backward_pass
     const Pair& pr = n->pairs[pair];
     const PoissonGrid g{g0.nx, g0.ny, g0.nz, pr.pin, pr.solid};
     const int* d0 = n->dims[0];
-    const long long nf = (long long)g.nx * g.ny * g.nz;
     const float* omega = n->w + num_parameters() - 1;
     k_restrict<<<grid_for(nvox(d0)), 256, 0, s>>>(g, pr.r, (float*)n->act[T_X0], d0[0], d0[1], d0[2], nullptr, 0.0);
     UCK(forward(n, s));
-    k_combine<<<grid_for(nf), 256, 0, s>>>(g, pr.r, (const float*)n->act[T_Y], d0[0], d0[1], d0[2], omega, 1, nullptr,
-                                           0.0, n->z);
+    combine(g, pr.r, (const float*)n->act[T_Y], d0, omega, 1, nullptr, 0.0, n->z, s);
     k_loss<<<kRedBlocks, 256, 0, s>>>(g, n->z, pr.p, pr.r, omega, 1.0 / pr.denom, backward_pass ? 1 : 0, 0, n->gz,
                                       n->part);
     k_sum_parts<<<1, 256, 0, s>>>(n->part, kRedBlocks, 2, n->sums);
@@ -1598,12 +1779,10 @@ cudaError_t net_calibrate(Net* n, const PoissonGrid& g0, int pair, cudaStream_t 
     const Pair& pr = n->pairs[pair];
     const PoissonGrid g{g0.nx, g0.ny, g0.nz, pr.pin, pr.solid};
     const int* d0 = n->dims[0];
-    const long long nf = (long long)g.nx * g.ny * g.nz;
     const float* omega = n->w + num_parameters() - 1;
     k_restrict<<<grid_for(nvox(d0)), 256, 0, s>>>(g, pr.r, (float*)n->act[T_X0], d0[0], d0[1], d0[2], nullptr, 0.0);
     UCK(forward(n, s));
-    k_combine<<<grid_for(nf), 256, 0, s>>>(g, pr.r, (const float*)n->act[T_Y], d0[0], d0[1], d0[2], omega, 0, nullptr,
-                                           0.0, n->z);
+    combine(g, pr.r, (const float*)n->act[T_Y], d0, omega, 0, nullptr, 0.0, n->z, s);
     k_loss<<<kRedBlocks, 256, 0, s>>>(g, n->z, pr.p, pr.r, omega, 1.0, 0, 1, nullptr, n->part);
     k_sum_parts<<<1, 256, 0, s>>>(n->part, kRedBlocks, 2, n->sums);
     k_ratio<<<1, 1, 0, s>>>(n->sums, n->sums + 4);
