@@ -68,7 +68,7 @@ constexpr int HX = TX + 2, HY = TY + 2, HZ = TZ + 2;
 constexpr int HV = HX * HY * HZ;                // 432 halo voxels
 constexpr int kConvThreads = 128;               // 4 warps x 2 lines of 16 voxels
 
-enum SrcKind : int { SRC_BF16 = 1, SRC_BF16_UP = 2, SRC_BF16_POOL = 3, SRC_F32 = 4, SRC_F32_GATED = 5 };
+enum SrcKind : int { SRC_BF16 = 1, SRC_BF16_UP = 2, SRC_F32 = 4, SRC_F32_GATED = 5 };
 
 struct Src {
     int kind;
@@ -106,53 +106,28 @@ __device__ __forceinline__ long long vox(const int* d, int x, int y, int z) {
     return ((long long)x * d[1] + y) * d[2] + z;
 }
 
-// 8 channels [c, c+8) of source s at voxel (x,y,z) of the convolution's grid, as bf16x8
-__device__ uint4 load_unit(const Src& s, int x, int y, int z, int c) {
+// 8 channels [c, c+8) of the 2 x 2 x 2 average of s at coarse voxel (x,y,z), as bf16x8
+__device__ __forceinline__ uint4 pool_unit(const Src& s, int x, int y, int z, int c) {
     float f[8];
-    switch (s.kind) {
-        case SRC_BF16:
-        case SRC_BF16_UP: {
-            if (s.kind == SRC_BF16_UP) { x >>= 1; y >>= 1; z >>= 1; }
-            const __nv_bfloat16* p = (const __nv_bfloat16*)s.p + vox(s.dims, x, y, z) * s.cstride + s.coff + c;
-            return *reinterpret_cast<const uint4*>(p);
-        }
-        case SRC_BF16_POOL: {
-            for (int i = 0; i < 8; ++i) f[i] = 0.f;
-            int cnt = 0;
-            for (int i = 0; i < 2; ++i)
-                for (int j = 0; j < 2; ++j)
-                    for (int k = 0; k < 2; ++k) {
-                        const int cx = 2 * x + i, cy = 2 * y + j, cz = 2 * z + k;
-                        if (cx >= s.dims[0] || cy >= s.dims[1] || cz >= s.dims[2]) continue;
-                        const uint4 u = *reinterpret_cast<const uint4*>(
-                            (const __nv_bfloat16*)s.p + vox(s.dims, cx, cy, cz) * s.cstride + s.coff + c);
-                        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-                        for (int q = 0; q < 4; ++q) {
-                            const float2 t = __bfloat1622float2(h[q]);
-                            f[2 * q] += t.x; f[2 * q + 1] += t.y;
-                        }
-                        ++cnt;
-                    }
-            const float inv = 1.f / (float)cnt;
-            for (int i = 0; i < 8; ++i) f[i] *= inv;
-            break;
-        }
-        default: {   // SRC_F32, SRC_F32_GATED
-            const long long v = vox(s.dims, x, y, z);
-            const float4* p = reinterpret_cast<const float4*>((const float*)s.p + v * s.cstride + s.coff + c);
-            const float4 a = p[0], b = p[1];
-            f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-            if (s.kind == SRC_F32_GATED) {
-                const uint4 u = *reinterpret_cast<const uint4*>(s.gate + v * s.gstride + s.goff + c);
-                const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&u);
-                for (int i = 0; i < 8; ++i)
-                    if (!(__bfloat162float(h[i]) > 0.f)) f[i] = 0.f;
+    for (int i = 0; i < 8; ++i) f[i] = 0.f;
+    int cnt = 0;
+    for (int i = 0; i < 2; ++i)
+        for (int j = 0; j < 2; ++j)
+            for (int k = 0; k < 2; ++k) {
+                const int cx = 2 * x + i, cy = 2 * y + j, cz = 2 * z + k;
+                if (cx >= s.dims[0] || cy >= s.dims[1] || cz >= s.dims[2]) continue;
+                const uint4 u = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)s.p + vox(s.dims, cx, cy, cz) * s.cstride +
+                                                                s.coff + c);
+                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+                for (int q = 0; q < 4; ++q) {
+                    const float2 t = __bfloat1622float2(h[q]);
+                    f[2 * q] += t.x; f[2 * q + 1] += t.y;
+                }
+                ++cnt;
             }
-        }
-    }
-    uint4 r;
-    r.x = pack_bf16(f[0], f[1]); r.y = pack_bf16(f[2], f[3]); r.z = pack_bf16(f[4], f[5]); r.w = pack_bf16(f[6], f[7]);
-    return r;
+    const float inv = 1.f / (float)cnt;
+    for (int i = 0; i < 8; ++i) f[i] *= inv;
+    return make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
 }
 
 // one scalar (channel 0) of an fp32 source at (x,y,z)
@@ -168,24 +143,7 @@ __global__ void k_pool(Src src, int d0, int d1, int d2, uint4* __restrict__ out)
     const unsigned n = (unsigned)d0 * d1 * d2 * nu;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const unsigned v = i / nu, t = v / (unsigned)d2;
-        out[i] = load_unit(src, (int)(t / (unsigned)d1), (int)(t % (unsigned)d1), (int)(v - t * (unsigned)d2), (int)(i - v * nu) * 8);
-    }
-}
-
-// Stages the halo brick of the convolution input (channels-last, swizzled 16-byte units).
-__device__ void stage_units(const ConvArgs& a, uint4* sm, int bx, int by, int bz) {
-    const int ncu = a.cin >> 3;
-    const int total = HV * ncu;
-    for (int u = threadIdx.x; u < total; u += blockDim.x) {
-        const int hv = u / ncu, cu = u - hv * ncu;
-        const int hz = hv % HZ, hy = (hv / HZ) % HY, hx = hv / (HZ * HY);
-        const int x = bx + hx - 1, y = by + hy - 1, z = bz + hz - 1;
-        uint4 val = make_uint4(0, 0, 0, 0);
-        if (x >= 0 && y >= 0 && z >= 0 && x < a.dims[0] && y < a.dims[1] && z < a.dims[2]) {
-            const int c = cu << 3;
-            val = c < a.s0.C ? load_unit(a.s0, x, y, z, c) : load_unit(a.s1, x, y, z, c - a.s0.C);
-        }
-        sm[swz(u)] = val;
+        out[i] = pool_unit(src, (int)(t / (unsigned)d1), (int)(t % (unsigned)d1), (int)(v - t * (unsigned)d2), (int)(i - v * nu) * 8);
     }
 }
 
@@ -234,23 +192,17 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 __host__ __device__ __forceinline__ int odd_units(int cin) { return (cin >> 3) | 1; }
 
-__device__ __forceinline__ void stage_one(const Src& src, int x, int y, int z, int c, bool in, uint32_t dst,
-                                          uint4* dptr) {
-    if (src.kind == SRC_BF16 || src.kind == SRC_BF16_UP) {
-        int sx = x, sy = y, sz = z;
-        if (src.kind == SRC_BF16_UP) { sx >>= 1; sy >>= 1; sz >>= 1; }
-        const __nv_bfloat16* gp = (const __nv_bfloat16*)src.p;
-        if (in) gp += vox(src.dims, sx, sy, sz) * src.cstride + src.coff + c;
-        cp_async16(dst, gp, in ? 16 : 0);
-    } else {
-        *dptr = in ? load_unit(src, x, y, z, c) : make_uint4(0, 0, 0, 0);
-    }
+// one unit of a plain or upsampled BF16 source
+__device__ __forceinline__ void stage_bf16(const Src& src, int x, int y, int z, int c, bool in, uint32_t dst) {
+    if (src.kind == SRC_BF16_UP) { x >>= 1; y >>= 1; z >>= 1; }
+    const __nv_bfloat16* gp = (const __nv_bfloat16*)src.p;
+    if (in) gp += vox(src.dims, x, y, z) * src.cstride + src.coff + c;
+    cp_async16(dst, gp, in ? 16 : 0);
 }
 
-template <int MT>
-__device__ void stage2(const ConvArgs& a, uint4* sm, int bx, int by, int bz) {
-    constexpr int HY = 6, HZ = 18, HV = (MT + 2) * HY * HZ;
-    const int ncu = a.cin >> 3, ncp = odd_units(a.cin);
+// Stages the halo brick of a layer's input for k_wgrad (channels-last, swizzled 16-byte units).
+__device__ void stage_units(const ConvArgs& a, uint4* sm, int bx, int by, int bz) {
+    const int ncu = a.cin >> 3;
     const int total = HV * ncu;
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
     for (int u = threadIdx.x; u < total; u += blockDim.x) {
@@ -258,9 +210,80 @@ __device__ void stage2(const ConvArgs& a, uint4* sm, int bx, int by, int bz) {
         const int hz = hv % HZ, hy = (hv / HZ) % HY, hx = hv / (HZ * HY);
         const int x = bx + hx - 1, y = by + hy - 1, z = bz + hz - 1;
         const bool in = x >= 0 && y >= 0 && z >= 0 && x < a.dims[0] && y < a.dims[1] && z < a.dims[2];
-        const int c = cu << 3, su = hv * ncp + cu;
-        if (c < a.s0.C) stage_one(a.s0, x, y, z, c, in, sbase + su * 16, sm + su);
-        else stage_one(a.s1, x, y, z, c - a.s0.C, in, sbase + su * 16, sm + su);
+        const int c = cu << 3;
+        const Src& src = c < a.s0.C ? a.s0 : a.s1;
+        stage_bf16(src, x, y, z, c < a.s0.C ? c : c - a.s0.C, in, sbase + swz(u) * 16);
+    }
+}
+
+// 8 channels of an FP32 source, gated or not: the loads, and their conversion
+struct F32Unit {
+    float4 a, b;
+    uint4 gate;
+};
+__device__ __forceinline__ F32Unit load_f32(const Src& s, long long v, int c, bool in) {
+    F32Unit u{make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f), make_uint4(0, 0, 0, 0)};
+    if (in) {
+        const float4* p = reinterpret_cast<const float4*>((const float*)s.p + v * s.cstride + s.coff + c);
+        u.a = __ldg(p); u.b = __ldg(p + 1);
+        if (s.kind == SRC_F32_GATED) u.gate = __ldg(reinterpret_cast<const uint4*>(s.gate + v * s.gstride + s.goff + c));
+    }
+    return u;
+}
+__device__ __forceinline__ uint4 pack_f32(const Src& s, const F32Unit& u) {
+    float f[8] = {u.a.x, u.a.y, u.a.z, u.a.w, u.b.x, u.b.y, u.b.z, u.b.w};
+    if (s.kind == SRC_F32_GATED) {
+        const uint32_t w[4] = {u.gate.x, u.gate.y, u.gate.z, u.gate.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (!(__uint_as_float(i & 1 ? w[i >> 1] & 0xffff0000u : w[i >> 1] << 16) > 0.f)) f[i] = 0.f;
+    }
+    return make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+}
+
+// The halo brick of the backward convolutions comes from FP32 gradients: four units' loads are in
+// flight before the first is converted (one at a time, each waited for L2).
+template <int MT>
+__device__ void stage2(const ConvArgs& a, uint4* sm, int bx, int by, int bz) {
+    constexpr int HY = 6, HZ = 18, HV = (MT + 2) * HY * HZ;
+    const int ncu = a.cin >> 3, ncp = odd_units(a.cin);
+    const int total = HV * ncu;
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(sm);
+    auto place = [&](int u, int& x, int& y, int& z, int& c) {
+        const int hv = u / ncu, cu = u - hv * ncu;
+        const int hz = hv % HZ, hy = (hv / HZ) % HY, hx = hv / (HZ * HY);
+        x = bx + hx - 1; y = by + hy - 1; z = bz + hz - 1;
+        c = cu << 3;
+        return hv * ncp + cu;
+    };
+    auto inside = [&](int x, int y, int z) {
+        return x >= 0 && y >= 0 && z >= 0 && x < a.dims[0] && y < a.dims[1] && z < a.dims[2];
+    };
+    if (a.s0.kind == SRC_F32 || a.s0.kind == SRC_F32_GATED) {
+        constexpr int kBatch = 4;
+        for (int u0 = threadIdx.x; u0 < total; u0 += kBatch * blockDim.x) {
+            F32Unit v[kBatch];
+            int su[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int u = u0 + i * blockDim.x;
+                int x, y, z, c;
+                su[i] = place(u, x, y, z, c);
+                const bool in = u < total && inside(x, y, z);
+                v[i] = load_f32(a.s0, in ? vox(a.s0.dims, x, y, z) : 0, c, in);
+                if (u >= total) su[i] = -1;
+            }
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i)
+                if (su[i] >= 0) sm[su[i]] = pack_f32(a.s0, v[i]);
+        }
+        return;
+    }
+    for (int u = threadIdx.x; u < total; u += blockDim.x) {
+        int x, y, z, c;
+        const int su = place(u, x, y, z, c);
+        const Src& src = c < a.s0.C ? a.s0 : a.s1;
+        stage_bf16(src, x, y, z, c < a.s0.C ? c : c - a.s0.C, inside(x, y, z), sbase + su * 16);
     }
 }
 
@@ -521,30 +544,21 @@ __global__ void __launch_bounds__(THREADS) k_conv_tc(ConvArgs a, int n_out, int 
         const bool second = c >= a.s0.C;
         if (second) c -= a.s0.C;
         const Src& src = second ? a.s1 : a.s0;
-        const int kind = src.kind, up = kind == SRC_BF16_UP ? 1 : 0;
+        const int up = src.kind == SRC_BF16_UP ? 1 : 0;
         const bool zin = z >= 0 && z < a.dims[2];
         const uint32_t dst0 = halo + (uint32_t)(u * hvp + hz) * 16u;
-        if (kind == SRC_BF16 || kind == SRC_BF16_UP) {
-            const __nv_bfloat16* base = (const __nv_bfloat16*)src.p + src.coff + c;
-            const long long sy = (long long)src.dims[2] * src.cstride, sx = sy * src.dims[1];
-            const __nv_bfloat16* bzp = base + (zin ? (long long)(z >> up) * src.cstride : 0);
-            int hx = 0, hy = l0;
+        const __nv_bfloat16* base = (const __nv_bfloat16*)src.p + src.coff + c;
+        const long long sy = (long long)src.dims[2] * src.cstride, sx = sy * src.dims[1];
+        const __nv_bfloat16* bzp = base + (zin ? (long long)(z >> up) * src.cstride : 0);
+        int hx = 0, hy = l0;
+        while (hy >= HCY) { hy -= HCY; ++hx; }
+        for (int l = l0; l < kLines; l += kStep) {
+            const int x = bx + hx - 1, y = by + hy - 1;
+            const bool in = zin && x >= 0 && y >= 0 && x < a.dims[0] && y < a.dims[1];
+            const __nv_bfloat16* gp = in ? bzp + (x >> up) * sx + (y >> up) * sy : base;
+            cp_async16(dst0 + (uint32_t)l * (HCZ * 16u), gp, in ? 16 : 0);
+            hy += kStep;
             while (hy >= HCY) { hy -= HCY; ++hx; }
-            for (int l = l0; l < kLines; l += kStep) {
-                const int x = bx + hx - 1, y = by + hy - 1;
-                const bool in = zin && x >= 0 && y >= 0 && x < a.dims[0] && y < a.dims[1];
-                const __nv_bfloat16* gp = in ? bzp + (x >> up) * sx + (y >> up) * sy : base;
-                cp_async16(dst0 + (uint32_t)l * (HCZ * 16u), gp, in ? 16 : 0);
-                hy += kStep;
-                while (hy >= HCY) { hy -= HCY; ++hx; }
-            }
-        } else {
-            for (int l = l0; l < kLines; l += kStep) {
-                const int hx = l / HCY, x = bx + hx - 1, y = by + l - hx * HCY - 1;
-                const bool in = zin && x >= 0 && y >= 0 && x < a.dims[0] && y < a.dims[1];
-                *reinterpret_cast<uint4*>(tsm + (dst0 - halo) + (size_t)l * (HCZ * 16)) =
-                    in ? load_unit(src, x, y, z, c) : make_uint4(0, 0, 0, 0);
-            }
         }
     }
     cp_async_wait_all();
@@ -711,14 +725,25 @@ __global__ void __launch_bounds__(kConvThreads) k_wgrad(ConvArgs a, Src gs, floa
     const int xunits = ((HV * ncu + 7) / 8) * 8;
     stage_units(a, smem, bx, by, bz);
     uint4* gsm = smem + xunits;
-    for (int u = threadIdx.x; u < TX * TY * TZ * GU; u += blockDim.x) {
-        const int vrow = u / GU, cu = u - vrow * GU;
-        const int L = vrow / TZ, z = vrow % TZ;
-        const int x = bx + L / TY, y = by + L % TY, zz = bz + z;
-        uint4 val = make_uint4(0, 0, 0, 0);
-        if (x < a.dims[0] && y < a.dims[1] && zz < a.dims[2]) val = load_unit(gs, x, y, zz, cu * 8);
-        gsm[swz(u)] = val;
+    constexpr int kUnits = TX * TY * TZ * GU / kConvThreads;   // of a thread
+    static_assert(kUnits * kConvThreads == TX * TY * TZ * GU, "whole units");
+    constexpr int kBatch = kUnits % 4 == 0 ? 4 : 2;
+#pragma unroll 1
+    for (int i0 = 0; i0 < kUnits; i0 += kBatch) {
+        F32Unit v[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+            const int u = threadIdx.x + (i0 + i) * kConvThreads;
+            const int vrow = u / GU, cu = u - vrow * GU;
+            const int L = vrow / TZ, z = vrow % TZ;
+            const int x = bx + L / TY, y = by + L % TY, zz = bz + z;
+            const bool in = x < a.dims[0] && y < a.dims[1] && zz < a.dims[2];
+            v[i] = load_f32(gs, in ? vox(gs.dims, x, y, zz) : 0, cu * 8, in);
+        }
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) gsm[swz(threadIdx.x + (i0 + i) * kConvThreads)] = pack_f32(gs, v[i]);
     }
+    cp_async_wait_all();
     __syncthreads();
     const uint32_t xb = (uint32_t)__cvta_generic_to_shared(smem);
     const uint32_t gb = (uint32_t)__cvta_generic_to_shared(gsm);
@@ -1465,7 +1490,7 @@ cudaError_t forward(Net* n, cudaStream_t s) {
         ConvArgs a;
         layer_sources(n, l, a);
         if (d.mode == IN_POOL) {
-            const Src src = make_src(SRC_BF16_POOL, n->act[d.in0], d.shape.cin, d.shape.cin, 0, n->dims[d.shape.level - 1]);
+            const Src src = make_src(SRC_BF16, n->act[d.in0], d.shape.cin, d.shape.cin, 0, n->dims[d.shape.level - 1]);
             const int* pd = n->dims[d.shape.level];
             k_pool<<<grid_for(nvox(pd) * (d.shape.cin / 8)), 256, 0, s>>>(src, pd[0], pd[1], pd[2], (uint4*)n->pool[l]);
             ++n->launches;
