@@ -665,14 +665,27 @@ __global__ void k_rest_clip32(PassDesc d, int fam, PieceStore ps) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     LocalFace g;
     face_geometry(d, fam, 0, nullptr, g);
+    // in a shared pool, or else in local memory, as k_clip32_deferred (12 us a launch in local memory)
+    typedef ClipPool<36, 28, 1, unsigned long long> RestPool;
+    __shared__ float pool[RestPool::kWords];
+    const RestPool P{pool};
     unsigned st = 0;
-    int npieces = 0;
+    int npieces = 0, nst = 0, nfwd = 0;
     bool multi = false;
+    float N = 0.f, Nr = 0.f;
+    if (clip_both(d, g, P, npieces, multi, nst, nfwd, N, Nr)) {
+        reinterpret_cast<int4*>(ps.rest)[0] = make_int4(nst, range_bits(nfwd, nst - nfwd, multi), npieces, 0);
+        ps.rest[1] = make_float4(N, Nr, 0.f, 0.f);
+        for (int q = 0; q < nst; ++q) ps.rest[2 + q] = P.piece(q);
+        return;
+    }
+    npieces = 0;
+    multi = false;
     PieceSink sink;
     clip32(d, g, st, npieces, multi, sink);
-    const int nfwd = sink.n;
-    const float N = sink.ny.value();
-    float Nr = -N;
+    nfwd = sink.n;
+    N = sink.ny.value();
+    Nr = -N;
     if (multi) {
         int np2 = 0;
         bool m2 = false;
@@ -709,13 +722,16 @@ __global__ void k_rest_fill32(PassDesc d, int fam, PieceStore ps, unsigned* stat
     normal_of(ps, fam)[id] = make_float2(nr.x, nr.y);
 }
 
-// Tiles of kQuadThreads pieces, `run` consecutive ones at a time per CTA: pieces are stored
-// nearly in face order, so a run covers neighbouring z-lines and finds their records in L1.
+// Tiles of kQuadThreads pieces, `run` (up to 8) consecutive ones at a time per CTA: pieces are stored
+// nearly in face order, so a run covers neighbouring z-lines and finds their records in L1.  The number
+// of pieces is the store's own, so a stage whose pieces surely fit is launched without waiting for it.
 // The next tile's piece is loaded before the present one is integrated.  Each piece's flux takes
 // the place of its face tag.
 template <class Body>
-__device__ __forceinline__ void for_pieces(const PassDesc& d, const PieceStore& ps, long long npc, int run, const Body& body) {
+__device__ __forceinline__ void for_pieces(const PassDesc& d, const PieceStore& ps, const Body& body) {
+    const long long npc = min((long long)ps.count[0], (long long)ps.cap);
     const long long ntile = (npc + kQuadThreads - 1) / kQuadThreads;
+    const int run = (int)max(1LL, min(8LL, ntile / (4LL * gridDim.x)));
     long long tile = (long long)blockIdx.x * run;
     int left = run;
     const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -742,11 +758,11 @@ __device__ __forceinline__ void for_pieces(const PassDesc& d, const PieceStore& 
 template <class W>
 __global__ void __launch_bounds__(kQuadThreads, 4) k_quad32(PassDesc d, typename W::Records ar,
                                                             const float4* __restrict__ prec,
-                                                            const float2* __restrict__ psi, PieceStore ps, long long npc,
-                                                            int run, unsigned long long* counters) {
+                                                            const float2* __restrict__ psi, PieceStore ps,
+                                                            unsigned long long* counters) {
     __shared__ float zcol[42 * kQuadThreads];   // each thread's z-pass column (rec_zpass)
     unsigned long long ec = 0;
-    for_pieces(d, ps, npc, run, [&](const float4& p, const int* anc) {
+    for_pieces(d, ps, [&](const float4& p, const int* anc) {
         const float2 b = __ldg(psi + psi_node(d.P, anc[0], anc[1], anc[2]));
         Kahan F;
         ec += (unsigned long long)piece_quad32<W>(d, anc, p.x, p.y, p.z, p.w, ar, prec, PsiLoad{psi, b.x, b.y}, F,
@@ -759,9 +775,8 @@ __global__ void __launch_bounds__(kQuadThreads, 4) k_quad32(PassDesc d, typename
 
 template <int METHOD>
 __global__ void __launch_bounds__(kQuadThreads) k_quad32_plain(PassDesc d, const float* __restrict__ a,
-                                                               const float2* __restrict__ psi, PieceStore ps,
-                                                                long long npc, int run) {
-    for_pieces(d, ps, npc, run, [&](const float4& p, const int* anc) {
+                                                               const float2* __restrict__ psi, PieceStore ps) {
+    for_pieces(d, ps, [&](const float4& p, const int* anc) {
         const float2 b = __ldg(psi + psi_node(d.P, anc[0], anc[1], anc[2]));
         Kahan F;
         piece_quad32_plain<METHOD>(d, anc, p.x, p.y, p.z, p.w, a, PsiLoad{psi, b.x, b.y}, F);
@@ -901,6 +916,10 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
             if (d.volumes) cudaMemsetAsync(w.fvol[fam], 0, nface[fam] * sizeof(float2), s);
         }
     }
+    // At rest at most one line of each colour crosses the unit square: four pieces.  With room for that
+    // many the host does not wait for the count (a density step at 16^3: 9 us less).
+    constexpr long long kRestPieces = 4;
+    const bool fits = rest && ps.clip_fast && ps.cap >= kRestPieces * nface[1];
     unsigned npc = 0;
     cudaError_t ea = cudaFuncSetAttribute(k_clip32, cudaFuncAttributeMaxDynamicSharedMemorySize, kClipSmem);
     if (ea == cudaSuccess)
@@ -921,6 +940,10 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
             k_clip32<<<fb.first[3], kClipThreads, kClipSmem, s>>>(d, fb, disp, ps, w.status, w.counters, ps.clip_fast);
             k_clip32_deferred<<<152 * 4, kDeferThreads, 0, s>>>(d, disp, ps, w.status, w.counters, ps.clip_fast);
         }
+        if (fits) {
+            npc = (unsigned)(kRestPieces * nface[1]);
+            break;
+        }
         cudaError_t e = cudaMemcpyAsync(&npc, ps.count, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return e;
@@ -933,20 +956,19 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
     if (npc > 0) {
         const long long ntile = ((long long)npc + kQuadThreads - 1) / kQuadThreads;
         const unsigned grid = (unsigned)std::min<long long>(ntile, 152 * 8);
-        const int run = (int)std::max<long long>(1, std::min<long long>(8, ntile / (4 * grid)));
         prof_mark(w, 0, s);
         if (d.interp == INTERP_LINEAR)
-            k_quad32_plain<INTERP_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, run);
+            k_quad32_plain<INTERP_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps);
         else if (d.interp != INTERP_WENO6)
-            k_quad32_plain<INTERP_1DY_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, run);
+            k_quad32_plain<INTERP_1DY_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps);
         else if (!w.arec)
-            k_quad32_plain<INTERP_WENO6><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps, (long long)npc, run);
+            k_quad32_plain<INTERP_WENO6><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps);
         else if (d.comp < 0)
             k_quad32<WenoNewton><<<grid, kQuadThreads, 0, s>>>(d, newton_records(d.A, w.arec), (const float4*)w.prec, psi,
-                                                               ps, (long long)npc, run, w.counters);
+                                                               ps, w.counters);
         else
             k_quad32<WenoSamples><<<grid, kQuadThreads, 0, s>>>(d, sample_records(d.A, w.arec), nullptr, psi, ps,
-                                                                (long long)npc, run, w.counters);
+                                                                w.counters);
         prof_mark(w, 1, s);
     }
     FaceSums fs;
