@@ -70,6 +70,7 @@ struct PieceStore {
     int* deferred = nullptr;     // those faces (family << 29 | face index), room for every face
     float4* rest = nullptr;      // the pieces of a face at rest (same for every face of a family)
     unsigned long long* saved = nullptr;   // the session's work counters before a clip (restored on a retry)
+    void* block = nullptr;       // the allocation of range .. saved
     long long cap = 0;           // pieces the buffers hold
     int clip_fast = 1;           // 0: every face through the local-memory clipper
 };

@@ -917,7 +917,7 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
         }
     }
     // At rest at most one line of each colour crosses the unit square: four pieces.  With room for that
-    // many the host does not wait for the count (a density step at 16^3: 9 us less).
+    // many the host does not wait for the count.
     constexpr long long kRestPieces = 4;
     const bool fits = rest && ps.clip_fast && ps.cap >= kRestPieces * nface[1];
     unsigned npc = 0;
@@ -1045,28 +1045,27 @@ cudaError_t piece_store_reserve(PieceStore& p, long long pieces, long long faces
         if (e != cudaSuccess) return e;
         p.cap = pieces;
     }
-    if (!p.count) {
-        cudaError_t e = cudaMalloc(&p.count, 2 * sizeof(unsigned));
-        if (e == cudaSuccess) e = cudaMalloc(&p.saved, 5 * sizeof(unsigned long long));
-        if (e != cudaSuccess) return e;
-    }
-    if (!p.range[0]) {
-        for (int f = 0; f < 3; ++f) {
-            cudaError_t e = cudaMalloc(&p.range[f], faces_per_family * sizeof(int2));
-            if (e == cudaSuccess) e = cudaMalloc(&p.normal[f], faces_per_family * sizeof(float2));
-            if (e != cudaSuccess) return e;
-        }
-        cudaError_t e = cudaMalloc(&p.deferred, 3 * faces_per_family * sizeof(int));
-        if (e == cudaSuccess) e = cudaMalloc(&p.rest, (2 + kMaxPieces32) * sizeof(float4));
-        if (e != cudaSuccess) return e;
+    if (!p.block) {
+        // what does not grow, in one allocation
+        auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+        const size_t nf = (size_t)faces_per_family;
+        const size_t rb = up(nf * sizeof(int2)), nb = up(nf * sizeof(float2)), db = up(3 * nf * sizeof(int));
+        const size_t eb = up((2 + kMaxPieces32) * sizeof(float4)), cb = 256;
+        cudaError_t e = cudaMalloc(&p.block, 3 * rb + 3 * nb + db + eb + 2 * cb);
+        if (e != cudaSuccess) { p.block = nullptr; return e; }
+        char* q = (char*)p.block;
+        auto take = [&](size_t b) { char* r = q; q += b; return r; };
+        p.count = (unsigned*)take(cb);
+        p.saved = (unsigned long long*)take(cb);
+        for (int f = 0; f < 3; ++f) { p.range[f] = (int2*)take(rb); p.normal[f] = (float2*)take(nb); }
+        p.deferred = (int*)take(db);
+        p.rest = (float4*)take(eb);
     }
     return cudaSuccess;
 }
 
 void piece_store_free(PieceStore& p) {
-    cudaFree(p.rec); cudaFree(p.face); cudaFree(p.count); cudaFree(p.deferred); cudaFree(p.rest);
-    cudaFree(p.saved);
-    for (int f = 0; f < 3; ++f) { cudaFree(p.range[f]); cudaFree(p.normal[f]); }
+    cudaFree(p.rec); cudaFree(p.face); cudaFree(p.block);
     p = PieceStore();
 }
 

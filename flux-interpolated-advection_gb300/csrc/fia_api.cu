@@ -163,16 +163,23 @@ cudaError_t reduce(fia_session* s, const void* a, long long n, int kind, bool ac
     return cudaGetLastError();
 }
 
-// kernels launched by one run_pass: psi, backtrace (moving passes), the face stages (one, or
-// three for the flux MacCormack scheme, plus its second trace), gather.  A face stage is three
-// face-family launches (FP64), or three clips, the per-piece quadrature and three per-face
-// sums (FP32 form).
-inline unsigned pass_launches(const PassDesc& d, int precision) {
-    // FP32 form: faces at rest clip and sum the y-faces only (the others emit no piece)
-    const unsigned stage = precision == FIA_FP64 ? 3u : 8u, rest = precision == FIA_FP64 ? 3u : 4u;
-    if (d.zero_velocity) return 2u + rest;
-    if (d.maccormack) return 4u + rest + 2u * stage;
-    return 3u + stage;
+// kernels launched by one run_pass: psi (increments and sums; the plain mode the sums alone), the
+// records, backtrace (moving passes), the face stages (one, or three for the flux MacCormack scheme,
+// plus its second trace), gather.  A face stage of the FP32 form is the clip of the three face
+// families, of the listed faces (at rest: the clip of one face and its copies), the quadrature and the
+// per-face sums; of the FP64 form a clip and a sum per family, the quadrature and the listed faces, or a
+// launch per family with the piece pipeline off.
+inline unsigned pass_launches(const fia_session* s, const PassDesc& d) {
+    const bool fp64 = s->precision == FIA_FP64;
+    const unsigned psi = d.psi_mode == PSI_PLAIN ? 1u : 2u;
+    unsigned rec = 0;
+    if (d.interp == INTERP_WENO6 && s->arec) {
+        if (!fp64 && d.comp >= 0) rec = d.use_integral ? 1u : 0u;
+        else if (!fp64 || (s->piece_pipeline && !d.full_weno)) rec = d.use_integral ? 2u : 1u;
+    }
+    const unsigned stage = !fp64 ? 4u : (s->piece_pipeline ? 8u : 3u);
+    if (d.zero_velocity) return psi + rec + stage + 1u;
+    return psi + rec + 1u + (d.maccormack ? 1u + 3u * stage : stage) + 1u;
 }
 
 // Split offsets (colour = pos/h - off) per field for the main and the error-advection pass
@@ -379,7 +386,7 @@ cudaError_t advect_field(fia_session* s, int comp, const T* in, T* out, double d
     const bool volumes = p->enable_cell_volume_correction && comp < 0;
     d.volumes = volumes ? 1 : 0;
     cudaError_t e = run_pass<T>(d, vel, in, w, in, out, 0, s->stream);
-    s->launches += pass_launches(d, s->precision) + (volumes ? 1 : 0);
+    s->launches += pass_launches(s, d) + (volumes ? 1 : 0);
     if (e == cudaSuccess && volumes) e = volume_correction<T>(s, out);
     d.volumes = 0;
     if (e != cudaSuccess || !p->enable_eliminate_zero_velocity_false_diffusion) return e;
@@ -387,12 +394,12 @@ cudaError_t advect_field(fia_session* s, int comp, const T* in, T* out, double d
     T* c = (T*)s->cbuf;
     d.zero_velocity = 1; d.use_integral = 0; d.psi_mode = PSI_PLAIN;
     e = run_pass<T>(d, vel, in, w, in, c, 1, s->stream);
-    s->launches += pass_launches(d, s->precision);
+    s->launches += pass_launches(s, d);
     if (e != cudaSuccess) return e;
     // pass 3: advect the error with 1Dy-linear interpolation and the error split
     d.zero_velocity = 0; d.interp = INTERP_1DY_LINEAR;
     split_offsets(comp, 1, p->split_method, d.color_off);
-    s->launches += pass_launches(d, s->precision);
+    s->launches += pass_launches(s, d);
     return run_pass<T>(d, vel, c, w, nullptr, out, 2, s->stream);
 }
 
@@ -960,32 +967,42 @@ fia_session* fia_create(int nx, int ny, int nz, double cell_length, int precisio
         g_last_error = "fia_create: stream"; delete s; return nullptr;
     }
     const long long big = (long long)(nx + 2) * (ny + 2) * (nz + 2);
-    auto alloc = [&](size_t bytes) -> void* {
-        void* p = nullptr;
-        if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
-        cudaMemset(p, 0, bytes);
-        s->allocations.push_back(p);
-        return p;
-    };
-    bool ok = true;
-    auto A = [&](void*& dst, size_t bytes) { dst = alloc(bytes); ok = ok && dst != nullptr; };
+    // the session's arrays in one allocation (one by one, a third of the call at 64^3), zeroed
     const size_t fb = (size_t)big * s->es;
     const size_t pb = (size_t)big * 8;   // psi and face fluxes: one double or one float pair per node
-    A(s->rho, fb); A(s->rho_next, fb); A(s->pres, fb); A(s->cbuf, (size_t)big * 8); A(s->psi, pb);
-    for (int c = 0; c < 3; ++c) { A(s->vel[c], fb); A(s->vel_next[c], fb); A(s->flux[c], pb); A(s->flux_rev[c], pb); }
-    A(s->verts, 3 * fb);
+    char* base = nullptr;
+    size_t used = 0;
+    auto take = [&](size_t bytes) -> void* {
+        void* p = base ? base + used : nullptr;
+        used += (bytes + 255) & ~(size_t)255;
+        return p;
+    };
+    auto place = [&] {
+        used = 0;
+        s->rho = take(fb); s->rho_next = take(fb); s->pres = take(fb); s->cbuf = take((size_t)big * 8); s->psi = take(pb);
+        for (int c = 0; c < 3; ++c) {
+            s->vel[c] = take(fb); s->vel_next[c] = take(fb); s->flux[c] = take(pb); s->flux_rev[c] = take(pb);
+        }
+        s->verts = take(3 * fb);
+        for (int q = 0; q < 5; ++q) s->pw[q] = take(fb);
+        s->ticket = (unsigned*)take(4 * sizeof(unsigned));
+        s->part = (double*)take(pressure_partials() * sizeof(double));
+        s->slots = (unsigned long long*)take(pressure_slots() * sizeof(unsigned long long));
+        s->scal = (double*)take(kScalDoubles * sizeof(double));
+        s->sums = (double*)take(8 * sizeof(double));
+        s->status = (unsigned*)take(sizeof(unsigned));
+        s->counters = (unsigned long long*)take(5 * sizeof(unsigned long long));
+        s->red_part = (double*)take(kRedBlocks * sizeof(double));
+        s->red_out = (double*)take(4 * sizeof(double));
+    };
+    place();
     s->verts_bytes = fb;
-    for (int q = 0; q < 5; ++q) A(s->pw[q], fb);
-    { void* t2; A(t2, 4 * sizeof(unsigned)); s->ticket = (unsigned*)t2; }
-    void* t;
-    A(t, pressure_partials() * sizeof(double)); s->part = (double*)t;
-    A(t, pressure_slots() * sizeof(unsigned long long)); s->slots = (unsigned long long*)t;
-    A(t, kScalDoubles * sizeof(double)); s->scal = (double*)t;
-    A(t, 8 * sizeof(double)); s->sums = (double*)t;
-    A(t, sizeof(unsigned)); s->status = (unsigned*)t;
-    A(t, 5 * sizeof(unsigned long long)); s->counters = (unsigned long long*)t;
-    A(t, kRedBlocks * sizeof(double)); s->red_part = (double*)t;
-    A(t, 4 * sizeof(double)); s->red_out = (double*)t;
+    bool ok = cudaMalloc(&base, used) == cudaSuccess;
+    if (ok) {
+        cudaMemset(base, 0, used);
+        s->allocations.push_back(base);
+        place();
+    }
     if (ok && precision == FIA_FP32C) {
         // about 2.8 pieces per face at CFL 2, three face families per pass; grown on demand
         // faces of one family of any (staggered) field fit in (nx+2)(ny+2)(nz+2)
@@ -996,10 +1013,11 @@ fia_session* fia_create(int nx, int ny, int nz, double cell_length, int precisio
         // the z-pass records; a session that finds no memory for them interpolates without
         const size_t ab = (size_t)big * (precision == FIA_FP64 ? kRecBytes64 : kRecBytes);
         const size_t rb = (size_t)big * (precision == FIA_FP64 ? kRecBytes64 : kPsiRecBytes);
-        if (cudaMalloc(&s->arec, ab) != cudaSuccess) s->arec = nullptr;
-        if (!s->arec || cudaMalloc(&s->prec, rb) != cudaSuccess) {
-            cudaFree(s->arec);
-            s->arec = s->prec = nullptr;
+        const size_t at = (ab + 255) & ~(size_t)255;
+        if (cudaMalloc(&s->arec, at + rb) == cudaSuccess) {
+            s->prec = (char*)s->arec + at;
+        } else {
+            s->arec = nullptr;
             cudaGetLastError();
         }
     }
@@ -1049,7 +1067,7 @@ void fia_destroy(fia_session* s) {
     unet::net_destroy(s->net);
     piece_store_free(s->pieces);
     piece_store64_free(s->pieces64);
-    cudaFree(s->arec); cudaFree(s->prec);
+    cudaFree(s->arec);
     if (s->p64) cudaFree(s->p64);
     if (s->solid) cudaFree(s->solid);
     for (void* p : s->allocations) cudaFree(p);
