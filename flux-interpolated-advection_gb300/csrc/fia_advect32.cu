@@ -546,18 +546,6 @@ __device__ __forceinline__ bool clip_both(const PassDesc& d, const LocalFace& g,
     return true;
 }
 
-// The face families of one launch: blocks [first[f], first[f + 1]) hold family f.  One launch for
-// the three instead of one each leaves one partly filled last wave, not three: a MacCormack
-// step on 70 x 97 x 51 cells took 3.50 ms before this and the larger pool below, 2.97 with both.
-struct FamilyBlocks {
-    unsigned first[4];
-    __device__ __forceinline__ int family(unsigned b) const { return b < first[1] ? 0 : (b < first[2] ? 1 : 2); }
-    __device__ __forceinline__ unsigned start(int fam) const { return fam == 0 ? first[0] : (fam == 1 ? first[1] : first[2]); }
-};
-__device__ __forceinline__ long long family_faces(const PassDesc& d, int fam) {
-    return (long long)(d.A.Mx + (fam == 0)) * (d.A.My + (fam == 1)) * (d.A.Mz + (fam == 2));
-}
-
 // fast = 0 sends every face to the list
 __global__ void __launch_bounds__(kClipThreads, kClipBlocks) k_clip32(PassDesc d, FamilyBlocks fb,
                                                                       const float* __restrict__ disp, PieceStore ps,
@@ -884,14 +872,6 @@ __global__ void k_gather32(PassDesc d, const float2* __restrict__ fx, const floa
     if (mode == 0) out[id] = val;
     else if (mode == 1) out[id] = in[id] - val;
     else out[id] = out[id] + val;
-}
-
-// blocks of t threads over the faces of the three families (faces at rest: the y-faces)
-inline FamilyBlocks family_blocks(const long long* nface, bool rest, int t) {
-    FamilyBlocks fb;
-    fb.first[0] = 0;
-    for (int f = 0; f < 3; ++f) fb.first[f + 1] = fb.first[f] + (rest && f != 1 ? 0u : nblk(nface[f], t));
-    return fb;
 }
 
 }  // namespace

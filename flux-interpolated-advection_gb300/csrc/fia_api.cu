@@ -167,7 +167,7 @@ cudaError_t reduce(fia_session* s, const void* a, long long n, int kind, bool ac
 // records, backtrace (moving passes), the face stages (one, or three for the flux MacCormack scheme,
 // plus its second trace), gather.  A face stage of the FP32 form is the clip of the three face
 // families, of the listed faces (at rest: the clip of one face and its copies), the quadrature and the
-// per-face sums; of the FP64 form a clip and a sum per family, the quadrature and the listed faces, or a
+// per-face sums; of the FP64 form the clip, the quadrature, a sum per family and the listed faces, or a
 // launch per family with the piece pipeline off.
 inline unsigned pass_launches(const fia_session* s, const PassDesc& d) {
     const bool fp64 = s->precision == FIA_FP64;
@@ -177,7 +177,7 @@ inline unsigned pass_launches(const fia_session* s, const PassDesc& d) {
         if (!fp64 && d.comp >= 0) rec = d.use_integral ? 1u : 0u;
         else if (!fp64 || (s->piece_pipeline && !d.full_weno)) rec = d.use_integral ? 2u : 1u;
     }
-    const unsigned stage = !fp64 ? 4u : (s->piece_pipeline ? 8u : 3u);
+    const unsigned stage = !fp64 ? 4u : (s->piece_pipeline ? 6u : 3u);
     if (d.zero_velocity) return psi + rec + stage + 1u;
     return psi + rec + 1u + (d.maccormack ? 1u + 3u * stage : stage) + 1u;
 }
