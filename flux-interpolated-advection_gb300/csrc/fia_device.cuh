@@ -283,23 +283,6 @@ __device__ T weno6_3d_collapse(const T* __restrict__ a, const NodeField& F, T h,
     return cxn ? yv[2] : weno6_eval(yv, cx);
 }
 
-// WENO6 along y only; x and z take the node whose cell holds p
-// (WENO6_interpolation_1d.cpp:315-430).
-template <typename T>
-__device__ T weno6_1dy(const T* __restrict__ a, const NodeField& F, T h, T px, T py, T pz) {
-    const int ix = clampi((int)floor(snap_int((px - (T(F.ox) * h - T(0.5) * h)) / h)), F.Mx - 1);
-    const int iz = clampi((int)floor(snap_int((pz - (T(F.oz) * h - T(0.5) * h)) / h)), F.Mz - 1);
-    const T ry = (py - T(F.oy) * h) / h;
-    const int by = (int)floor(ry);
-    T t[6], f[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        t[i] = ry - T(by - 2 + i);
-        f[i] = ldg(a + idx3(F, ix, clampi(by - 2 + i, F.My - 1), iz));
-    }
-    return weno6_eval(f, weno_coef(t));
-}
-
 // Trilinear interpolation with clamped indices (linear_interpolation_3d.cpp:7-95).
 template <typename T>
 __device__ T lin3d(const T* __restrict__ a, const NodeField& F, T h, T px, T py, T pz) {

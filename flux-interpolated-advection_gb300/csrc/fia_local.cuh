@@ -124,22 +124,6 @@ __device__ float weno6_3d_loc(const L& load, const NodeField& F, const int* anc,
 }
 
 template <class L>
-__device__ float weno6_1dy_loc(const L& load, const NodeField& F, const int* anc, const float* q) {
-    int by;
-    float sy;
-    const int ix = clampi(cell_of(anc[0], q[0], F.oxf - 0.5f), F.Mx - 1);
-    const int iz = clampi(cell_of(anc[2], q[2], F.ozf - 0.5f), F.Mz - 1);
-    locate(anc[1], q[1], F.oyf, by, sy);
-    float t[6], f[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        t[i] = sy + float(2 - i);
-        f[i] = load(F.Mz * (F.My * ix + clampi(by - 2 + i, F.My - 1)) + iz);
-    }
-    return weno6_call(f, weno_coef(t));
-}
-
-template <class L>
 __device__ float lin3d_loc(const L& load, const NodeField& F, const int* anc, const float* q) {
     int bx, by, bz;
     float sx, sy, sz;

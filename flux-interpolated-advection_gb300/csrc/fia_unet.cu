@@ -147,16 +147,6 @@ __global__ void k_pool(Src src, int d0, int d1, int d2, uint4* __restrict__ out)
     }
 }
 
-__device__ void stage_scalars(const ConvArgs& a, __nv_bfloat16* sm, int bx, int by, int bz) {
-    for (int hv = threadIdx.x; hv < HV; hv += blockDim.x) {
-        const int hz = hv % HZ, hy = (hv / HZ) % HY, hx = hv / (HZ * HY);
-        const int x = bx + hx - 1, y = by + hy - 1, z = bz + hz - 1;
-        float v = 0.f;
-        if (x >= 0 && y >= 0 && z >= 0 && x < a.dims[0] && y < a.dims[1] && z < a.dims[2]) v = load_scalar(a.s0, x, y, z);
-        sm[hv] = __float2bfloat16_rn(v);
-    }
-}
-
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
