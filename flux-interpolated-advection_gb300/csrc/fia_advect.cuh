@@ -66,8 +66,9 @@ struct PieceStore {
     int* face = nullptr;         // family << 29 | face index; after the quadrature the piece's flux (its bits)
     int2* range[3] = {nullptr, nullptr, nullptr};   // per face: start, nfwd | nrev << 15 | multi << 30
     float2* normal[3] = {nullptr, nullptr, nullptr};  // per face: y-normal sums of both clips (lower, upper cell)
-    unsigned* count = nullptr;   // device counters: [0] pieces, [1] faces listed for the local-memory clipper
+    unsigned* count = nullptr;   // device counters: [0] pieces, [1] faces listed, [2] of them for the local-memory clipper
     int* deferred = nullptr;     // those faces (family << 29 | face index), room for every face
+    long long listcap = 0;       // ints the list array holds
     float4* rest = nullptr;      // the pieces of a face at rest (same for every face of a family)
     unsigned long long* saved = nullptr;   // the session's work counters before a clip (restored on a retry)
     void* block = nullptr;       // the allocation of range .. saved
@@ -132,6 +133,7 @@ struct PassWork {
     void* arec = nullptr;           // z-pass records of the advected field and of psi (fia_weno_rec.cuh)
     void* prec = nullptr;
     PieceStore* pieces = nullptr;   // FP32 form only
+    unsigned long long* launches = nullptr;   // counts the kernels that only some inputs need
     PieceStore64* pieces64 = nullptr;   // FP64 form: the piece pipeline; null: one thread per face (k_faces)
 };
 

@@ -474,8 +474,8 @@ __device__ __forceinline__ int range_bits(int nfwd, int nrev, bool multi) {
 //               when an iso-line crosses a piece more than twice), pieces appended
 //               contiguously per face (warp prefix sum + one atomic per warp), y-normal sums;
 //               a face the shared pool cannot hold goes to a list
-//  k_clip32_deferred  the listed faces, in a larger shared pool or else in local memory, appended
-//               the same way
+//  k_clip32_deferred  the listed faces in a larger shared pool, appended the same way
+//  k_clip32_local  those that outgrow it too, in local memory
 //  k_quad32     one thread per piece: quadrature + WENO6 (uniform work per thread, no clip
 //               code, so fewer registers and no divergence from the piece count);
 //  k_facesum32  one thread per face: compensated sum of its pieces in emission order.
@@ -567,12 +567,12 @@ __global__ void __launch_bounds__(kClipThreads, kClipBlocks) k_clip32(PassDesc d
         if (ok) {
             normal_of(ps, fam)[id] = make_float2(N, Nr);
         } else {
+            npieces = 0;
             const unsigned q = atomicAdd(ps.count + 1, 1u);
             ps.deferred[q] = (fam << 29) | (int)id;
-            npieces = 0; nst = 0; multi = false;
         }
     }
-    const int cnt = nst;
+    const int cnt = ok ? nst : 0;
     const long long start = warp_slots(ps.count, cnt, lane);
     if (ok) {
         if (start + cnt <= ps.cap) {
@@ -586,61 +586,116 @@ __global__ void __launch_bounds__(kClipThreads, kClipBlocks) k_clip32(PassDesc d
     warp_counters((unsigned long long)npieces, ok ? 1u : 0u, (ok && multi) ? 1u : 0u, 0u, lane, status, counters);
 }
 
-// The faces k_clip32 listed (all families): with a larger pool, or else by clip32 in local
-// memory; grid-stride over the list length the clip kernels left in ps.count[1].
+// f(entry of a list of nd, or -1) by whole warps; a short list is spread over the warps: the faces of
+// one would wait for each other.
+template <class Body>
+__device__ __forceinline__ void for_listed(long long nd, const Body& body) {
+    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
+    const long long warps = (long long)gridDim.x * wpb;
+    const int per = (int)min(32LL, (nd + warps - 1) / warps);
+    for (long long base = ((long long)blockIdx.x * wpb + (threadIdx.x >> 5)) * per; base < nd; base += warps * per)
+        body(lane < per && base + lane < nd ? base + lane : -1);
+}
+
+// One listed face a lane (tag -1: none), clipped by clip32 in local memory.
+__device__ __forceinline__ void clip_local(const PassDesc& d, int tag, const float* __restrict__ disp,
+                                           const PieceStore& ps, unsigned* status, unsigned long long* counters) {
+    const int fam = tag >> 29, lane = threadIdx.x & 31;
+    const long long id = tag & ((1 << 29) - 1);
+    unsigned st = 0;
+    int npieces = 0, nfwd = 0;
+    bool multi = false;
+    PieceSink sink;
+    if (tag >= 0) {
+        LocalFace g;
+        face_geometry(d, fam, id, disp, g);
+        clip32(d, g, st, npieces, multi, sink);
+        nfwd = sink.n;
+        const float N = sink.ny.value();
+        float Nr = -N;
+        if (multi) {
+            int np2 = 0;
+            bool m2 = false;
+            sink.ny = Kahan();
+            clip32(d, reversed_face(g), st, np2, m2, sink);
+            Nr = sink.ny.value();
+        }
+        normal_of(ps, fam)[id] = make_float2(N, Nr);
+    }
+    const int cnt = sink.n;
+    const long long start = warp_slots(ps.count, cnt, lane);
+    if (tag >= 0) {
+        if (start + cnt <= ps.cap)
+            for (int q = 0; q < cnt; ++q) { ps.rec[start + q] = sink.p[q]; ps.face[start + q] = tag; }
+        range_of(ps, fam)[id] = make_int2((int)start, range_bits(nfwd, cnt - nfwd, multi));
+    }
+    warp_counters((unsigned long long)npieces, tag >= 0 ? 1u : 0u, (tag >= 0 && multi) ? 1u : 0u, st, lane, status, counters);
+}
+
+// The faces k_clip32 listed (all families), ps.count[1] of them, in a larger pool.  Those that outgrow it
+// too are for the local-memory clipper.  Of a short list (a face a warp) they are clipped here; of a longer
+// one they are moved to the back of the list array and counted in ps.count[2], or keep their place
+// where the array has no room left, the other places blanked.
+//
+// The local-memory clipper then has a kernel of its own, because a warp in which one face needs it waits
+// for that face, and because the pools leave 8 warps on an SM here: with it in this kernel for every
+// list, a density step at 64^3 took 7.7 ms at CFL 16 (two faces in five listed, one in fifty past the larger
+// pool) and 23 ms at CFL 24, and 3.6 and 6.6 ms so.  Faces over kDeferCells cells or more (clip_cells) are moved
+// without an attempt: of those over 20 to 30 half would fit, of larger ones hardly any.
+constexpr int kDeferBlocks = 152 * 4, kDeferCells = 20;
+__host__ __device__ __forceinline__ bool short_list(unsigned listed) {
+    return listed <= (unsigned)(kDeferBlocks * (kDeferThreads / 32));
+}
 __global__ void __launch_bounds__(kDeferThreads) k_clip32_deferred(PassDesc d, const float* __restrict__ disp, PieceStore ps,
                                                                    unsigned* status, unsigned long long* counters,
                                                                    int fast) {
     __shared__ float pool[DeferPool::kWords * kDeferThreads];
     const DeferPool P{pool + threadIdx.x};
-    const long long nd = (long long)ps.count[1];
+    const unsigned nd = ps.count[1];
+    const bool few = short_list(nd);
     const int lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x == 0 && nd > 0) atomicAdd(&counters[4], (unsigned long long)nd);
-    // a short list is spread over the warps: the faces of one would wait for each other
-    const long long warps = (long long)gridDim.x * (kDeferThreads / 32);
-    const int per = (int)min(32LL, (nd + warps - 1) / warps);
-    for (long long base = ((long long)blockIdx.x * (kDeferThreads / 32) + (threadIdx.x >> 5)) * per; base < nd;
-         base += warps * per) {
-        const long long t = base + lane;
-        const bool valid = lane < per && t < nd;
-        const int tag = valid ? ps.deferred[t] : 0;
+    for_listed(nd, [&](long long t) {
+        const int tag = t >= 0 ? ps.deferred[t] : 0;
         const int fam = tag >> 29;
         const long long id = tag & ((1 << 29) - 1);
-        unsigned st = 0;
         int npieces = 0, cnt = 0, nfwd = 0;
-        bool multi = false, pooled = false;
-        PieceSink sink;
-        if (valid) {
+        bool multi = false, ok = false;
+        if (t >= 0) {
             LocalFace g;
             face_geometry(d, fam, id, disp, g);
             float N = 0.f, Nr = 0.f;
-            pooled = fast != 0 && clip_both(d, g, P, npieces, multi, cnt, nfwd, N, Nr);
-            if (!pooled) {
-                npieces = 0;
-                multi = false;
-                clip32(d, g, st, npieces, multi, sink);
-                nfwd = sink.n;
-                N = sink.ny.value();
-                Nr = -N;
-                if (multi) {
-                    int np2 = 0;
-                    bool m2 = false;
-                    sink.ny = Kahan();
-                    clip32(d, reversed_face(g), st, np2, m2, sink);
-                    Nr = sink.ny.value();
-                }
-                cnt = sink.n;
-            }
-            normal_of(ps, fam)[id] = make_float2(N, Nr);
+            ok = fast != 0 && (few || clip_cells(d, g) < kDeferCells) && clip_both(d, g, P, npieces, multi, cnt, nfwd, N, Nr);
+            if (ok) normal_of(ps, fam)[id] = make_float2(N, Nr);
         }
+        if (!ok) npieces = cnt = 0;
         const long long start = warp_slots(ps.count, cnt, lane);
-        if (valid) {
+        if (ok) {
             if (start + cnt <= ps.cap)
-                for (int q = 0; q < cnt; ++q) { ps.rec[start + q] = pooled ? P.piece(q) : sink.p[q]; ps.face[start + q] = tag; }
+                for (int q = 0; q < cnt; ++q) { ps.rec[start + q] = P.piece(q); ps.face[start + q] = tag; }
             range_of(ps, fam)[id] = make_int2((int)start, range_bits(nfwd, cnt - nfwd, multi));
         }
-        warp_counters((unsigned long long)npieces, valid ? 1u : 0u, (valid && multi) ? 1u : 0u, st, lane, status, counters);
-    }
+        warp_counters((unsigned long long)npieces, ok ? 1u : 0u, (ok && multi) ? 1u : 0u, 0u, lane, status, counters);
+        const bool left = t >= 0 && !ok;
+        if (few) {
+            if (__any_sync(0xffffffffu, left)) clip_local(d, left ? tag : -1, disp, ps, status, counters);
+        } else if (t >= 0) {
+            const long long q = left ? (long long)atomicAdd(ps.count + 2, 1u) : 0;
+            const bool keep = left && nd + q >= ps.listcap;
+            if (left && !keep) ps.deferred[ps.listcap - 1 - q] = tag;
+            if (!keep) ps.deferred[t] = -1;
+        }
+    });
+}
+
+// The faces that k_clip32_deferred leaves: ps.count[2] of them, those past the room in their old places.
+__global__ void __launch_bounds__(128) k_clip32_local(PassDesc d, const float* __restrict__ disp, PieceStore ps,
+                                                      unsigned* status, unsigned long long* counters) {
+    const long long nd = ps.count[1], left = ps.count[2], room = ps.listcap - nd, moved = min(left, room);
+    for_listed(left > room ? moved + nd : moved, [&](long long t) {
+        const int tag = t < 0 ? -1 : (t < moved ? ps.deferred[ps.listcap - 1 - t] : ps.deferred[t - moved]);
+        clip_local(d, tag, disp, ps, status, counters);
+    });
 }
 
 // Faces at rest (the zero-velocity pass, the MacCormack face at rest) are the same square in
@@ -653,7 +708,7 @@ __global__ void k_rest_clip32(PassDesc d, int fam, PieceStore ps) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     LocalFace g;
     face_geometry(d, fam, 0, nullptr, g);
-    // in a shared pool, or else in local memory, as k_clip32_deferred (12 us a launch in local memory)
+    // in a shared pool, or else in local memory (12 us a launch)
     typedef ClipPool<36, 28, 1, unsigned long long> RestPool;
     __shared__ float pool[RestPool::kWords];
     const RestPool P{pool};
@@ -909,7 +964,7 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
     ea = cudaMemcpyAsync(ps.saved, w.counters, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s);
     if (ea != cudaSuccess) return ea;
     for (int attempt = 0; attempt < 2; ++attempt) {
-        cudaMemsetAsync(ps.count, 0, 2 * sizeof(unsigned), s);
+        cudaMemsetAsync(ps.count, 0, 3 * sizeof(unsigned), s);
         if (attempt > 0)
             cudaMemcpyAsync(w.counters, ps.saved, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s);
         if (rest && ps.clip_fast) {
@@ -918,15 +973,23 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
         } else {
             const FamilyBlocks fb = family_blocks(nface, rest, kClipThreads);
             k_clip32<<<fb.first[3], kClipThreads, kClipSmem, s>>>(d, fb, disp, ps, w.status, w.counters, ps.clip_fast);
-            k_clip32_deferred<<<152 * 4, kDeferThreads, 0, s>>>(d, disp, ps, w.status, w.counters, ps.clip_fast);
+            k_clip32_deferred<<<kDeferBlocks, kDeferThreads, 0, s>>>(d, disp, ps, w.status, w.counters, ps.clip_fast);
         }
         if (fits) {
             npc = (unsigned)(kRestPieces * nface[1]);
             break;
         }
-        cudaError_t e = cudaMemcpyAsync(&npc, ps.count, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+        unsigned counts[3];   // pieces, faces listed, faces left
+        cudaError_t e = cudaMemcpyAsync(counts, ps.count, sizeof(counts), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e == cudaSuccess && counts[2] > 0) {
+            k_clip32_local<<<152 * 8, 128, 0, s>>>(d, disp, ps, w.status, w.counters);
+            if (w.launches) ++*w.launches;
+            e = cudaMemcpyAsync(counts, ps.count, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        }
         if (e != cudaSuccess) return e;
+        npc = counts[0];
         if ((long long)npc <= ps.cap) break;
         // more pieces than the store holds: grow it and clip again
         e = piece_store_reserve(ps, (long long)npc + npc / 4 + 1024, std::max(nface[0], std::max(nface[1], nface[2])));
@@ -1039,6 +1102,7 @@ cudaError_t piece_store_reserve(PieceStore& p, long long pieces, long long faces
         p.saved = (unsigned long long*)take(cb);
         for (int f = 0; f < 3; ++f) { p.range[f] = (int2*)take(rb); p.normal[f] = (float2*)take(nb); }
         p.deferred = (int*)take(db);
+        p.listcap = 3 * faces_per_family;
         p.rest = (float4*)take(eb);
     }
     return cudaSuccess;

@@ -166,8 +166,8 @@ cudaError_t reduce(fia_session* s, const void* a, long long n, int kind, bool ac
 // kernels launched by one run_pass: psi (increments and sums; the plain mode the sums alone), the
 // records, backtrace (moving passes), the face stages (one, or three for the flux MacCormack scheme,
 // plus its second trace), gather.  A face stage of the FP32 form is the clip of the three face
-// families, of the listed faces (at rest: the clip of one face and its copies), the quadrature and the
-// per-face sums; of the FP64 form the clip, the quadrature, a sum per family and the listed faces, or a
+// families, of the listed faces (at rest: the clip of one face and its copies; the local-memory clipper's
+// launch, which few passes need, counts itself), the quadrature and the per-face sums; of the FP64 form the clip, the quadrature, a sum per family and the listed faces, or a
 // launch per family with the piece pipeline off.
 inline unsigned pass_launches(const fia_session* s, const PassDesc& d) {
     const bool fp64 = s->precision == FIA_FP64;
@@ -252,6 +252,7 @@ PassWork<T> work(fia_session* s) {
     w.prof_cap = (int)(s->prof_ev.size() / 2);
     w.arec = s->arec; w.prec = s->prec;
     w.pieces = &s->pieces;
+    w.launches = &s->launches;
     w.pieces64 = (s->precision == FIA_FP64 && s->piece_pipeline) ? &s->pieces64 : nullptr;
     return w;
 }

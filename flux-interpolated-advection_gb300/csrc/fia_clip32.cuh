@@ -537,6 +537,17 @@ static __host__ __device__ bool clip32_fast(const PassDesc& d, const LocalFace& 
     }
 }
 
+// cells under the bounding box of a face's colours (a bound on its pieces where no polygon is split in
+// more than two)
+__host__ __device__ __forceinline__ int clip_cells(const PassDesc& d, const LocalFace& g) {
+    auto span = [](const float* v, float off) {
+        const float mn = fminf(fminf(v[0], v[1]), fminf(v[2], v[3])) - off;
+        const float mx = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3])) - off;
+        return fminf(fmaxf(ceilf(mx) - floorf(mn), 1.f), 1000.f);
+    };
+    return (int)(span(g.x, d.color_off_f[0]) * span(g.z, d.color_off_f[1]));
+}
+
 // the upper cell's vertex order (v0, v3, v2, v1)
 __host__ __device__ __forceinline__ LocalFace reversed_face(const LocalFace& g) {
     LocalFace r = g;

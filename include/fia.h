@@ -316,8 +316,8 @@ int fia_debug_learned_grad(fia_session* s, int pair, float* grads, double* loss)
 int fia_debug_learned_tc(fia_session* s, int enable, unsigned* status);
 /* FP32 form: the face clipper's shared-memory path: enable 1 / 0 switches it on / off (on
  * by default; off clips every face in local memory, with the same pieces), -1 leaves it;
- * *deferred (if not null) receives the faces the local-memory clipper took since fia_create
- * (faces the shared pool cannot hold, or all faces while the path is off). */
+ * *deferred (if not null) receives the faces listed since fia_create (those the first shared
+ * pool cannot hold, for a larger one or the local-memory clipper; all faces while the path is off). */
 int fia_debug_clip_fast(fia_session* s, int enable, unsigned long long* deferred);
 /* FP64 form: enable 1 evaluates every WENO6 interpolation in full, 0 (the default) collapses
  * it along the axes on which the point lies on a node plane of the field (vertices at rest,
