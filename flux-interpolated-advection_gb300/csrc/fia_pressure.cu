@@ -316,20 +316,24 @@ __device__ __forceinline__ void stv(T* __restrict__ p, const T (&v)[W]) {
     else p[0] = v[0];
 }
 
-// warp sum of a float-float accumulator; lane 0 holds the total
-__device__ __forceinline__ double warp_total(const DotAcc<float>& a) {
-    float hi = a.hi, lo = a.lo;
+// warp sum of an accumulator, as one; lane 0 holds the total
+__device__ __forceinline__ DotAcc<float> acc_warp(DotAcc<float> a) {
     for (int o = 16; o > 0; o >>= 1) {
-        const float h2 = __shfl_down_sync(0xffffffffu, hi, o), l2 = __shfl_down_sync(0xffffffffu, lo, o);
-        const float s = __fadd_rn(hi, h2);
-        const float bb = __fsub_rn(s, hi);
-        const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(h2, bb));
-        hi = s;
-        lo = __fadd_rn(__fadd_rn(lo, l2), e);
+        const float h2 = __shfl_down_sync(0xffffffffu, a.hi, o), l2 = __shfl_down_sync(0xffffffffu, a.lo, o);
+        const float s = __fadd_rn(a.hi, h2);
+        const float bb = __fsub_rn(s, a.hi);
+        const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(h2, bb));
+        a.hi = s;
+        a.lo = __fadd_rn(__fadd_rn(a.lo, l2), e);
     }
-    return (double)hi + (double)lo;
+    return a;
 }
-__device__ __forceinline__ double warp_total(const DotAcc<double>& a) { return warp_sum(a.s); }
+__device__ __forceinline__ DotAcc<double> acc_warp(DotAcc<double> a) {
+    a.s = warp_sum(a.s);
+    return a;
+}
+template <typename T>
+__device__ __forceinline__ double warp_total(const DotAcc<T>& a) { return acc_warp(a).value(); }
 
 // block sums of NV accumulators into part[b + nb*q] (FP64 conversions only per warp)
 template <typename T, int NV>
@@ -535,15 +539,16 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update(PoissonGrid g, double
 // Along y and z the operator reads shared memory; along x the neighbour's d = z + beta d_old is
 // formed from the z and d_old that its block stored before the last meeting, as in
 // k_cg_direction_apply.  The arithmetic on the vectors is that of the two kernels above, cell by
-// cell; only the order of the (FP64-accurate) dot sums differs.
+// cell, and its dots are float pairs within a warp and FP64 from there on, as theirs; only their order
+// differs.
 //
-// What an iteration costs is latency: FP64 operations run in one thread (one of every thread of a
-// block takes a quarter of a microsecond; the FP32 form adds its dots up as float pairs), the
-// neighbours' loads are issued before the block's own cells are updated, and what a group of cells
-// needs of its place in the grid is one word, made once.  Microseconds an iteration, with the two
-// kernels above and with this one: FP32 16^3 18 -> 7.0, 64^3 23 -> 10.7, 128^3 36 -> 18.7, 160^3 53 ->
-// 48, 176^3 71 -> 71; FP64 64^3 46 -> 18, 128^3 134 -> 79.  (Slots polled by every block, with the
-// meeting's number beside the value instead of a counter, were slower: 19.8 against 14 us at 64^3.)
+// What an iteration costs is latency: FP64 operations run in one thread or one warp (one of every
+// thread of a block takes a quarter of a microsecond), the neighbours' loads are issued before the
+// block's own cells are updated, and what a group of cells needs of its place in the grid is one word,
+// made once.  Microseconds an iteration, with the two kernels above and with this one: FP32 16^3 18 ->
+// 7.1, 64^3 23 -> 10.3, 128^3 36 -> 17.9, 160^3 53 -> 48; FP64 64^3 46 -> 17.6, 128^3 134 -> 79.  (Slots
+// polled by every block, with the meeting's number beside the value instead of a counter, were slower:
+// 19.8 against 14 us at 64^3.)
 // Larger grids, whose chunks leave no room for two shared arrays, keep the two kernels: there the
 // vectors' traffic is the time (256^3: 152 us for 11 vectors of 67 MB, 108 us at the copy rate).
 constexpr int kPcgThreadsMax = 1024;
@@ -551,7 +556,7 @@ constexpr int kPcgIters = 256;           // iterations per launch
 constexpr int kPcgSpinLimit = 1 << 21;   // polls of a meeting before the kernel gives up
 constexpr unsigned kPcgStuck = 1u << 30; // set in the counter when one did
 constexpr size_t kPcgSmem = 224 * 1024;  // dynamic shared memory of a block (227 KB less the static part)
-constexpr int kPcgPartWords = 3;         // 64-bit words a block: one value, then two
+constexpr int kPcgPartWords = 3;         // doubles a block: one sum, then two
 constexpr int kPcgBlocksMax = 1024;
 constexpr unsigned kPcgOneBlock = 1024;  // groups that one block takes alone
 
@@ -560,7 +565,7 @@ struct PcgArgs {
     PoissonGrid g;
     T *x, *r, *z, *d0, *d1;
     double* scal;
-    unsigned long long* parts;   // kPcgPartWords * gridDim.x
+    double* parts;               // kPcgPartWords * gridDim.x
     unsigned* bar;               // arrivals, zero at launch
     unsigned chunk;              // cells per block, a multiple of W
     int iters;                   // at most this many iterations
@@ -593,35 +598,15 @@ __device__ __forceinline__ unsigned pcg_place(const PoissonGrid& g, unsigned c) 
     return p;
 }
 
-// Sums of accumulators, kept as accumulators (a float pair in the FP32 form, whose sums then need
-// no FP64 operation).
-__device__ __forceinline__ void acc_join(DotAcc<float>& a, float hi, float lo) {
-    const float s = __fadd_rn(a.hi, hi);
-    const float bb = __fsub_rn(s, a.hi);
-    const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(hi, bb));
-    a.hi = s;
-    a.lo = __fadd_rn(__fadd_rn(a.lo, lo), e);
-}
-__device__ __forceinline__ DotAcc<float> acc_warp(DotAcc<float> a) {
-    for (int o = 16; o > 0; o >>= 1)
-        acc_join(a, __shfl_down_sync(0xffffffffu, a.hi, o), __shfl_down_sync(0xffffffffu, a.lo, o));
-    return a;
-}
-__device__ __forceinline__ DotAcc<double> acc_warp(DotAcc<double> a) {
-    a.s = warp_sum(a.s);
-    return a;
-}
-
 // All blocks meet: publishes the block's NV sums of its threads' accumulators and returns their
 // sums over the blocks in tot[] (thread 0; every block adds them up in the same order).  What the
 // block's threads stored to global memory before is visible to every block after (loads past L1).
-// parts: NV words a block, not those of the meeting before.  False when the wait ran out.
+// FP64 from the warps' sums on, as block_dots; by one warp a sum, which has the blocks' sums in flight
+// together.  parts: NV doubles a block, not those of the meeting before.  False when the wait ran out.
 template <typename T, int NV>
-__device__ __forceinline__ bool pcg_meet(const DotAcc<T> (&acc)[NV], unsigned long long* parts, unsigned* bar,
-                                         unsigned target, double* tot) {
-    static_assert(sizeof(DotAcc<T>) == 8, "an accumulator is one 64-bit word");
+__device__ __forceinline__ bool pcg_meet(const DotAcc<T> (&acc)[NV], double* parts, unsigned* bar, unsigned target,
+                                         double* tot) {
     __shared__ DotAcc<T> sh[NV][32];
-    __shared__ DotAcc<T> bsum[NV][kPcgBlocksMax / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, nb = gridDim.x;
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
@@ -631,17 +616,21 @@ __device__ __forceinline__ bool pcg_meet(const DotAcc<T> (&acc)[NV], unsigned lo
     __syncthreads();
     bool ok = true;
     if (warp == 0) {
-        DotAcc<T> t[NV];
+        double t[NV];
 #pragma unroll
-        for (int q = 0; q < NV; ++q) t[q] = acc_warp(lane < nw ? sh[q][lane] : DotAcc<T>());
+        for (int q = 0; q < NV; ++q) t[q] = lane < nw ? sh[q][lane].value() : 0.0;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            if (nw > 16) t[q] += __shfl_down_sync(0xffffffffu, t[q], 16);
+            for (int o = 8; o > 0; o >>= 1) t[q] += __shfl_down_sync(0xffffffffu, t[q], o);
+        }
         if (lane == 0) {
             if (nb == 1) {
 #pragma unroll
-                for (int q = 0; q < NV; ++q) tot[q] = t[q].value();
+                for (int q = 0; q < NV; ++q) tot[q] = t[q];
             } else {
 #pragma unroll
-                for (int q = 0; q < NV; ++q)
-                    __stcg(parts + (size_t)q * nb + blockIdx.x, *reinterpret_cast<const unsigned long long*>(&t[q]));
+                for (int q = 0; q < NV; ++q) __stcg(parts + (size_t)q * nb + blockIdx.x, t[q]);
                 unsigned seen;
                 asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
                 int it = 0;
@@ -655,26 +644,20 @@ __device__ __forceinline__ bool pcg_meet(const DotAcc<T> (&acc)[NV], unsigned lo
     }
     if (nb == 1) return true;
     if (!__syncthreads_and(ok)) return false;
-    const int per = (nb + 31) >> 5;
-    for (int job = warp; job < NV * per; job += nw) {
-        const int q = job / per, b = (job - q * per) * 32 + lane;
-        DotAcc<T> t;
-        if (b < nb) {
-            const unsigned long long w = __ldcg(parts + (size_t)q * nb + b);
-            t = *reinterpret_cast<const DotAcc<T>*>(&w);
+    if (warp < NV) {
+        constexpr int kAhead = 5;   // loads in flight: all of 152 blocks
+        double t = 0.0;
+        for (int b0 = lane; b0 < nb; b0 += 32 * kAhead) {
+            double v[kAhead];
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) v[j] = b0 + 32 * j < nb ? __ldcg(parts + (size_t)warp * nb + b0 + 32 * j) : 0.0;
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) t += v[j];
         }
-        t = acc_warp(t);
-        if (lane == 0) bsum[q][job - q * per] = t;
+        t = warp_sum(t);
+        if (lane == 0) tot[warp] = t;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            double t = 0.0;
-            for (int j = 0; j < per; ++j) t += bsum[q][j].value();
-            tot[q] = t;
-        }
-    }
     return true;
 }
 
@@ -1164,9 +1147,9 @@ PcgPlan pcg_plan(const PoissonGrid& g) {
         const size_t smem = ((size_t)a * chunk + 2 * (size_t)g.nz) * sizeof(T);
         if (smem > kPcgSmem) continue;
         p.blocks = (int)blocks;
-        // a thread a group; in FP64, whose sums across a warp cost most, two where there are many
-        // (64^3 18.4 against 20.2 us an iteration)
-        const unsigned per = sizeof(T) == 8 && chunk / W > 512 ? 2 : 1;
+        // a thread a group; two where there are many in FP64, whose sums across a warp cost most
+        // (64^3 18.4 against 20.2 us an iteration), and in one block (16^3 FP32 4.8 against 5.1)
+        const unsigned per = (sizeof(T) == 8 || blocks == 1) && chunk / W > 512 ? 2 : 1;
         p.threads = (int)std::min<unsigned>(kPcgThreadsMax, std::max<unsigned>(128u, (chunk / W / per + 31) / 32 * 32));
         p.placed = chunk / W <= 4u * p.threads;
         p.arrays = a; p.chunk = chunk; p.smem = smem;
@@ -1216,7 +1199,7 @@ cudaError_t pressure_pcg(const PressureWork<T>& W, const PoissonGrid& g, double 
         const int batch = std::min(plan.blocks ? kPcgIters : kCgBatch, max_iter - launched);
         if (plan.blocks) {
             cudaError_t e = cudaMemsetAsync(W.slots, 0, sizeof(unsigned long long), s);
-            const PcgArgs<T> A{g, W.p, W.r, W.z, dold, dnew, W.scal, W.slots + 1, (unsigned*)W.slots, plan.chunk, batch, launched == 0};
+            const PcgArgs<T> A{g, W.p, W.r, W.z, dold, dnew, W.scal, (double*)(W.slots + 1), (unsigned*)W.slots, plan.chunk, batch, launched == 0};
             if (e == cudaSuccess) e = launch_pcg<T>(plan, A, s);
             if (e == cudaErrorCooperativeLaunchTooLarge) {   // not all blocks fit at once: launch by launch
                 cudaGetLastError();
