@@ -449,8 +449,9 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_direction_apply(PoissonGrid 
     }
     block_dots<T, 2>(acc, part);
     if (last_block(ticket)) {
-        double t[2];
-        block_totals<2>(part, gridDim.x, t);   // without rres the second is zero
+        double t[2] = {0.0, 0.0};
+        if (rres) block_totals<2>(part, gridDim.x, t);
+        else block_totals<1>(part, gridDim.x, reinterpret_cast<double (&)[1]>(t));
         if (threadIdx.x == 0) {
             const double num = rres ? t[1] : scal[S_RZ];
             scal[S_ALPHA] = t[0] != 0.0 ? num / t[0] : 0.0;
@@ -549,6 +550,8 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update(PoissonGrid g, double
 // 7.1, 64^3 23 -> 10.3, 128^3 36 -> 17.9, 160^3 53 -> 48; FP64 64^3 46 -> 17.6, 128^3 134 -> 79.  (Slots
 // polled by every block, with the meeting's number beside the value instead of a counter, were slower:
 // 19.8 against 14 us at 64^3.)
+// Rows that are no whole groups take one cell a step, and their places are formed at each visit from 4096
+// cells a block on: 127^3 49 -> 41, 143^3 61 -> 61, 151^3 70 -> 70, 161^3 82 -> 81; FP64 127^3 136 -> 81.
 // Larger grids, whose chunks leave no room for two shared arrays, keep the two kernels: there the
 // vectors' traffic is the time (256^3: 152 us for 11 vectors of 67 MB, 108 us at the copy rate).
 constexpr int kPcgThreadsMax = 1024;
