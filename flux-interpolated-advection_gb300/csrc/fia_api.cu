@@ -62,6 +62,7 @@ struct fia_session {
     bool fcg_ready = false;
     double* p64 = nullptr;       // FP32 form: pressure accumulated in FP64 by the refinement
     int full_weno = 0;           // FP64 form: no WENO6 collapse on node planes (fia_debug_full_weno)
+    int pcg_stuck = 0;           // the one-kernel CG's first wait counts as run out (fia_debug_pcg_stuck)
     double vertex_jitter = 0.0;  // FP64 form: backtraced vertices jittered (fia_debug_vertex_jitter)
     mutable unsigned jitter_calls = 0;
     // clipped pieces of a pass (FP64 form); piece_pipeline 0: one thread per face instead
@@ -443,7 +444,7 @@ PressureWork<T> pressure_work(fia_session* s) {
     PressureWork<T> W;
     W.p = (T*)s->pres; W.r = (T*)s->pw[0]; W.z = (T*)s->pw[1]; W.d = (T*)s->pw[2]; W.q = (T*)s->pw[3];
     W.d2 = (T*)s->pw[4]; W.ticket = s->ticket; W.slots = s->slots;
-    W.part = s->part; W.scal = s->scal; W.sums = s->sums;
+    W.part = s->part; W.scal = s->scal; W.sums = s->sums; W.stuck = s->pcg_stuck != 0;
     return W;
 }
 
@@ -1544,6 +1545,12 @@ int fia_debug_piece_pipeline(fia_session* s, int enable) {
         s->piece_pipeline = enable;
     }
     return s->precision == FIA_FP64 ? s->piece_pipeline : 0;
+}
+
+int fia_debug_pcg_stuck(fia_session* s, int enable) {
+    if (!s || enable < -1 || enable > 1) return FIA_ERR_INVALID;
+    if (enable >= 0) s->pcg_stuck = enable;
+    return s->pcg_stuck;
 }
 
 int fia_debug_full_weno(fia_session* s, int enable) {

@@ -1201,7 +1201,8 @@ cudaError_t pressure_pcg(const PressureWork<T>& W, const PoissonGrid& g, double 
     while (launched < max_iter && st[0] == 0.0) {
         const int batch = std::min(plan.blocks ? kPcgIters : kCgBatch, max_iter - launched);
         if (plan.blocks) {
-            cudaError_t e = cudaMemsetAsync(W.slots, 0, sizeof(unsigned long long), s);
+            static_assert(0x40404040u >= kPcgStuck && 0x40404040u < 2 * kPcgStuck, "a counter in which a wait ran out");
+            cudaError_t e = cudaMemsetAsync(W.slots, W.stuck ? 0x40 : 0, sizeof(unsigned long long), s);
             const PcgArgs<T> A{g, W.p, W.r, W.z, dold, dnew, W.scal, (double*)(W.slots + 1), (unsigned*)W.slots, plan.chunk, batch, launched == 0};
             if (e == cudaSuccess) e = launch_pcg<T>(plan, A, s);
             if (e == cudaErrorCooperativeLaunchTooLarge) {   // not all blocks fit at once: launch by launch

@@ -35,6 +35,7 @@ struct PressureWork {
     double* sums;               // 4 doubles
     unsigned* ticket;           // 4 last-block counters (zero between kernels)
     unsigned long long* slots;  // pressure_slots() words: where the blocks of k_pcg meet
+    bool stuck = false;         // tests: the first meeting of k_pcg finds that a wait ran out
 };
 
 struct PressureReport {

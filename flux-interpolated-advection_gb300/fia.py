@@ -184,6 +184,7 @@ def _declare(lib):
     lib.fia_debug_learned_tc.argtypes = [vp, ip, ctypes.POINTER(ctypes.c_uint)]
     lib.fia_debug_clip_fast.argtypes = [vp, ip, ctypes.POINTER(ctypes.c_ulonglong)]
     lib.fia_debug_full_weno.argtypes = [vp, ip]
+    lib.fia_debug_pcg_stuck.argtypes = [vp, ip]
     lib.fia_debug_piece_pipeline.argtypes = [vp, ip]
     lib.fia_debug_vertex_jitter.argtypes = [vp, ctypes.c_double]
     lib.fia_debug_learned_grad.argtypes = [vp, ip, fp, dp]
@@ -505,6 +506,9 @@ class Grid3D:
         """FP64 form: 1 evaluates every WENO6 in full, 0 collapses it on node planes (default),
         -1 leaves it; returns the setting"""
         return _check(self.lib.fia_debug_full_weno(self.s, enable), "fia_debug_full_weno")
+
+    def debug_pcg_stuck(self, enable=-1):
+        return _check(self.lib.fia_debug_pcg_stuck(self.s, enable), "fia_debug_pcg_stuck")
 
     def debug_piece_pipeline(self, enable=-1):
         """FP64 form: 1 runs the faces as the piece pipeline (default), 0 as one thread per face,

@@ -324,6 +324,10 @@ int fia_debug_clip_fast(fia_session* s, int enable, unsigned long long* deferred
  * psi points of the pieces: equal in exact arithmetic, fewer evaluations), -1 leaves it;
  * returns the setting. */
 int fia_debug_full_weno(fia_session* s, int enable);
+/* the one-kernel Jacobi-PCG: enable 1 makes the first meeting of its blocks find that a bounded wait
+ * ran out (the call then returns FIA_ERR_CUDA; the session stays usable), 0 (the default) not, -1
+ * leaves it; returns the setting. */
+int fia_debug_pcg_stuck(fia_session* s, int enable);
 /* FP64 form: enable 1 (the default) runs each pass's faces as the piece pipeline (a thread per
  * face clips and stores its pieces, a thread per piece integrates, a thread per face sums in
  * emission order), 0 as one thread per face that integrates each piece as it is clipped (the
