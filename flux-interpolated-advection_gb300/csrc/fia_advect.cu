@@ -877,24 +877,45 @@ __device__ __forceinline__ int base64(double r, double& s) {
     return b;
 }
 
+// What a z-interpolation at stencil base b1 - 1 of a row needs: from the field's records, or, in a session
+// that has no memory for them, from the six samples (a density step at 40^3: 6.5 and 9.1 ms; 20.7
+// before there were records).
+struct RowRecords {
+    const WenoRec<double>* __restrict__ r;
+    int Mz;
+    __device__ __forceinline__ WenoData<double> data(int row, int b1) const {
+        return weno_unpack(ldg_rec(r + (long long)row * (Mz + 1) + b1));
+    }
+};
+struct RowSamples {
+    const double* __restrict__ a;
+    int Mz;
+    __device__ __forceinline__ WenoData<double> data(int row, int b1) const {
+        double f[6];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) f[i] = __ldg(a + (long long)row * Mz + clampi(b1 - 3 + i, Mz - 1));
+        return weno_data(f);
+    }
+};
+
 // WENO6 of row (., j) at (x, z): 7 evaluations
-__device__ __forceinline__ double row64(const WenoRec<double>* __restrict__ rec, const NodeField& F, int bx, int b1, int j,
+template <class Rows>
+__device__ __forceinline__ double row64(const Rows& rows, const NodeField& F, int bx, int b1, int j,
                                         const WenoPos<double>& pz, const WenoPos<double>& px) {
     double xv[6];
 #pragma unroll 1
-    for (int ix = 0; ix < 6; ++ix)
-        xv[ix] = weno_at(weno_unpack(ldg_rec(rec + ((long long)clampi(bx - 2 + ix, F.Mx - 1) * F.My + j) * (F.Mz + 1) + b1)), pz);
+    for (int ix = 0; ix < 6; ++ix) xv[ix] = weno_at(rows.data(clampi(bx - 2 + ix, F.Mx - 1) * F.My + j, b1), pz);
     return weno_at(weno_data(xv), px);
 }
 
-// piece_quad with WENO6 from records: the z-pass of the 6 x 7 (x, y) stencil rows into the
+// piece_quad with WENO6: the z-pass of the 6 x 7 (x, y) stencil rows into the
 // thread's column zs, then, for each half of the cell below the centroid, the y-stencils' data
 // once for its Gauss points (as piece_quad32, fia_advect32.cu).  Bound by the FP64 pipe, and so by
 // its count of FP64 instructions: about 2400 a piece against 6500 with every 1D interpolant
 // formed from its samples; three passes of a 64^3 density step 51.1 -> 13.6 ms.
+template <class Rows>
 __device__ __forceinline__ double piece_quad64(const PassDesc& d, double cx, double cy, double cz, double ny,
-                                               const WenoRec<double>* __restrict__ arec,
-                                               const WenoRec<double>* __restrict__ prec, const double* __restrict__ psi,
+                                               const Rows& arec, const Rows& prec, const double* __restrict__ psi,
                                                double* zs) {
     const double h = d.h;
     double sx, sz;
@@ -918,9 +939,7 @@ __device__ __forceinline__ double piece_quad64(const PassDesc& d, double cx, dou
         const int row0 = clampi(bx - 2 + ix, d.A.Mx - 1) * d.A.My;
 #pragma unroll 1
         for (int r = 0; r < 7; ++r) {
-            const int row = row0 + clampi(iy0 - 3 + r, d.A.My - 1);
-            zs[(7 * ix + r) * kQuad64Threads] =
-                weno_at(weno_unpack(ldg_rec(arec + (long long)row * (d.A.Mz + 1) + b1)), pz);
+            zs[(7 * ix + r) * kQuad64Threads] = weno_at(arec.data(row0 + clampi(iy0 - 3 + r, d.A.My - 1), b1), pz);
         }
     }
     const int k = d.k;
@@ -963,8 +982,8 @@ __global__ void __launch_bounds__(kQuad64Threads) k_quad64(PassDesc d, const dou
         ps.rec[t].x = piece_quad(d, p.x, p.y, p.z, p.w, a, psi);
     }
 }
-__global__ void __launch_bounds__(kQuad64Threads) k_quad64_weno(PassDesc d, const WenoRec<double>* __restrict__ arec,
-                                                                const WenoRec<double>* __restrict__ prec,
+template <class Rows>
+__global__ void __launch_bounds__(kQuad64Threads) k_quad64_weno(PassDesc d, Rows arec, Rows prec,
                                                                 const double* __restrict__ psi, PieceStore64 ps,
                                                                 long long npc) {
     __shared__ double zcol[42 * kQuad64Threads];   // each thread's z-pass column
@@ -1153,8 +1172,12 @@ static cudaError_t face_stage64(const PassDesc& d, const double* a, const PassWo
         const long long nb = std::min<long long>(blocks_for(npc, kQuad64Threads), 152LL * 16);
         prof_mark(w, 0, s);
         if (weno_records64(d, w))
-            k_quad64_weno<<<(unsigned)nb, kQuad64Threads, 0, s>>>(d, (const WenoRec<double>*)w.arec,
-                                                                  (const WenoRec<double>*)w.prec, w.psi, ps, (long long)npc);
+            k_quad64_weno<<<(unsigned)nb, kQuad64Threads, 0, s>>>(d, RowRecords{(const WenoRec<double>*)w.arec, d.A.Mz},
+                                                                  RowRecords{(const WenoRec<double>*)w.prec, d.P.Mz}, w.psi,
+                                                                  ps, (long long)npc);
+        else if (d.interp == INTERP_WENO6 && !d.full_weno)
+            k_quad64_weno<<<(unsigned)nb, kQuad64Threads, 0, s>>>(d, RowSamples{a, d.A.Mz}, RowSamples{w.psi, d.P.Mz}, w.psi,
+                                                                  ps, (long long)npc);
         else
             k_quad64<<<(unsigned)nb, kQuad64Threads, 0, s>>>(d, a, w.psi, ps, (long long)npc);
         prof_mark(w, 1, s);

@@ -336,7 +336,7 @@ constexpr int kQuadThreads = 128;
 // evaluations.  The advected field's nodes sit half a cell from the y-faces, so the points of
 // one half share their six y-rows, the points of the other half the rows one further up.
 //
-// Density: bound by the L1 data path (86% busy; issue slots 64%, 16 warps per SM by registers): a
+// Density: bound by the L1 data path (72% busy) and issue (67%; 16 warps per SM by registers): a
 // piece reads 42 + 6 records of 32 bytes, and the lanes of a warp spread over several cells.  One
 // launch on the main pass at 128^3 (18.6M pieces): 4.99 ms evaluating every 1D interpolant from its
 // samples, 2.12 ms now; a density step's launches at 256^3: 44.5 -> 21.0 ms.  Measured beside it, with
@@ -405,12 +405,10 @@ __device__ __forceinline__ int piece_quad32(const PassDesc& d, const int* anc, f
 }
 
 // The same with every value interpolated on its own: linear interpolation (main passes with
-// interpolation_method linear), linear in y with the nearest column (the error pass), WENO6 where
-// the records found no memory.
+// interpolation_method linear), linear in y with the nearest column (the error pass).
 template <int METHOD, class L>
 __device__ __forceinline__ float plain_loc(const L& load, const NodeField& F, const int* anc, const float* q) {
-    if constexpr (METHOD == INTERP_WENO6) return weno6_3d_loc(load, F, anc, q);
-    else if constexpr (METHOD == INTERP_LINEAR) return lin3d_loc(load, F, anc, q);
+    if constexpr (METHOD == INTERP_LINEAR) return lin3d_loc(load, F, anc, q);
     else return lin1dy_loc(load, F, anc, q);
 }
 template <int METHOD>
@@ -1004,8 +1002,10 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
             k_quad32_plain<INTERP_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps);
         else if (d.interp != INTERP_WENO6)
             k_quad32_plain<INTERP_1DY_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps);
+        else if (!w.arec && d.comp < 0)
+            k_quad32<FromField<WenoNewton>><<<grid, kQuadThreads, 0, s>>>(d, {FieldRows{a, d.A.Mz}}, nullptr, psi, ps, w.counters);
         else if (!w.arec)
-            k_quad32_plain<INTERP_WENO6><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps);
+            k_quad32<FromField<WenoSamples>><<<grid, kQuadThreads, 0, s>>>(d, {FieldRows{a, d.A.Mz}}, nullptr, psi, ps, w.counters);
         else if (d.comp < 0)
             k_quad32<WenoNewton><<<grid, kQuadThreads, 0, s>>>(d, newton_records(d.A, w.arec), (const float4*)w.prec, psi,
                                                                ps, w.counters);

@@ -360,6 +360,26 @@ cudaError_t volume_correction(fia_session* s, T* rho) {
     return cudaGetLastError();
 }
 
+// The z-pass records; false if there is no memory for them.
+bool make_records(fia_session* s) {
+    const size_t big = (size_t)(s->N[0] + 2) * (s->N[1] + 2) * (s->N[2] + 2);
+    const size_t ab = big * (s->precision == FIA_FP64 ? kRecBytes64 : kRecBytes);
+    const size_t rb = big * (s->precision == FIA_FP64 ? kRecBytes64 : kPsiRecBytes);
+    const size_t at = (ab + 255) & ~(size_t)255;
+    if (cudaMalloc(&s->arec, at + rb) != cudaSuccess) {
+        s->arec = nullptr;
+        cudaGetLastError();
+        return false;
+    }
+    s->prec = (char*)s->arec + at;
+    return true;
+}
+void drop_records(fia_session* s) {
+    cudaStreamSynchronize(s->stream);
+    cudaFree(s->arec);
+    s->arec = s->prec = nullptr;
+}
+
 // One field through move_substances_3D's pass structure (move_substances_3d.cpp:58-226);
 // velocity components follow the same structure with their own split methods.
 template <typename T>
@@ -1011,18 +1031,7 @@ fia_session* fia_create(int nx, int ny, int nz, double cell_length, int precisio
         ok = piece_store_reserve(s->pieces, 10 * big + 1024, big) == cudaSuccess;
     }
     if (ok && precision == FIA_FP64) ok = piece_store64_reserve(s->pieces64, 10 * big + 1024, big) == cudaSuccess;
-    if (ok) {
-        // the z-pass records; a session that finds no memory for them interpolates without
-        const size_t ab = (size_t)big * (precision == FIA_FP64 ? kRecBytes64 : kRecBytes);
-        const size_t rb = (size_t)big * (precision == FIA_FP64 ? kRecBytes64 : kPsiRecBytes);
-        const size_t at = (ab + 255) & ~(size_t)255;
-        if (cudaMalloc(&s->arec, at + rb) == cudaSuccess) {
-            s->prec = (char*)s->arec + at;
-        } else {
-            s->arec = nullptr;
-            cudaGetLastError();
-        }
-    }
+    if (ok) make_records(s);   // a session that finds no memory for them interpolates without
     if (!ok) {
         g_last_error = "fia_create: device allocation failed";
         fia_destroy(s);
@@ -1545,6 +1554,13 @@ int fia_debug_piece_pipeline(fia_session* s, int enable) {
         s->piece_pipeline = enable;
     }
     return s->precision == FIA_FP64 ? s->piece_pipeline : 0;
+}
+
+int fia_debug_records(fia_session* s, int enable) {
+    if (!s || enable < -1 || enable > 1) return FIA_ERR_INVALID;
+    if (enable == 0 && s->arec) drop_records(s);
+    if (enable == 1 && !s->arec && !make_records(s)) return FIA_ERR_NOMEM;
+    return s->arec ? 1 : 0;
 }
 
 int fia_debug_pcg_stuck(fia_session* s, int enable) {

@@ -185,6 +185,7 @@ def _declare(lib):
     lib.fia_debug_clip_fast.argtypes = [vp, ip, ctypes.POINTER(ctypes.c_ulonglong)]
     lib.fia_debug_full_weno.argtypes = [vp, ip]
     lib.fia_debug_pcg_stuck.argtypes = [vp, ip]
+    lib.fia_debug_records.argtypes = [vp, ip]
     lib.fia_debug_piece_pipeline.argtypes = [vp, ip]
     lib.fia_debug_vertex_jitter.argtypes = [vp, ctypes.c_double]
     lib.fia_debug_learned_grad.argtypes = [vp, ip, fp, dp]
@@ -506,6 +507,9 @@ class Grid3D:
         """FP64 form: 1 evaluates every WENO6 in full, 0 collapses it on node planes (default),
         -1 leaves it; returns the setting"""
         return _check(self.lib.fia_debug_full_weno(self.s, enable), "fia_debug_full_weno")
+
+    def debug_records(self, enable=-1):
+        return _check(self.lib.fia_debug_records(self.s, enable), "fia_debug_records")
 
     def debug_pcg_stuck(self, enable=-1):
         return _check(self.lib.fia_debug_pcg_stuck(self.s, enable), "fia_debug_pcg_stuck")

@@ -324,6 +324,9 @@ int fia_debug_clip_fast(fia_session* s, int enable, unsigned long long* deferred
  * psi points of the pieces: equal in exact arithmetic, fewer evaluations), -1 leaves it;
  * returns the setting. */
 int fia_debug_full_weno(fia_session* s, int enable);
+/* the records of the interpolated fields: enable 0 gives them back, as a session that found no memory for
+ * them runs, 1 makes them again, -1 leaves them; returns whether the session has them. */
+int fia_debug_records(fia_session* s, int enable);
 /* the one-kernel Jacobi-PCG: enable 1 makes the first meeting of its blocks find that a bounded wait
  * ran out (the call then returns FIA_ERR_CUDA; the session stays usable), 0 (the default) not, -1
  * leaves it; returns the setting. */
