@@ -1135,7 +1135,7 @@ static cudaError_t launch_faces_from(const PassDesc& d, const T* a, const PassWo
 // WENO6 from records: where the pass interpolates with it, unless every evaluation is wanted in
 // full or the records found no memory (fia_create)
 static bool weno_records64(const PassDesc& d, const PassWork<double>& w) {
-    return w.pieces64 && w.arec && w.prec && d.interp == INTERP_WENO6 && !d.full_weno;
+    return w.pieces64 && w.records->field && d.interp == INTERP_WENO6 && !d.full_weno;
 }
 
 // One face stage of the piece pipeline: clip (growing the store and clipping again when it is
@@ -1164,7 +1164,7 @@ static cudaError_t face_stage64(const PassDesc& d, const double* a, const PassWo
         if (e != cudaSuccess) return e;
         if ((long long)npc <= ps.cap) break;
         // more pieces than the store holds: grow it and clip again
-        e = piece_store64_reserve(ps, (long long)npc + npc / 4 + 1024, big);
+        e = piece_store64_reserve(ps, (long long)npc + npc / 4 + 1024, big, *w.records);
         if (e != cudaSuccess) return e;
     }
     if ((long long)npc > ps.cap) return cudaErrorMemoryAllocation;
@@ -1172,8 +1172,8 @@ static cudaError_t face_stage64(const PassDesc& d, const double* a, const PassWo
         const long long nb = std::min<long long>(blocks_for(npc, kQuad64Threads), 152LL * 16);
         prof_mark(w, 0, s);
         if (weno_records64(d, w))
-            k_quad64_weno<<<(unsigned)nb, kQuad64Threads, 0, s>>>(d, RowRecords{(const WenoRec<double>*)w.arec, d.A.Mz},
-                                                                  RowRecords{(const WenoRec<double>*)w.prec, d.P.Mz}, w.psi,
+            k_quad64_weno<<<(unsigned)nb, kQuad64Threads, 0, s>>>(d, RowRecords{(const WenoRec<double>*)w.records->field, d.A.Mz},
+                                                                  RowRecords{(const WenoRec<double>*)w.records->psi, d.P.Mz}, w.psi,
                                                                   ps, (long long)npc);
         else if (d.interp == INTERP_WENO6 && !d.full_weno)
             k_quad64_weno<<<(unsigned)nb, kQuad64Threads, 0, s>>>(d, RowSamples{a, d.A.Mz}, RowSamples{w.psi, d.P.Mz}, w.psi,
@@ -1216,28 +1216,66 @@ cudaError_t launch_faces(const PassDesc& d, const T* a, const PassWork<T>& w, cu
     return faces_weighted<T>(d, a, w, w.verts, T(1), 0, s);
 }
 
-cudaError_t piece_store64_reserve(PieceStore64& p, long long pieces, long long faces_per_family) {
+cudaError_t RecordStore::make(size_t field_bytes, size_t psi_bytes) {
+    const size_t at = (field_bytes + 255) & ~(size_t)255;
+    const cudaError_t e = cudaMalloc(&field, at + psi_bytes);
+    if (e == cudaSuccess) {
+        psi = (char*)field + at;
+    } else {
+        field = nullptr;
+        cudaGetLastError();
+    }
+    return e;
+}
+
+cudaError_t RecordStore::alloc(void** p, size_t bytes) {
+    auto get = [&] {
+        if (fail > 0) {
+            --fail;
+            return cudaErrorMemoryAllocation;
+        }
+        return cudaMalloc(p, bytes);
+    };
+    cudaError_t e = get();
+    if (e == cudaErrorMemoryAllocation && field) {
+        release();
+        e = get();
+    }
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();
+    }
+    return e;
+}
+
+void RecordStore::release() {
+    cudaDeviceSynchronize();
+    cudaFree(field);
+    field = psi = nullptr;
+}
+
+cudaError_t piece_store64_reserve(PieceStore64& p, long long pieces, long long faces_per_family, RecordStore& mem) {
     cudaDeviceSynchronize();
     // ranges hold 31-bit starts
     if (pieces >= (1LL << 31)) pieces = (1LL << 31) - 1;
     if (pieces > p.cap) {
         cudaFree(p.rec);
         p.rec = nullptr; p.cap = 0;
-        cudaError_t e = cudaMalloc(&p.rec, pieces * sizeof(double4_32a));
+        cudaError_t e = mem.alloc((void**)&p.rec, pieces * sizeof(double4_32a));
         if (e != cudaSuccess) return e;
         p.cap = pieces;
     }
     if (!p.count) {
-        cudaError_t e = cudaMalloc(&p.count, 2 * sizeof(unsigned));
-        if (e == cudaSuccess) e = cudaMalloc(&p.saved, 5 * sizeof(unsigned long long));
+        cudaError_t e = mem.alloc((void**)&p.count, 2 * sizeof(unsigned));
+        if (e == cudaSuccess) e = mem.alloc((void**)&p.saved, 5 * sizeof(unsigned long long));
         if (e != cudaSuccess) return e;
     }
     if (!p.range[0]) {
         for (int f = 0; f < 3; ++f) {
-            cudaError_t e = cudaMalloc(&p.range[f], faces_per_family * sizeof(int2));
+            cudaError_t e = mem.alloc((void**)&p.range[f], faces_per_family * sizeof(int2));
             if (e != cudaSuccess) return e;
         }
-        cudaError_t e = cudaMalloc(&p.deferred, 3 * faces_per_family * sizeof(int));
+        cudaError_t e = mem.alloc((void**)&p.deferred, 3 * faces_per_family * sizeof(int));
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -1265,8 +1303,8 @@ cudaError_t run_pass(const PassDesc& d, const VelocityFields& vel, const T* a, c
     if constexpr (sizeof(T) == sizeof(double)) {
         if (weno_records64(d, w)) {
             if (d.use_integral)
-                k_records64<<<blocks_for(weno_rec_count(d.A), 256), 256, 0, s>>>(d.A, a, (WenoRec<double>*)w.arec);
-            k_records64<<<blocks_for(weno_rec_count(d.P), 256), 256, 0, s>>>(d.P, w.psi, (WenoRec<double>*)w.prec);
+                k_records64<<<blocks_for(weno_rec_count(d.A), 256), 256, 0, s>>>(d.A, a, (WenoRec<double>*)w.records->field);
+            k_records64<<<blocks_for(weno_rec_count(d.P), 256), 256, 0, s>>>(d.P, w.psi, (WenoRec<double>*)w.records->psi);
         }
     }
     if (!d.zero_velocity) {

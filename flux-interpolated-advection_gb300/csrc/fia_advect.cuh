@@ -59,6 +59,17 @@ enum StatusBits : unsigned {
     ST_SUBDIV_OVERFLOW = 8u,    // triangle subdivision stack exhausted
 };
 
+// The z-pass records of the advected field and of psi (fia_weno_rec.cuh), which a session can do without,
+// and the session's other allocations: where there is no memory for one, the records are given back.
+struct RecordStore {
+    void* field = nullptr;
+    void* psi = nullptr;
+    int fail = 0;   // tests: as many of the next allocations find no memory
+    cudaError_t make(size_t field_bytes, size_t psi_bytes);
+    cudaError_t alloc(void** p, size_t bytes);
+    void release();
+};
+
 // Pieces of the FP32 face pipeline (clip -> per-piece quadrature -> per-face sum): the
 // clipped pieces of every face of a pass, contiguous per face, and per face its range.
 struct PieceStore {
@@ -76,7 +87,7 @@ struct PieceStore {
     int clip_fast = 1;           // 0: every face through the local-memory clipper
 };
 // (re)allocates the piece buffers for at least `pieces` pieces; ranges for `faces` per family
-cudaError_t piece_store_reserve(PieceStore& p, long long pieces, long long faces_per_family);
+cudaError_t piece_store_reserve(PieceStore& p, long long pieces, long long faces_per_family, RecordStore& mem);
 void piece_store_free(PieceStore& p);
 
 // The face families of one launch: blocks [first[f], first[f + 1]) hold family f.  One launch for
@@ -110,7 +121,7 @@ struct PieceStore64 {
     unsigned long long* saved = nullptr;   // the session's work counters before a clip (restored on a retry)
     long long cap = 0;           // pieces the buffers hold
 };
-cudaError_t piece_store64_reserve(PieceStore64& p, long long pieces, long long faces_per_family);
+cudaError_t piece_store64_reserve(PieceStore64& p, long long pieces, long long faces_per_family, RecordStore& mem);
 void piece_store64_free(PieceStore64& p);
 
 // Workspace owned by the caller (device pointers).
@@ -130,8 +141,7 @@ struct PassWork {
     cudaEvent_t* prof_ev;   // 2 * prof_cap events, or null
     int* prof_n;            // pairs recorded so far
     int prof_cap;
-    void* arec = nullptr;           // z-pass records of the advected field and of psi (fia_weno_rec.cuh)
-    void* prec = nullptr;
+    RecordStore* records = nullptr; // null: none, and no piece store
     PieceStore* pieces = nullptr;   // FP32 form only
     unsigned long long* launches = nullptr;   // counts the kernels that only some inputs need
     PieceStore64* pieces64 = nullptr;   // FP64 form: the piece pipeline; null: one thread per face (k_faces)

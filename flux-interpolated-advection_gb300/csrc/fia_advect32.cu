@@ -990,27 +990,29 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
         npc = counts[0];
         if ((long long)npc <= ps.cap) break;
         // more pieces than the store holds: grow it and clip again
-        e = piece_store_reserve(ps, (long long)npc + npc / 4 + 1024, std::max(nface[0], std::max(nface[1], nface[2])));
+        e = piece_store_reserve(ps, (long long)npc + npc / 4 + 1024, std::max(nface[0], std::max(nface[1], nface[2])),
+                                *w.records);
         if (e != cudaSuccess) return e;
     }
     if ((long long)npc > ps.cap) return cudaErrorMemoryAllocation;
     if (npc > 0) {
         const long long ntile = ((long long)npc + kQuadThreads - 1) / kQuadThreads;
         const unsigned grid = (unsigned)std::min<long long>(ntile, 152 * 8);
+        const RecordStore& rec = *w.records;   // growing the piece store may have taken them
         prof_mark(w, 0, s);
         if (d.interp == INTERP_LINEAR)
             k_quad32_plain<INTERP_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps);
         else if (d.interp != INTERP_WENO6)
             k_quad32_plain<INTERP_1DY_LINEAR><<<grid, kQuadThreads, 0, s>>>(d, a, psi, ps);
-        else if (!w.arec && d.comp < 0)
+        else if (!rec.field && d.comp < 0)
             k_quad32<FromField<WenoNewton>><<<grid, kQuadThreads, 0, s>>>(d, {FieldRows{a, d.A.Mz}}, nullptr, psi, ps, w.counters);
-        else if (!w.arec)
+        else if (!rec.field)
             k_quad32<FromField<WenoSamples>><<<grid, kQuadThreads, 0, s>>>(d, {FieldRows{a, d.A.Mz}}, nullptr, psi, ps, w.counters);
         else if (d.comp < 0)
-            k_quad32<WenoNewton><<<grid, kQuadThreads, 0, s>>>(d, newton_records(d.A, w.arec), (const float4*)w.prec, psi,
+            k_quad32<WenoNewton><<<grid, kQuadThreads, 0, s>>>(d, newton_records(d.A, rec.field), (const float4*)rec.psi, psi,
                                                                ps, w.counters);
         else
-            k_quad32<WenoSamples><<<grid, kQuadThreads, 0, s>>>(d, sample_records(d.A, w.arec), nullptr, psi, ps,
+            k_quad32<WenoSamples><<<grid, kQuadThreads, 0, s>>>(d, sample_records(d.A, rec.field), nullptr, psi, ps,
                                                                 w.counters);
         prof_mark(w, 1, s);
     }
@@ -1033,17 +1035,18 @@ cudaError_t run_pass<float>(const PassDesc& d64, const VelocityFields& vel64, co
     vel.fu = field32(vel64.fu); vel.fv = field32(vel64.fv); vel.fw = field32(vel64.fw);
     float2* psi = (float2*)w.psi;
     psi32(d, a, psi, s);
-    if (d.interp == INTERP_WENO6 && w.arec) {
+    if (d.interp == INTERP_WENO6 && w.records->field) {
         // without the y-integral no point of the field itself is interpolated
         if (d.comp >= 0) {
-            const WenoSamples::Records r = sample_records(d.A, w.arec);
+            const WenoSamples::Records r = sample_records(d.A, w.records->field);
             if (d.use_integral)
                 k_records_samples<<<nblk(weno_rec_count(d.A), 256), 256, 0, s>>>(d.A, a, const_cast<float4*>(r.r),
                                                                                  const_cast<float*>(r.r2));
         } else {
             if (d.use_integral)
-                k_records_newton<false><<<nblk(weno_rec_count(d.A), 256), 256, 0, s>>>(d.A, a, (float4*)w.arec);
-            k_records_newton<true><<<nblk(weno_rec_count(d.P), 256), 256, 0, s>>>(d.P, psi, (float4*)w.prec);
+                k_records_newton<false><<<nblk(weno_rec_count(d.A), 256), 256, 0, s>>>(d.A, a, (float4*)w.records->field);
+            k_records_newton<true><<<nblk(weno_rec_count(d.P), 256), 256, 0, s>>>(d.P, psi,
+                                                                                   (float4*)w.records->psi);
         }
     }
     const long long nv = (long long)(d.A.Mx + 1) * (d.A.My + 1) * (d.A.Mz + 1);
@@ -1078,13 +1081,13 @@ cudaError_t run_pass<float>(const PassDesc& d64, const VelocityFields& vel64, co
     return cudaGetLastError();
 }
 
-cudaError_t piece_store_reserve(PieceStore& p, long long pieces, long long faces_per_family) {
+cudaError_t piece_store_reserve(PieceStore& p, long long pieces, long long faces_per_family, RecordStore& mem) {
     cudaDeviceSynchronize();
     if (pieces > p.cap) {
         cudaFree(p.rec); cudaFree(p.face);
         p.rec = nullptr; p.face = nullptr; p.cap = 0;
-        cudaError_t e = cudaMalloc(&p.rec, pieces * sizeof(float4));
-        if (e == cudaSuccess) e = cudaMalloc(&p.face, pieces * sizeof(int));
+        cudaError_t e = mem.alloc((void**)&p.rec, pieces * sizeof(float4));
+        if (e == cudaSuccess) e = mem.alloc((void**)&p.face, pieces * sizeof(int));
         if (e != cudaSuccess) return e;
         p.cap = pieces;
     }
@@ -1094,7 +1097,7 @@ cudaError_t piece_store_reserve(PieceStore& p, long long pieces, long long faces
         const size_t nf = (size_t)faces_per_family;
         const size_t rb = up(nf * sizeof(int2)), nb = up(nf * sizeof(float2)), db = up(3 * nf * sizeof(int));
         const size_t eb = up((2 + kMaxPieces32) * sizeof(float4)), cb = 256;
-        cudaError_t e = cudaMalloc(&p.block, 3 * rb + 3 * nb + db + eb + 2 * cb);
+        cudaError_t e = mem.alloc(&p.block, 3 * rb + 3 * nb + db + eb + 2 * cb);
         if (e != cudaSuccess) { p.block = nullptr; return e; }
         char* q = (char*)p.block;
         auto take = [&](size_t b) { char* r = q; q += b; return r; };

@@ -33,7 +33,7 @@ struct fia_session {
     void* vel[3]; void* vel_next[3];
     void* cbuf;                  // correction field (pass 2 result)
     void* psi; void* verts; void* flux[3]; void* flux_rev[3];
-    void* arec = nullptr; void* prec = nullptr;   // z-pass records of the advected field and of psi
+    RecordStore records;         // z-pass records; allocates what the session needs later
     void* verts2 = nullptr;      // flux MacCormack: the vertices traced back (allocated on first use)
     // cell-volume correction (allocated on first use): per-face y n_y sums, cell volumes, the
     // right-hand side and the potential of its Poisson solve
@@ -174,7 +174,7 @@ inline unsigned pass_launches(const fia_session* s, const PassDesc& d) {
     const bool fp64 = s->precision == FIA_FP64;
     const unsigned psi = d.psi_mode == PSI_PLAIN ? 1u : 2u;
     unsigned rec = 0;
-    if (d.interp == INTERP_WENO6 && s->arec) {
+    if (d.interp == INTERP_WENO6 && s->records.field) {
         if (!fp64 && d.comp >= 0) rec = d.use_integral ? 1u : 0u;
         else if (!fp64 || (s->piece_pipeline && !d.full_weno)) rec = d.use_integral ? 2u : 1u;
     }
@@ -251,7 +251,7 @@ PassWork<T> work(fia_session* s) {
     w.prof_ev = s->prof_ev.empty() ? nullptr : s->prof_ev.data();
     w.prof_n = &s->prof_n;
     w.prof_cap = (int)(s->prof_ev.size() / 2);
-    w.arec = s->arec; w.prec = s->prec;
+    w.records = &s->records;
     w.pieces = &s->pieces;
     w.launches = &s->launches;
     w.pieces64 = (s->precision == FIA_FP64 && s->piece_pipeline) ? &s->pieces64 : nullptr;
@@ -315,11 +315,12 @@ PressureWork<T> pressure_work(fia_session* s);
 
 // allocates the buffers of the cell-volume correction on first use
 cudaError_t volume_buffers(fia_session* s) {
-    if (s->vol) return cudaSuccess;
+    if (s->vol_p) return cudaSuccess;
     const size_t fb = s->verts_bytes;                    // one value per node of the largest field
     const size_t pb = s->verts_bytes / s->es * 8;        // one double, or one float pair (FP32 form)
     auto A = [&](void*& dst, size_t bytes) -> cudaError_t {
-        cudaError_t e = cudaMalloc(&dst, bytes);
+        if (dst) return cudaSuccess;
+        cudaError_t e = s->records.alloc(&dst, bytes);
         if (e == cudaSuccess) { s->allocations.push_back(dst); cudaMemsetAsync(dst, 0, bytes, s->stream); }
         return e;
     };
@@ -360,24 +361,10 @@ cudaError_t volume_correction(fia_session* s, T* rho) {
     return cudaGetLastError();
 }
 
-// The z-pass records; false if there is no memory for them.
 bool make_records(fia_session* s) {
     const size_t big = (size_t)(s->N[0] + 2) * (s->N[1] + 2) * (s->N[2] + 2);
-    const size_t ab = big * (s->precision == FIA_FP64 ? kRecBytes64 : kRecBytes);
-    const size_t rb = big * (s->precision == FIA_FP64 ? kRecBytes64 : kPsiRecBytes);
-    const size_t at = (ab + 255) & ~(size_t)255;
-    if (cudaMalloc(&s->arec, at + rb) != cudaSuccess) {
-        s->arec = nullptr;
-        cudaGetLastError();
-        return false;
-    }
-    s->prec = (char*)s->arec + at;
-    return true;
-}
-void drop_records(fia_session* s) {
-    cudaStreamSynchronize(s->stream);
-    cudaFree(s->arec);
-    s->arec = s->prec = nullptr;
+    const bool fp64 = s->precision == FIA_FP64;
+    return s->records.make(big * (fp64 ? kRecBytes64 : kRecBytes), big * (fp64 ? kRecBytes64 : kPsiRecBytes)) == cudaSuccess;
 }
 
 // One field through move_substances_3D's pass structure (move_substances_3d.cpp:58-226);
@@ -392,7 +379,7 @@ cudaError_t advect_field(fia_session* s, int comp, const T* in, T* out, double d
     d.maccormack = p->use_MacCormack_scheme ? 1 : 0;
     if (d.maccormack && !s->verts2) {
         const size_t bytes = 3 * s->verts_bytes;
-        if (cudaMalloc(&s->verts2, bytes) != cudaSuccess) return cudaErrorMemoryAllocation;
+        if (s->records.alloc(&s->verts2, bytes) != cudaSuccess) return cudaErrorMemoryAllocation;
         s->allocations.push_back(s->verts2);
     }
     const VelocityFields vel = velocity(s, vel_fields);
@@ -500,8 +487,8 @@ int pressure_fcg(fia_session* s, const fia_solver_params* sp, PressureReport& r,
     if (!s->pev[0]) { CK(cudaEventCreate(&s->pev[0])); CK(cudaEventCreate(&s->pev[1])); }
     if (!s->fcg_ready) {
         for (int j = 0; j <= kFcgMaxDirs; ++j) {
-            CK(cudaMalloc(&s->fcg.d[j], nc * sizeof(T)));
-            CK(cudaMalloc(&s->fcg.q[j], nc * sizeof(T)));
+            if (!s->fcg.d[j]) CK(s->records.alloc((void**)&s->fcg.d[j], nc * sizeof(T)));
+            if (!s->fcg.q[j]) CK(s->records.alloc((void**)&s->fcg.q[j], nc * sizeof(T)));
         }
         s->fcg_ready = true;
     }
@@ -557,7 +544,7 @@ int refine_fp32(fia_session* s, const fia_solver_params* sp, PressureReport& r, 
     const long long nc = (long long)s->N[0] * s->N[1] * s->N[2];
     const double bb = r.bb;
     if (!(bb > 0.0)) return FIA_OK;
-    if (!s->p64) CK(cudaMalloc(&s->p64, nc * sizeof(double)));
+    if (!s->p64) CK(s->records.alloc((void**)&s->p64, nc * sizeof(double)));
     CK(widen(W.p, s->p64, nc, false, s->stream));
     double rr = 0.0;
     CK(true_residual(W, g, s->h, u, v, w, s->p64, &rr, s->stream));
@@ -1028,9 +1015,9 @@ fia_session* fia_create(int nx, int ny, int nz, double cell_length, int precisio
     if (ok && precision == FIA_FP32C) {
         // about 2.8 pieces per face at CFL 2, three face families per pass; grown on demand
         // faces of one family of any (staggered) field fit in (nx+2)(ny+2)(nz+2)
-        ok = piece_store_reserve(s->pieces, 10 * big + 1024, big) == cudaSuccess;
+        ok = piece_store_reserve(s->pieces, 10 * big + 1024, big, s->records) == cudaSuccess;
     }
-    if (ok && precision == FIA_FP64) ok = piece_store64_reserve(s->pieces64, 10 * big + 1024, big) == cudaSuccess;
+    if (ok && precision == FIA_FP64) ok = piece_store64_reserve(s->pieces64, 10 * big + 1024, big, s->records) == cudaSuccess;
     if (ok) make_records(s);   // a session that finds no memory for them interpolates without
     if (!ok) {
         g_last_error = "fia_create: device allocation failed";
@@ -1073,12 +1060,11 @@ void fia_destroy(fia_session* s) {
     cudaStreamSynchronize(s->stream);
     for (cudaEvent_t e : s->prof_ev) cudaEventDestroy(e);
     for (cudaEvent_t e : s->pev) if (e) cudaEventDestroy(e);
-    if (s->fcg_ready)
-        for (int j = 0; j <= kFcgMaxDirs; ++j) { cudaFree(s->fcg.d[j]); cudaFree(s->fcg.q[j]); }
+    for (int j = 0; j <= kFcgMaxDirs; ++j) { cudaFree(s->fcg.d[j]); cudaFree(s->fcg.q[j]); }
     unet::net_destroy(s->net);
     piece_store_free(s->pieces);
     piece_store64_free(s->pieces64);
-    cudaFree(s->arec);
+    cudaFree(s->records.field);
     if (s->p64) cudaFree(s->p64);
     if (s->solid) cudaFree(s->solid);
     for (void* p : s->allocations) cudaFree(p);
@@ -1365,7 +1351,7 @@ int fia_set_solid_spheres(fia_session* s, int count, const double* centers, cons
     long long pin = nc - 1;
     while (pin >= 0 && m[pin]) --pin;
     if (pin < 0) return FIA_ERR_INVALID;   // no fluid cell left
-    if (!s->solid) CK(cudaMalloc(&s->solid, nc));
+    if (!s->solid) CK(s->records.alloc((void**)&s->solid, nc));
     CK(cudaMemcpy(s->solid, m.data(), nc, cudaMemcpyHostToDevice));
     s->pin = (int)pin;
     s->n_free = nc - nsolid - 1;
@@ -1401,7 +1387,7 @@ static int ensure_net(fia_session* s) {
         return FIA_ERR_UNSUPPORTED;
     }
     if (!s->net) {
-        s->net = unet::net_create(s->N[0], s->N[1], s->N[2], s->stream);
+        s->net = unet::net_create(s->N[0], s->N[1], s->N[2], s->records, s->stream);
         if (!s->net) { g_last_error = "fia_learned: device allocation failed"; return FIA_ERR_NOMEM; }
     }
     return FIA_OK;
@@ -1530,13 +1516,13 @@ int fia_debug_set_piece_capacity(fia_session* s, long long pieces) {
     const long long big = (long long)(s->N[0] + 2) * (s->N[1] + 2) * (s->N[2] + 2);
     if (s->precision == FIA_FP64) {
         piece_store64_free(s->pieces64);
-        CK(piece_store64_reserve(s->pieces64, pieces, big));
+        CK(piece_store64_reserve(s->pieces64, pieces, big, s->records));
         return FIA_OK;
     }
     const int fast = s->pieces.clip_fast;
     piece_store_free(s->pieces);
     s->pieces.clip_fast = fast;
-    CK(piece_store_reserve(s->pieces, pieces, big));
+    CK(piece_store_reserve(s->pieces, pieces, big, s->records));
     return FIA_OK;
 }
 
@@ -1558,9 +1544,15 @@ int fia_debug_piece_pipeline(fia_session* s, int enable) {
 
 int fia_debug_records(fia_session* s, int enable) {
     if (!s || enable < -1 || enable > 1) return FIA_ERR_INVALID;
-    if (enable == 0 && s->arec) drop_records(s);
-    if (enable == 1 && !s->arec && !make_records(s)) return FIA_ERR_NOMEM;
-    return s->arec ? 1 : 0;
+    if (enable == 0 && s->records.field) s->records.release();
+    if (enable == 1 && !s->records.field && !make_records(s)) return FIA_ERR_NOMEM;
+    return s->records.field ? 1 : 0;
+}
+
+int fia_debug_fail_allocations(fia_session* s, int count) {
+    if (!s || count < -1) return FIA_ERR_INVALID;
+    if (count >= 0) s->records.fail = count;
+    return s->records.fail;
 }
 
 int fia_debug_pcg_stuck(fia_session* s, int enable) {

@@ -1214,6 +1214,7 @@ struct TcConfig {
 constexpr bool tc_planes(int txc, int nu, int tpc) { return txc > 1 && nu <= 6 && tpc == 27; }
 
 struct Net {
+    RecordStore* mem;
     int fine[3];
     int dims[4][3];
     cudaStream_t stream;
@@ -1256,7 +1257,7 @@ void combine(const PoissonGrid& g, const float* r, const float* y, const int* di
 
 void* dalloc(Net* n, size_t bytes) {
     void* p = nullptr;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
+    if (n->mem->alloc(&p, bytes) != cudaSuccess) return nullptr;
     cudaMemset(p, 0, bytes);
     n->allocs.push_back(p);
     return p;
@@ -1572,8 +1573,9 @@ cudaError_t pack_all(Net* n, cudaStream_t s) {
 
 }  // namespace
 
-Net* net_create(int nx, int ny, int nz, cudaStream_t s) {
+Net* net_create(int nx, int ny, int nz, RecordStore& mem, cudaStream_t s) {
     Net* n = new Net();
+    n->mem = &mem;
     n->fine[0] = nx; n->fine[1] = ny; n->fine[2] = nz;
     n->stream = s;
     n->adam_t = 0;
@@ -1723,14 +1725,14 @@ int net_add_pair(Net* n, const PoissonGrid& g, const float* r_dev, const float* 
     Pair pr;
     pr.solid = nullptr;
     pr.pin = g.pin;
-    if (cudaMalloc(&pr.r, nf * 4) != cudaSuccess) return -1;
-    if (cudaMalloc(&pr.p, nf * 4) != cudaSuccess) { cudaFree(pr.r); return -1; }
+    if (n->mem->alloc((void**)&pr.r, nf * 4) != cudaSuccess) return -1;
+    if (n->mem->alloc((void**)&pr.p, nf * 4) != cudaSuccess) { cudaFree(pr.r); return -1; }
     auto fail = [&]() { cudaFree(pr.r); cudaFree(pr.p); if (pr.solid) cudaFree(pr.solid); return -1; };
     cudaMemcpyAsync(pr.r, r_dev, nf * 4, cudaMemcpyDeviceToDevice, s);
     cudaMemcpyAsync(pr.p, p_dev, nf * 4, cudaMemcpyDeviceToDevice, s);
     long long nfree = nf - 1;
     if (g.solid) {
-        if (cudaMalloc(&pr.solid, nf) != cudaSuccess) return fail();
+        if (n->mem->alloc((void**)&pr.solid, nf) != cudaSuccess) return fail();
         cudaMemcpyAsync(pr.solid, g.solid, nf, cudaMemcpyDeviceToDevice, s);
         std::vector<unsigned char> m(nf);
         if (cudaMemcpyAsync(m.data(), g.solid, nf, cudaMemcpyDeviceToHost, s) != cudaSuccess ||

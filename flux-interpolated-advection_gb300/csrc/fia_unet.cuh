@@ -23,6 +23,7 @@
 #include <cstdint>
 #include <vector>
 
+#include "fia_advect.cuh"
 #include "fia_pressure.cuh"
 
 namespace fia {
@@ -42,7 +43,8 @@ long long layer_offset(int l);           // offset of layer l's weights [tap][ci
 
 // Device state of one network on one grid size (the fine grid's nx, ny, nz).
 struct Net;
-Net* net_create(int nx, int ny, int nz, cudaStream_t s);
+// mem (which outlives the network) allocates
+Net* net_create(int nx, int ny, int nz, RecordStore& mem, cudaStream_t s);
 void net_destroy(Net* n);
 cudaError_t net_set_weights(Net* n, const float* host, long long count);    // FP32 master
 cudaError_t net_get_weights(Net* n, float* host, long long count);

@@ -186,6 +186,7 @@ def _declare(lib):
     lib.fia_debug_full_weno.argtypes = [vp, ip]
     lib.fia_debug_pcg_stuck.argtypes = [vp, ip]
     lib.fia_debug_records.argtypes = [vp, ip]
+    lib.fia_debug_fail_allocations.argtypes = [vp, ip]
     lib.fia_debug_piece_pipeline.argtypes = [vp, ip]
     lib.fia_debug_vertex_jitter.argtypes = [vp, ctypes.c_double]
     lib.fia_debug_learned_grad.argtypes = [vp, ip, fp, dp]
@@ -510,6 +511,9 @@ class Grid3D:
 
     def debug_records(self, enable=-1):
         return _check(self.lib.fia_debug_records(self.s, enable), "fia_debug_records")
+
+    def debug_fail_allocations(self, count=-1):
+        return _check(self.lib.fia_debug_fail_allocations(self.s, count), "fia_debug_fail_allocations")
 
     def debug_pcg_stuck(self, enable=-1):
         return _check(self.lib.fia_debug_pcg_stuck(self.s, enable), "fia_debug_pcg_stuck")

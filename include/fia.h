@@ -169,7 +169,8 @@ const char* fia_error_string(int code);
  * pass's clipped pieces, sized for 10 pieces per node of the largest field at creation
  * (20 bytes a piece in the FP32C form, 32 in the FP64 form) and grown when a pass needs more,
  * and records of the interpolated fields (68 bytes per node of the largest field in the FP32C
- * form, 128 in the FP64 form), without which, when memory is short, it runs slower. */
+ * form, 128 in the FP64 form), which speed the quadrature up by about a half: they are left out when
+ * there is no memory for them, and given back when something that the session needs later finds none. */
 fia_session* fia_create(int nx, int ny, int nz, double cell_length, int precision);
 void fia_destroy(fia_session* s);
 int fia_last_status(const fia_session* s);
@@ -327,6 +328,9 @@ int fia_debug_full_weno(fia_session* s, int enable);
 /* the records of the interpolated fields: enable 0 gives them back, as a session that found no memory for
  * them runs, 1 makes them again, -1 leaves them; returns whether the session has them. */
 int fia_debug_records(fia_session* s, int enable);
+/* the next `count` allocations of the session's (those made after fia_create) fail as if there were no
+ * device memory; -1 leaves the count; returns it. */
+int fia_debug_fail_allocations(fia_session* s, int count);
 /* the one-kernel Jacobi-PCG: enable 1 makes the first meeting of its blocks find that a bounded wait
  * ran out (the call then returns FIA_ERR_CUDA; the session stays usable), 0 (the default) not, -1
  * leaves it; returns the setting. */
