@@ -547,11 +547,12 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update(PoissonGrid g, double
 // thread of a block takes a quarter of a microsecond), the neighbours' loads are issued before the
 // block's own cells are updated, and what a group of cells needs of its place in the grid is one word,
 // made once.  Microseconds an iteration, with the two kernels above and with this one: FP32 16^3 18 ->
-// 7.1, 64^3 23 -> 10.3, 128^3 36 -> 17.9, 160^3 53 -> 48; FP64 64^3 46 -> 17.6, 128^3 134 -> 79.  (Slots
+// 7.1, 64^3 23 -> 10.2, 128^3 36 -> 18.2, 160^3 53 -> 48; FP64 64^3 46 -> 17.7, 128^3 134 -> 81.  (Slots
 // polled by every block, with the meeting's number beside the value instead of a counter, were slower:
 // 19.8 against 14 us at 64^3.)
-// Rows that are no whole groups take one cell a step, and their places are formed at each visit from 4096
-// cells a block on: 127^3 49 -> 41, 143^3 61 -> 61, 151^3 70 -> 70, 161^3 82 -> 81; FP64 127^3 136 -> 81.
+// Rows that are no whole groups take one cell a step, and from 4096 cells a block on their places are formed
+// at each visit: 127^3 49 -> 41, 141^3 61 -> 55; FP64 127^3 133 -> 82.  FP32 143^3 to 161^3 are
+// within 2% of the two kernels.
 // Larger grids, whose chunks leave no room for two shared arrays, keep the two kernels: there the
 // vectors' traffic is the time (256^3: 152 us for 11 vectors of 67 MB, 108 us at the copy rate).
 constexpr int kPcgThreadsMax = 1024;
@@ -561,6 +562,12 @@ constexpr unsigned kPcgStuck = 1u << 30; // set in the counter when one did
 constexpr size_t kPcgSmem = 224 * 1024;  // dynamic shared memory of a block (227 KB less the static part)
 constexpr int kPcgPartWords = 3;         // doubles a block: one sum, then two
 constexpr int kPcgBlocksMax = 1024;
+// SMs left to other kernels.  A cooperative launch starts when all of its blocks find room, and a block of
+// this kernel shares an SM with nothing that runs there already (its shared memory is another split of
+// L1).  With blocks on all 152 SMs one small kernel of another stream, however long it ran, held the
+// call up: 1.2 s beside a one-thread kernel of 1.2 s.  Costs 1 to 2% from 128^3 on (128^3 17.8 -> 18.1 us,
+// FP64 79.8 -> 81.7).
+constexpr int kPcgLeave = 4;
 constexpr unsigned kPcgOneBlock = 1024;  // groups that one block takes alone
 
 template <typename T>
@@ -1138,7 +1145,7 @@ PcgPlan pcg_plan(const PoissonGrid& g) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
         return p;
-    sms = std::min(sms, kPcgBlocksMax);
+    sms = std::min(std::max(1, sms - kPcgLeave), kPcgBlocksMax);
     const unsigned n = (unsigned)g.nx * g.ny * g.nz, W = g.nz % VecW<T>::W == 0 ? VecW<T>::W : 1, groups = n / W;
     // 512 groups a block in FP32, 256 in FP64 (64^3 FP32 10.7 against 11.2 us an iteration with 256;
     // 20^3 FP64 11.6 against 13.9 with 512)
