@@ -551,8 +551,8 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update(PoissonGrid g, double
 // polled by every block, with the meeting's number beside the value instead of a counter, were slower:
 // 19.8 against 14 us at 64^3.)
 // Rows that are no whole groups take one cell a step, and from 4096 cells a block on their places are formed
-// at each visit: 127^3 49 -> 41, 141^3 61 -> 55; FP64 127^3 133 -> 82.  FP32 143^3 to 161^3 are
-// within 2% of the two kernels.
+// at each visit: 127^3 49 -> 41, 141^3 61 -> 55; FP64 127^3 133 -> 82.  In FP32 they need three shared
+// arrays: with two the two kernels are as fast (143^3 to 161^3 within 2%).
 // Larger grids, whose chunks leave no room for two shared arrays, keep the two kernels: there the
 // vectors' traffic is the time (256^3: 152 us for 11 vectors of 67 MB, 108 us at the copy rate).
 constexpr int kPcgThreadsMax = 1024;
@@ -1138,6 +1138,8 @@ struct PcgPlan {
     size_t smem = 0;
 };
 template <typename T>
+constexpr int pcg_least_arrays(int W) { return sizeof(T) == 4 && W == 1 ? 3 : 2; }
+template <typename T>
 PcgPlan pcg_plan(const PoissonGrid& g) {
     PcgPlan p;
     int dev = 0, sms = 0, coop = 0;
@@ -1153,7 +1155,7 @@ PcgPlan pcg_plan(const PoissonGrid& g) {
     unsigned blocks = groups <= kPcgOneBlock ? 1u : std::min<unsigned>((unsigned)sms, (groups + least - 1) / least);
     const unsigned chunk = (groups + blocks - 1) / blocks * W;
     blocks = (n + chunk - 1) / chunk;
-    for (int a = 4; a >= 2; --a) {
+    for (int a = 4; a >= pcg_least_arrays<T>(W); --a) {
         const size_t smem = ((size_t)a * chunk + 2 * (size_t)g.nz) * sizeof(T);
         if (smem > kPcgSmem) continue;
         p.blocks = (int)blocks;
@@ -1183,7 +1185,9 @@ cudaError_t launch_pcg_w(const PcgPlan& p, const PcgArgs<T>& A, cudaStream_t s) 
     switch (p.arrays) {
         case 4: return p.placed ? launch_pcg_t<T, W, 4, 4>(p, A, s) : launch_pcg_t<T, W, 4, 0>(p, A, s);
         case 3: return p.placed ? launch_pcg_t<T, W, 3, 4>(p, A, s) : launch_pcg_t<T, W, 3, 0>(p, A, s);
-        default: return launch_pcg_t<T, W, 2, 0>(p, A, s);
+        default:
+            if constexpr (pcg_least_arrays<T>(W) == 2) return launch_pcg_t<T, W, 2, 0>(p, A, s);
+            else return cudaErrorInvalidValue;
     }
 }
 template <typename T>
