@@ -22,6 +22,7 @@
 #include "fia_trace.cuh"
 
 #include <algorithm>
+#include <climits>
 
 namespace fia {
 
@@ -983,6 +984,12 @@ static cudaError_t face_stage32(const PassDesc& d, const float* a, const float2*
         if (e == cudaSuccess && counts[2] > 0) {
             k_clip32_local<<<152 * 8, 128, 0, s>>>(d, disp, ps, w.status, w.counters);
             if (w.launches) ++*w.launches;
+            // no second wait where the pieces these faces can have fit at any rate (7 us a pass)
+            const long long most = (long long)counts[0] + (long long)counts[2] * kMaxPieces32;
+            if (most <= std::min(ps.cap, (long long)INT_MAX)) {
+                npc = (unsigned)most;
+                break;
+            }
             e = cudaMemcpyAsync(counts, ps.count, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         }

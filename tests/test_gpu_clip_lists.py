@@ -25,7 +25,7 @@ def step(n, vel, cfl, fast):
     return out
 
 
-@pytest.mark.parametrize("n,cfl,long", [(12, 3.0, False), (24, 16.0, True)])
+@pytest.mark.parametrize("n,cfl,long", [(12, 3.0, False), (24, 16.0, True), (64, 8.0, True)])
 def test_listed_faces(n, cfl, long):
     vel = scenes.fourier_velocity(n, seed=6)
     a, listed, ca, sa = step(n, vel, cfl, 1)
