@@ -1408,11 +1408,11 @@ cudaError_t subtract_gradient_p64(const double* p64, float* u, float* v, float* 
     return cudaGetLastError();
 }
 
-// partial rows: the FCG dot kernel's kFcgMaxDirs + 1 and the direction kernel's 2 (the CG
-// kernels use fewer)
 // the arrival counter of k_pcg and its blocks' partial sums
 size_t pressure_slots() { return 1 + (size_t)kPcgBlocksMax * kPcgPartWords; }
 
+// partial rows: the FCG dot kernel's kFcgMaxDirs + 1 and the direction kernel's 2 (the CG
+// kernels use fewer)
 size_t pressure_partials() { return (size_t)kRedBlocks * (kFcgMaxDirs + 4); }
 
 #define FIA_PRESSURE_INST(T)                                                                                       \

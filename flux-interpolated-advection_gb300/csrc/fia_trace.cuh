@@ -6,7 +6,7 @@
 // density vertex (7 a component) and 45 for a velocity vertex (43 for the component itself); but
 // neighbours share their inner passes.  A block takes N x N x TZ vertices of one component: the
 // z-pass of all rows under the tile's stencils, the y-pass of those, the x-pass of those, each in
-// shared memory, which leaves 2.6 and 5.3 evaluations a vertex and component at N = 8 (3.3 and 9.6 at 4).
+// shared memory, which leaves 2.6 and 5.3 evaluations a vertex and component at N = 8 (3.3 and 8.3 at 4).
 // The items of a pass are dealt to the threads in one sequence, so the tile's depth TZ divides the
 // vertices along z evenly instead of padding them to a warp.
 //

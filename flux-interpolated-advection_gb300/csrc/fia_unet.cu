@@ -522,7 +522,7 @@ __global__ void __launch_bounds__(THREADS) k_conv_tc(ConvArgs a, int n_out, int 
     };
     // the first two chunks load while the halo is staged
     if (tid == 32) for (int c = 0; c < min(2, nchunks); ++c) issue_chunk(c);
-    // halo: plain and upsampled BF16 by cp.async (zero fill outside the grid), the rest computed
+    // halo: plain and upsampled BF16 by cp.async (zero fill outside the grid)
     // A thread keeps one unit and z-offset of the lines (x, y) of the halo and goes from line to line,
     // so that its source, channel and z-bounds are formed once (at 256^3 the 48 -> 16 layer 352 -> 285
     // us, the 16 -> 16 layers 89 -> 81, against one sequence over all units, each taken apart by
